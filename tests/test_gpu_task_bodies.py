@@ -117,3 +117,36 @@ def test_node_solve_singular(fs, cuda):
     # S = I - V1Tu1 V0Tu0 = 0  when V1Tu1 = V0Tu0 = I
     g = [dev(np.eye(r)), dev(np.eye(r)), dev(np.ones((r, 2))), dev(np.ones((r, 2)))]
     assert fs.node_lu_solve(*g) > 0
+
+
+def _gemm_bound(K, AB, C):
+    """Elementwise rounding bound of C + A B over K terms, any order of sums: (K + 3) u each."""
+    return (K + 3) * np.finfo(np.float64).eps * (AB + C)
+
+
+@pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("k,r,c", [(1, 1, 33), (31, 5, 63), (32, 16, 64), (33, 17, 65),
+                                   (63, 15, 100), (64, 32, 128), (65, 33, 129), (127, 48, 40),
+                                   (128, 100, 190), (129, 31, 64), (1000, 64, 257),
+                                   (20011, 37, 129)])
+def test_dmma_tiles_elementwise(fs, cuda, k, r, c, odd):
+    """The FP64 tile GEMM at the edges of its tiles and K stages, with operands
+    on and off 16-byte boundaries, C added in front (beta = 1) and behind."""
+    rng = np.random.default_rng(k + 7 * r + c)
+    X = rng.standard_normal((k, c + r + 1))
+    eta = rng.standard_normal((r, c))
+    U, d = X[:, c + 1:c + 1 + r], X[:, :c]
+    for alpha, beta in ((-1.0, 1.0), (1.0, 1.0), (0.5, -2.0)):
+        Xg = dev(X, k + 1 + (k + odd) % 2)   # even and odd leading dimensions
+        fs.gemm_broadcast(alpha, beta, Xg, c + 1, r, dev(eta, r + odd), 0)
+        got = host(Xg)
+        err = np.abs(got[:, :c] - (beta * d + alpha * (U @ eta)))
+        lim = _gemm_bound(r, abs(alpha) * (np.abs(U) @ np.abs(eta)), abs(beta) * np.abs(d))
+        assert (err <= lim).all()
+        assert (got[:, c:] == X[:, c:]).all()
+    V = rng.standard_normal((k, r))
+    W0 = rng.standard_normal((r, c))
+    Wg = dev(W0, r + odd)
+    fs.gemm_reduce(0.75, dev(V, k + odd), dev(X, k + 2 * odd), 0, c, Wg)
+    err = np.abs(host(Wg) - (W0 + 0.75 * (V.T @ d)))
+    assert (err <= _gemm_bound(k, 0.75 * (np.abs(V).T @ np.abs(d)), np.abs(W0))).all()
