@@ -6,12 +6,12 @@
 // LU of the augmented matrix [D | X]:
 //
 //   for each panel k0:
-//     leaf_panel_kernel   one CTA per leaf: LU with partial pivoting of
-//                         D[k0:n, k0:k0+NB] in shared memory (LAPACK idamax
+//     leaf_panel_reg_kernel  one CTA per leaf: LU with partial pivoting of
+//                         D[k0:n, k0:k0+NB] in registers (LAPACK idamax
 //                         tie rule), written back; the inverses of the
 //                         panel's unit-lower and upper diagonal blocks are
-//                         formed (one thread per column) for the solves;
-//                         ipiv / perm updated, per-leaf "had interchanges" flag
+//                         formed for the solves; ipiv / perm updated,
+//                         per-leaf "had interchanges" flag
 //     leaf_laswp_kernel   the panel's row interchanges on every other column
 //                         of D (LAPACK layout) and of X; a no-op for leaves
 //                         whose panel pivoted on the diagonal
@@ -50,223 +50,59 @@ __device__ inline T tabs(T v) {
   return v < T(0) ? -v : v;
 }
 
-// Panel LU with implicit row interchanges.  Thread t owns the panel rows
-// t, t + 256, ... (storage order, never moved in shared memory) and tracks
-// each row's position in LAPACK's current row order.  Column j: every warp
-// finds its best candidate (largest |a|, lowest current position on ties,
-// as idamax), one barrier, every thread combines the 8 warp results, reads
-// the pivot row and eliminates its own rows; the row at position j takes the
-// pivot's old position (the interchange) and the pivot takes position j.
-// One barrier per column.  At the end the rows are written to D in their
-// final order, which is exactly dgetf2's.
-template <typename T, int NB>
-__global__ void __launch_bounds__(kThreads)
-    leaf_panel_kernel(const LeafFactorTask<T> *__restrict__ tasks, int k0, int panel,
-                      int panel_stride, int *info) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int RPT = 4;  // rows per thread (panel rows <= 1024)
-  const LeafFactorTask<T> tk = tasks[blockIdx.x];
-  const int n = tk.n;
-  if (k0 >= n) return;
-  const int kb = min(NB, n - k0);
-  const int R = n - k0;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int PS = panel_stride;
-  T *P = reinterpret_cast<T *>(smem_raw);        // PS x NB, column-major, storage order
-  T *Lr = P + (size_t)PS * NB;                   // NB x NB row-major
-  T *Ur = Lr + NB * NB;                          // NB x NB row-major
-  int *pv = reinterpret_cast<int *>(Ur + NB * NB);   // NB: pivot position per column
-  int *ps = pv + NB;                                 // NB: pivot storage row per column
-  T *wv = reinterpret_cast<T *>(ps + NB);            // 2 x 8 warp best values
-  int *wp = reinterpret_cast<int *>(wv + 16);        // 2 x 8 warp best positions
-  int *wsr = wp + 16;                                // 2 x 8 warp best storage rows
-  int *dst = wsr + 16;                               // PS: final position of each row
-  T *D = tk.D;
-  const long long ldd = tk.ldd;
-  for (int j = 0; j < kb; ++j) {
-    const T *src = D + (long long)(k0 + j) * ldd + k0;
-    for (int i = tid; i < R; i += kThreads) P[i + (size_t)j * PS] = src[i];
-  }
-  int pos[RPT];
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) pos[q] = tid + q * kThreads;  // current positions
-  auto warp_best = [&](int j, int slot) {
-    T best = T(-1);
-    int bp = 1 << 30, bs = -1;
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int i = tid + q * kThreads;
-      if (i < R && pos[q] >= j) {
-        const T a = tabs(P[i + (size_t)j * PS]);
-        if (a > best || (a == best && pos[q] < bp)) { best = a; bp = pos[q]; bs = i; }
-      }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const T ob = __shfl_down_sync(0xffffffffu, best, off);
-      const int op = __shfl_down_sync(0xffffffffu, bp, off);
-      const int os = __shfl_down_sync(0xffffffffu, bs, off);
-      if (ob > best || (ob == best && op < bp)) { best = ob; bp = op; bs = os; }
-    }
-    if (lane == 0) { wv[slot * 8 + warp] = best; wp[slot * 8 + warp] = bp; wsr[slot * 8 + warp] = bs; }
-  };
-  __syncthreads();
-  warp_best(0, 0);
-  __syncthreads();
-  int info_local = 0;
-  bool swaps = false;
-  for (int j = 0; j < kb; ++j) {
-    const int slot = j & 1;
-    // combine the warp candidates (every thread, same result)
-    T b = wv[slot * 8];
-    int p = wp[slot * 8], sp = wsr[slot * 8];
-#pragma unroll
-    for (int w = 1; w < kThreads / 32; ++w) {
-      const T v = wv[slot * 8 + w];
-      const int vp = wp[slot * 8 + w];
-      if (v > b || (v == b && vp < p)) { b = v; p = vp; sp = wsr[slot * 8 + w]; }
-    }
-    if (sp < 0) { p = j; sp = -1; }  // no candidate (all NaN): keep position j
-    if (tid == 0) { pv[j] = p; ps[j] = sp; }
-    if (p != j) swaps = true;
-    // interchange: the row at position j moves to p, the pivot row to j
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int i = tid + q * kThreads;
-      if (i < R) {
-        if (pos[q] == j && i != sp) pos[q] = p;
-        else if (i == sp) pos[q] = j;
-      }
-    }
-    const T piv = sp >= 0 ? P[sp + (size_t)j * PS] : T(0);
-    if (piv == T(0)) {
-      if (info_local == 0) info_local = k0 + j + 1;
-    } else {
-      const T rinv = T(1) / piv;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        const int i = tid + q * kThreads;
-        if (i < R && pos[q] > j) {
-          const T l = P[i + (size_t)j * PS] * rinv;
-          P[i + (size_t)j * PS] = l;
-          for (int c = j + 1; c < kb; ++c) P[i + (size_t)c * PS] -= l * P[sp + (size_t)c * PS];
-        }
-      }
-    }
-    if (j + 1 < kb) warp_best(j + 1, slot ^ 1);
-    __syncthreads();
-  }
-  // write the rows back in their final order; build the diagonal block
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int i = tid + q * kThreads;
-    if (i < R) dst[i] = pos[q];
-  }
-  __syncthreads();
-  for (int j = 0; j < kb; ++j) {
-    T *col = D + (long long)(k0 + j) * ldd + k0;
-    for (int i = tid; i < R; i += kThreads) col[dst[i]] = P[i + (size_t)j * PS];
-  }
-  for (int e = tid; e < NB * NB; e += kThreads) { Lr[e] = T(0); Ur[e] = T(0); }
-  __syncthreads();
-  for (int i = tid; i < R; i += kThreads) {
-    const int r = dst[i];
-    if (r < kb)
-      for (int k = 0; k < kb; ++k) {
-        const T v = P[i + (size_t)k * PS];
-        if (k < r) Lr[r * NB + k] = v;
-        else Ur[r * NB + k] = v;
-      }
-  }
-  __syncthreads();
-  for (int i = tid; i < NB; i += kThreads) {
-    Lr[i * NB + i] = T(1);
-    if (i >= kb) Ur[i * NB + i] = T(1);
-  }
-  __syncthreads();
-  // inverses, one thread per column j (row-major storage: conflict-free reads)
-  T *Li = Lr, *Ui = Ur;
-  T *Lw = P, *Uw = P + NB * NB;  // the panel buffer is free now
-  if (tid < NB) {
-    const int j = tid;
-    for (int i = 0; i < NB; ++i) Lw[i * NB + j] = (i == j) ? T(1) : T(0);
-    for (int i = j + 1; i < NB; ++i) {
-      T acc = T(0);
-      for (int k = j; k < i; ++k) acc += Li[i * NB + k] * Lw[k * NB + j];
-      Lw[i * NB + j] = -acc;
-    }
-    for (int i = 0; i < NB; ++i) Uw[i * NB + j] = T(0);
-    for (int i = j; i >= 0; --i) {
-      T acc = (i == j) ? T(1) : T(0);
-      for (int k = i + 1; k <= j; ++k) acc -= Ui[i * NB + k] * Uw[k * NB + j];
-      Uw[i * NB + j] = acc / Ui[i * NB + i];
-    }
-  }
-  __syncthreads();
-  T *Lout = tk.Linv + (size_t)panel * NB * NB;
-  T *Uout = tk.Uinv + (size_t)panel * NB * NB;
-  for (int e = tid; e < NB * NB; e += kThreads) {
-    const int i = e % NB, k = e / NB;
-    Lout[e] = Lw[i * NB + k];
-    Uout[e] = Uw[i * NB + k];
-  }
-  if (tid == 0) {
-    tk.swapflag[panel] = swaps ? 1 : 0;
-    for (int j = 0; j < kb; ++j) {
-      const int p = pv[j];
-      tk.ipiv[k0 + j] = k0 + p + 1;
-      if (p != j) {
-        const int t = tk.perm[k0 + j];
-        tk.perm[k0 + j] = tk.perm[k0 + p];
-        tk.perm[k0 + p] = t;
-      }
-    }
-    if (info_local && info && info[tk.info_slot] == 0) info[tk.info_slot] = info_local;
-  }
-}
-
-// Register-resident panel LU, same semantics as leaf_panel_kernel (LAPACK
-// dgetf2 pivot order, implicit interchanges, inverses of the diagonal block).
-// 512 threads; thread t owns panel rows t + 512 q (q < RPT) in registers, so
-// an elimination step touches no shared memory except the pivot row.  Per
-// column: every warp finds its best candidate (largest |a|, lowest current
-// position on ties) and the winning lane publishes its whole row; one
-// barrier; every warp combines the candidates with four shuffles, reads the
-// pivot row (broadcast) and eliminates its rows.  The loop over the NB
-// columns is unrolled so that the row lives in registers.
+// Register-resident panel LU in LAPACK's dgetf2 pivot order, with implicit row
+// interchanges (rows stay in their threads, each tracking its current
+// position), and the inverses of the diagonal block's triangles.
+// Thread t owns panel rows t + threads q (q < RPT) in registers.
+//
+// What bounds it is one column's serial chain (search, publish, barrier,
+// combine, eliminate), so that chain is kept short.  The columns go in
+// sub-blocks of SB = 8: a column's elimination touches its own sub-block
+// only, and the columns behind it are updated once per sub-block, the
+// sub-block's pivot rows solved against each other first (one thread per
+// column).  Every element still gets its updates in column order, each one
+// fused multiply-add, so the factors are those of the column-by-column
+// elimination bit for bit.  Per column: every warp finds its best candidate (largest |a|,
+// lowest current position on ties) with one warp reduction and one ballot
+// unless several rows tie in the reduced bits, each thread having formed its
+// candidate's reciprocal beside the search, and the winning lane publishes
+// its SB values; one barrier; every warp finds the best warp the same way
+// and eliminates its rows.  Warps without live rows only keep the barriers
+// and share the inverses.  A column takes 780 (FP64) / 630 (FP32) cycles with
+// one live warp where the column-by-column form (every warp reducing full
+// keys, whole rows published and updated per column) took ~2500; a 256-row
+// panel with its inverses 27 us (FP64, 32 columns) and 41 us (FP32, 64) where
+// it took 50 and 87 us.
 constexpr int kRegThreads = 512;
-
-// Warp-wide argmax of |a| with the lowest position on ties (idamax order),
-// with warp reductions on the bit patterns (|a| >= 0 orders like its bits).
-// In: per lane (best = |a| or anything when pos == INT_MAX, pos, code).
-// Out: every lane holds the winner's (best, pos, code) and its lane index;
-// pos == INT_MAX when no lane had a candidate.
-__device__ inline void warp_argmax(float &best, int &pos, int &code, int &wlane) {
-  const bool cand = pos != 0x7fffffff;
-  const unsigned key = cand ? __float_as_uint(best) : 0u;
-  const unsigned mx = __reduce_max_sync(0xffffffffu, key);
-  const unsigned pm = __reduce_min_sync(0xffffffffu, key == mx ? (unsigned)pos : 0xffffffffu);
-  const unsigned win = __ballot_sync(0xffffffffu, cand && key == mx && (unsigned)pos == pm);
-  wlane = win ? __ffs(win) - 1 : 0;
-  best = __uint_as_float(mx);
-  pos = win ? (int)pm : 0x7fffffff;
-  code = __shfl_sync(0xffffffffu, code, wlane);
-  if (!win) code = -1;
+// order of the triangular blocks that are inverted on their own
+template <typename T, int NB>
+__host__ __device__ constexpr int panel_sub() {
+  return NB < 64 / (int)sizeof(T) * 2 ? NB : 64 / (int)sizeof(T) * 2;
 }
-__device__ inline void warp_argmax(double &best, int &pos, int &code, int &wlane) {
-  const bool cand = pos != 0x7fffffff;
-  const unsigned long long b = cand ? (unsigned long long)__double_as_longlong(best) : 0ull;
-  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  const bool top = hi == mh && lo == ml;
+
+// |a| as an integer that orders like it, plus one; 0 for a NaN (never a
+// candidate, as idamax skips it)
+__device__ inline unsigned abs_key(float a) {
+  const unsigned b = __float_as_uint(a) & 0x7fffffffu;
+  return b <= 0x7f800000u ? b + 1u : 0u;
+}
+__device__ inline unsigned long long abs_key(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+  return b <= 0x7ff0000000000000ull ? b + 1ull : 0ull;
+}
+__device__ inline unsigned key_high(unsigned k) { return k; }
+__device__ inline unsigned key_high(unsigned long long k) { return (unsigned)(k >> 32); }
+__device__ inline unsigned key_low(unsigned) { return 0u; }
+__device__ inline unsigned key_low(unsigned long long k) { return (unsigned)k; }
+
+// Of the lanes whose `high` is the warp's largest (mx; `win` their ballot,
+// more than one): the one with the largest low word, lowest position on ties.
+__device__ inline int tied_lane(unsigned high, unsigned mx, unsigned low, int pos) {
+  bool top = high == mx;
+  const unsigned ml = __reduce_max_sync(0xffffffffu, top ? low : 0u);
+  top = top && low == ml;
   const unsigned pm = __reduce_min_sync(0xffffffffu, top ? (unsigned)pos : 0xffffffffu);
-  const unsigned win = __ballot_sync(0xffffffffu, cand && top && (unsigned)pos == pm);
-  wlane = win ? __ffs(win) - 1 : 0;
-  best = __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
-  pos = win ? (int)pm : 0x7fffffff;
-  code = __shfl_sync(0xffffffffu, code, wlane);
-  if (!win) code = -1;
+  return __ffs(__ballot_sync(0xffffffffu, top && (unsigned)pos == pm)) - 1;
 }
 
 template <typename T, int NB, int RPT>
@@ -274,14 +110,18 @@ __global__ void __launch_bounds__(kRegThreads, 1)
     leaf_panel_reg_kernel(const LeafFactorTask<T> *__restrict__ tasks, int k0, int panel,
                           int *info) {
   constexpr int NW = kRegThreads / 32;
-  constexpr int LDL = NB + 1;
+  constexpr int SB = 8, NSB = NB / SB;
   constexpr int VW = 16 / sizeof(T);
   using V = typename Vec16<T>::V;
-  __shared__ __align__(16) T wrow[2][NW][NB];
-  __shared__ T wval[2][NW];
-  __shared__ int wpos[2][NW], wcode[2][NW];
-  __shared__ T Lr[NB * LDL], Ur[NB * LDL];
-  __shared__ T udr[NB];
+  __shared__ __align__(16) T wrow[2][NW][SB];  // a warp's candidate row, its sub-block
+  __shared__ T wrcp[2][NW];                    // 1 / candidate
+  __shared__ int4 wmeta[2][NW];                // its key (high, low), position, row
+  __shared__ __align__(16) T Us[SB][NB];           // the pivot rows behind the sub-block
+  __shared__ T Ls[SB][SB + 1];                     // their multipliers
+  // the diagonal block's triangles, both as lower ones, column-major: U with
+  // rows and columns reversed
+  __shared__ __align__(16) T Lk[NB * NB], Uk[NB * NB];
+  __shared__ T udr[NB];  // 1 / U's diagonal, reversed
   __shared__ int pv[NB];
   const LeafFactorTask<T> tk = tasks[blockIdx.x];
   const int n = tk.n;
@@ -289,148 +129,226 @@ __global__ void __launch_bounds__(kRegThreads, 1)
   const int kb = min(NB, n - k0);
   const int R = n - k0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // the launch gives one thread per row (RPT rows per thread) of the panel's
-  // live part, at most kRegThreads: later panels run with fewer warps
   const int nthr = blockDim.x, nw = nthr >> 5;
+  const int nlive = min(nw, (R + 31) >> 5);        // warps with live rows
   T *D = tk.D;
   const long long ldd = tk.ldd;
   T a[RPT][NB];
   int pos[RPT];
-  bool live[RPT];
+  bool live[RPT], act[RPT];  // a row of the panel; one not yet pivotal
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
     const int i = tid + q * nthr;
-    live[q] = i < R;
+    live[q] = act[q] = i < R;
     pos[q] = i;
-    const T *src = D + (k0 + i) + (long long)k0 * ldd;
+    // every load issued before any is used: rows beyond the leaf repeat its
+    // last row, columns beyond the panel its last column
+    const T *src = D + (k0 + min(i, R - 1)) + (long long)k0 * ldd;
+    if (kb == NB) {
 #pragma unroll
-    for (int c = 0; c < NB; ++c) a[q][c] = (live[q] && c < kb) ? src[(long long)c * ldd] : T(0);
+      for (int c = 0; c < NB; ++c) a[q][c] = src[(long long)c * ldd];
+    } else {
+#pragma unroll
+      for (int c = 0; c < NB; ++c) a[q][c] = src[(long long)min(c, kb - 1) * ldd];
+#pragma unroll
+      for (int c = 0; c < NB; ++c)
+        if (c >= kb) a[q][c] = T(0);
+    }
   }
-  bool warp_live = __any_sync(0xffffffffu, live[0]);
+  const bool warp_live = warp < nlive;
   int info_local = 0;
   bool swaps = false;
-  // The columns are factored QW at a time by one unrolled body inside a
-  // runtime loop (a quarter of the code of a fully unrolled panel, which
-  // kept missing the instruction cache): before quarter h every row is
-  // rotated left by h QW, so the quarter's columns sit at register positions
-  // 0 .. QW - 1; positions QW .. NB - h QW - 1 hold the later quarters (they
-  // are updated), the rest the finished ones (left alone).
-  constexpr int QW = NB < 16 ? NB : 16;
-  constexpr int NQ = NB / QW;
+  // Before sub-block h every row is rotated left by h SB, so the sub-block's
+  // columns sit at register positions 0 .. SB - 1; positions SB ..
+  // NB - h SB - 1 hold the later columns, the rest the finished ones.
 #pragma unroll 1
-  for (int h = 0; h < NQ; ++h) {
-    const int live_blocks = NQ - h;  // blocks of QW positions still being updated
+  for (int h = 0; h < NSB; ++h) {
+    const int j0 = h * SB;
+    const int behind = NB - j0 - SB;  // columns behind the sub-block
+    unsigned zero_piv = 0;            // columns without a pivot: no update (uniform)
 #pragma unroll
-    for (int jj = 0; jj < QW; ++jj) {
-      const int j = h * QW + jj;  // panel column
-      if (j < kb) {
-        const int slot = j & 1;
-        if (warp_live) {
-          T best = T(0);
-          int bp = 0x7fffffff, bc = -1;
+    for (int jj = 0; jj < SB; ++jj) {
+      const int j = j0 + jj;  // panel column
+      if (j >= kb) break;
+      const int slot = jj & 1;
+      if (warp_live) {
+        auto best = abs_key(a[0][jj]);
+        if (!act[0]) best = 0;
+        int bp = pos[0], bq = 0;
+        T cand = a[0][jj];
 #pragma unroll
-          for (int q = 0; q < RPT; ++q) {
-            if (live[q] && pos[q] >= j) {
-              const T av = tabs(a[q][jj]);
-              // NaN is never a candidate (as idamax, which skips it)
-              if (av == av && (bp == 0x7fffffff || av > best || (av == best && pos[q] < bp))) {
-                best = av; bp = pos[q]; bc = tid + q * nthr;
-              }
-            }
+        for (int q = 1; q < RPT; ++q) {
+          auto k = abs_key(a[q][jj]);
+          if (!act[q]) k = 0;
+          if (k > best || (k == best && pos[q] < bp)) {
+            best = k; bp = pos[q]; bq = q; cand = a[q][jj];
           }
-          int wl;
-          warp_argmax(best, bp, bc, wl);
-          // the winning lane publishes its row (rotated like every row)
-#pragma unroll
-          for (int q = 0; q < RPT; ++q) {
-            if (bc >= 0 && bc == tid + q * nthr) {
-              V *dst = reinterpret_cast<V *>(wrow[slot][warp]);
-#pragma unroll
-              for (int cv = 0; cv < NB / VW; ++cv) {
-                V v;
-                T *vp = reinterpret_cast<T *>(&v);
-#pragma unroll
-                for (int u = 0; u < VW; ++u) vp[u] = a[q][cv * VW + u];
-                dst[cv] = v;
-              }
-            }
-          }
-          if (lane == 0) { wval[slot][warp] = best; wpos[slot][warp] = bp; wcode[slot][warp] = bc; }
-        } else if (lane == 0) {
-          wval[slot][warp] = T(0); wpos[slot][warp] = 0x7fffffff; wcode[slot][warp] = -1;
         }
-        __syncthreads();
-        // combine the warp candidates (every thread, same result)
-        T pb = T(0);
-        int pp = 0x7fffffff, pc = -1, pw = 0;
-        if (lane < nw) { pb = wval[slot][lane]; pp = wpos[slot][lane]; pc = wcode[slot][lane]; }
-        warp_argmax(pb, pp, pc, pw);  // pw: the winning warp
-        int p = j;
-        T piv = T(0);
-        if (pc >= 0) { p = pp; piv = wrow[slot][pw][jj]; }
+        const unsigned mx = __reduce_max_sync(0xffffffffu, key_high(best));
+        const T rc = sizeof(T) == 4 ? T(__frcp_rn(float(cand))) : T(__drcp_rn(double(cand)));
+        const unsigned win = __ballot_sync(0xffffffffu, key_high(best) == mx);
+        int wl = __ffs(win) - 1;
+        if (win & (win - 1)) wl = tied_lane(key_high(best), mx, key_low(best), bp);
+        if (lane == wl) {
+          wmeta[slot][warp] = make_int4((int)key_high(best), (int)key_low(best), bp,
+                                        tid + bq * nthr);
+          wrcp[slot][warp] = rc;
+          V *dst = reinterpret_cast<V *>(wrow[slot][warp]);
+#pragma unroll
+          for (int cv = jj / VW; cv < SB / VW; ++cv) {
+            V v;
+            T *vp = reinterpret_cast<T *>(&v);
+#pragma unroll
+            for (int u = 0; u < VW; ++u) {
+              vp[u] = a[0][cv * VW + u];
+#pragma unroll
+              for (int q = 1; q < RPT; ++q)
+                if (q == bq) vp[u] = a[q][cv * VW + u];
+            }
+            dst[cv] = v;
+          }
+        }
+      }
+      __syncthreads();
+      if (warp_live) {
+        // the best warp (every warp, same result)
+        const unsigned key = lane < nlive ? (unsigned)wmeta[slot][lane].x : 0u;
+        const unsigned mx = __reduce_max_sync(0xffffffffu, key);
+        const unsigned win = __ballot_sync(0xffffffffu, key == mx);
+        int pw = __ffs(win) - 1;
+        if (win & (win - 1)) {
+          const int4 m = wmeta[slot][lane < nlive ? lane : 0];
+          pw = tied_lane(key, mx, (unsigned)m.y, lane < nlive ? m.z : 0x7fffffff);
+        }
+        const int4 m = wmeta[slot][pw];
+        const T rinv = wrcp[slot][pw];
+        const V *prow = reinterpret_cast<const V *>(wrow[slot][pw]);
+        T u[SB];
+#pragma unroll
+        for (int cv = jj / VW; cv < SB / VW; ++cv) {
+          const V v = prow[cv];
+          const T *vp = reinterpret_cast<const T *>(&v);
+#pragma unroll
+          for (int x = 0; x < VW; ++x) u[cv * VW + x] = vp[x];
+        }
+        // no candidate (FP64: its key's words are both 0): position j keeps its row
+        const bool any = (m.x | (sizeof(T) == 8 ? m.y : 0)) != 0;
+        const int p = any ? m.z : j, pc = any ? m.w : -1;
         if (tid == 0) pv[j] = p;
-        if (p != j) swaps = true;
-        if (warp_live) {
+        swaps |= p != j;
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          const bool me = tid + q * nthr == pc;
+          if (!me && pos[q] == j) pos[q] = p;
+          if (me) pos[q] = j;
+          act[q] = act[q] && pos[q] != j;
+        }
+        if (any && u[jj] != T(0)) {
 #pragma unroll
           for (int q = 0; q < RPT; ++q) {
-            if (live[q]) {
-              if (tid + q * nthr == pc) pos[q] = j;
-              else if (pos[q] == j) pos[q] = p;
+            if (act[q]) {
+              const T l = a[q][jj] * rinv;
+              a[q][jj] = l;
+#pragma unroll
+              for (int c = jj + 1; c < SB; ++c) a[q][c] -= l * u[c];
             }
           }
-          if (piv != T(0)) {
-            const T rinv = sizeof(T) == 4 ? T(__frcp_rn(float(piv))) : T(__drcp_rn(double(piv)));
-            const V *prow = reinterpret_cast<const V *>(wrow[slot][pw]);
+        } else {
+          zero_piv |= 1u << jj;
+          if (info_local == 0) info_local = k0 + j + 1;
+        }
+      }
+    }
+    if (behind > 0 && j0 + SB < kb) {
+      // the sub-block's pivot rows, un-updated behind it, and their multipliers
 #pragma unroll
-            for (int q = 0; q < RPT; ++q) {
-              if (live[q] && pos[q] > j) {
-                const T l = a[q][jj] * rinv;
-                a[q][jj] = l;
+      for (int q = 0; q < RPT; ++q) {
+        const int k = pos[q] - j0;
+        if (live[q] && k >= 0 && k < SB) {
+          V *dst = reinterpret_cast<V *>(Us[k]);
 #pragma unroll
-                for (int cv = (jj + 1) / VW; cv < NB / VW; ++cv) {
-                  if (cv * VW >= QW && (cv * VW) / QW >= live_blocks) continue;
-                  const V v = prow[cv];
+          for (int cv = SB / VW; cv < NB / VW; ++cv) {
+            V v;
+            T *vp = reinterpret_cast<T *>(&v);
+#pragma unroll
+            for (int x = 0; x < VW; ++x) vp[x] = a[q][cv * VW + x];
+            dst[cv] = v;
+          }
+#pragma unroll
+          for (int c = 0; c < SB; ++c) Ls[k][c] = zero_piv >> c & 1 ? T(0) : a[q][c];
+        }
+      }
+      __syncthreads();
+      if (tid < behind && warp_live) {
+        T u[SB];
+#pragma unroll
+        for (int k = 0; k < SB; ++k) u[k] = Us[k][SB + tid];
+#pragma unroll
+        for (int k = 0; k < SB - 1; ++k) {
+#pragma unroll
+          for (int i = k + 1; i < SB; ++i) u[i] -= Ls[i][k] * u[k];
+        }
+#pragma unroll
+        for (int k = 0; k < SB; ++k) Us[k][SB + tid] = u[k];
+      }
+      __syncthreads();
+      if (warp_live) {
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          if (live[q] && pos[q] >= j0 + SB) {
+#pragma unroll
+            for (int g = 1; g < NSB; ++g) {
+              if (g * SB > behind) break;  // uniform: finished columns from here
+#pragma unroll
+              for (int k = 0; k < SB; ++k) {
+                const T l = zero_piv >> k & 1 ? T(0) : a[q][k];
+                const V *ur = reinterpret_cast<const V *>(&Us[k][g * SB]);
+#pragma unroll
+                for (int cv = 0; cv < SB / VW; ++cv) {
+                  const V v = ur[cv];
                   const T *vp = reinterpret_cast<const T *>(&v);
+                  T *ac = &a[q][g * SB + cv * VW];
                   if constexpr (sizeof(T) == 4) {
-                    // pairs of columns through the packed FP32 FMA (each
-                    // half rounded as the scalar a - l p); which columns
-                    // change is known at compile time (jj is unrolled)
+                    // the packed FP32 FMA, each half rounded as a - l u
                     const float2 nl = make_float2(-float(l), -float(l));
 #pragma unroll
-                    for (int u = 0; u < VW; u += 2) {
-                      const int c = cv * VW + u;
-                      if (c > jj) {
-                        const float2 r = __ffma2_rn(nl, make_float2(vp[u], vp[u + 1]),
-                                                    make_float2(a[q][c], a[q][c + 1]));
-                        a[q][c] = r.x;
-                        a[q][c + 1] = r.y;
-                      } else if (c + 1 > jj) {
-                        a[q][c + 1] -= l * vp[u + 1];
-                      }
+                    for (int x = 0; x < VW; x += 2) {
+                      const float2 r = __ffma2_rn(nl, make_float2(vp[x], vp[x + 1]),
+                                                  make_float2(ac[x], ac[x + 1]));
+                      ac[x] = r.x;
+                      ac[x + 1] = r.y;
                     }
                   } else {
 #pragma unroll
-                    for (int u = 0; u < VW; ++u)
-                      if (cv * VW + u > jj) a[q][cv * VW + u] -= l * vp[u];
+                    for (int x = 0; x < VW; ++x) ac[x] -= l * vp[x];
                   }
                 }
               }
             }
+          } else if (live[q] && pos[q] >= j0) {  // this sub-block's pivot rows
+            const V *ur = reinterpret_cast<const V *>(Us[pos[q] - j0]);
+#pragma unroll
+            for (int cv = SB / VW; cv < NB / VW; ++cv) {
+              if (cv * VW >= SB + behind) break;  // uniform: finished columns from here
+              const V v = ur[cv];
+              const T *vp = reinterpret_cast<const T *>(&v);
+#pragma unroll
+              for (int x = 0; x < VW; ++x) a[q][cv * VW + x] = vp[x];
+            }
           }
         }
-        if (piv == T(0) && info_local == 0) info_local = k0 + j + 1;
       }
     }
-    // rotate every row left by QW (after NQ rotations the order is restored)
+    // rotate every row left by SB (after NSB rotations the order is restored)
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
-      T t[QW];
+      T t[SB];
 #pragma unroll
-      for (int c = 0; c < QW; ++c) t[c] = a[q][c];
+      for (int c = 0; c < SB; ++c) t[c] = a[q][c];
 #pragma unroll
-      for (int c = 0; c < NB - QW; ++c) a[q][c] = a[q][c + QW];
+      for (int c = 0; c < NB - SB; ++c) a[q][c] = a[q][c + SB];
 #pragma unroll
-      for (int c = 0; c < QW; ++c) a[q][NB - QW + c] = t[c];
+      for (int c = 0; c < SB; ++c) a[q][NB - SB + c] = t[c];
     }
   }
   // rows to their final positions; diagonal block rows to shared memory
@@ -447,16 +365,16 @@ __global__ void __launch_bounds__(kRegThreads, 1)
         const int r = pos[q];
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-          Lr[r * LDL + c] = c < r ? a[q][c] : (c == r ? T(1) : T(0));
-          Ur[r * LDL + c] = c >= r ? a[q][c] : T(0);
+          Lk[c * NB + r] = c < r ? a[q][c] : (c == r ? T(1) : T(0));
+          Uk[(NB - 1 - c) * NB + NB - 1 - r] = c >= r ? a[q][c] : T(0);
         }
       }
     }
   }
   for (int r = kb + tid; r < NB; r += nthr) {
     for (int c = 0; c < NB; ++c) {
-      Lr[r * LDL + c] = c == r ? T(1) : T(0);
-      Ur[r * LDL + c] = c == r ? T(1) : T(0);
+      Lk[c * NB + r] = c == r ? T(1) : T(0);
+      Uk[(NB - 1 - c) * NB + NB - 1 - r] = c == r ? T(1) : T(0);
     }
   }
   __syncthreads();  // every thread has read its perm entry and written its rows
@@ -464,77 +382,113 @@ __global__ void __launch_bounds__(kRegThreads, 1)
   for (int q = 0; q < RPT; ++q)
     if (live[q]) tk.perm[k0 + pos[q]] = pold[q];
   for (int j = tid; j < kb; j += nthr) tk.ipiv[k0 + j] = k0 + pv[j] + 1;
-  for (int r = tid; r < NB; r += nthr) udr[r] = T(1) / Ur[r * LDL + r];
+  for (int r = tid; r < NB; r += nthr) udr[r] = T(1) / Uk[r * NB + r];
   if (tid == 0) {
     tk.swapflag[panel] = swaps ? 1 : 0;
     if (info_local && info && info[tk.info_slot] == 0) info[tk.info_slot] = info_local;
   }
   __syncthreads();
-  // inverses of the diagonal block, four columns per warp pass: lanes hold
-  // rows lane + 32 r of the columns; x_k is broadcast with a shuffle
-  constexpr int RPL = (NB + 31) / 32;
+  // Inverses of the diagonal block's triangles, from those of their SUB x SUB
+  // diagonal blocks (SUB = 32, FP64 16: a lane's column in registers).  One warp
+  // per such block, a lane per column, the column in registers: after x_k,
+  // all later x_i -= A[i][k] x_k are independent, A[.][k] read as broadcasts.
+  // (With lanes as rows and x_k passed by shuffles the shuffles took 9.5 k
+  // cycles per 32 x 32 FP64 pair and 17.5 k per 64 x 64 FP32 pair.)
+  constexpr int SUB = panel_sub<T, NB>(), NT = NB / SUB, LDI = SUB + VW;
+  static_assert(NT <= 2, "two diagonal blocks at most");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *inv = reinterpret_cast<T *>(smem_raw);  // NT == 2: the four blocks' inverses, column-major
   T *Lout = tk.Linv + (size_t)panel * NB * NB;
   T *Uout = tk.Uinv + (size_t)panel * NB * NB;
-  for (int j0 = warp * 4; j0 < NB; j0 += nw * 4) {
-    T x[4][RPL];
-    // L^{-1}: forward substitution on e_j
+  for (int tri = warp; tri < 2 * NT; tri += nw) {
+    const bool upper = tri >= NT;
+    const int o = tri % NT * SUB;
+    const T *A = (upper ? Uk : Lk) + o * NB + o;
+    T x[SUB];
 #pragma unroll
-    for (int cc = 0; cc < 4; ++cc)
+    for (int i = 0; i < SUB; ++i) x[i] = lane == i ? T(1) : T(0);
 #pragma unroll
-      for (int r = 0; r < RPL; ++r) x[cc][r] = (lane + 32 * r == j0 + cc) ? T(1) : T(0);
+    for (int k = 0; k < SUB; ++k) {
+      __syncwarp();  // A's columns are read as needed (read ahead, they spill)
+      if (upper) x[k] *= udr[o + k];
 #pragma unroll
-    for (int k = 0; k < NB; ++k) {
-      T xk[4];
+      for (int cv = (k + 1) / VW; cv < SUB / VW; ++cv) {
+        const V v = reinterpret_cast<const V *>(A + k * NB)[cv];
+        const T *vp = reinterpret_cast<const T *>(&v);
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) xk[cc] = __shfl_sync(0xffffffffu, x[cc][k / 32], k % 32);
+        for (int u = 0; u < VW; ++u)
+          if (cv * VW + u > k) x[cv * VW + u] -= vp[u] * x[k];
+      }
+    }
+    if (lane < SUB) {
+      T *out = upper ? Uout + (NB - SUB - o) + (size_t)(NB - 1 - o - lane) * NB
+                     : Lout + o + (size_t)(o + lane) * NB;
 #pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (i > k && i < NB) {
-          const T l = Lr[i * LDL + k];
+      for (int cv = 0; cv < SUB / VW; ++cv) {
+        V v, w;
+        T *vp = reinterpret_cast<T *>(&v), *wp = reinterpret_cast<T *>(&w);
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) x[cc][r] -= l * xk[cc];
+        for (int u = 0; u < VW; ++u) {
+          vp[u] = x[cv * VW + u];
+          wp[u] = upper ? x[SUB - 1 - cv * VW - u] : vp[u];
+        }
+        reinterpret_cast<V *>(out)[cv] = w;
+        if constexpr (NT == 2) reinterpret_cast<V *>(inv + (tri * SUB + lane) * LDI)[cv] = v;
+      }
+    }
+  }
+  if constexpr (NT == 2) {
+    // off-diagonal blocks: -A22^{-1} (A21 A11^{-1}), the inner product kept in
+    // the triangle's zero block; a warp takes CB columns, lane = row
+    constexpr int CB = 4;
+    const int row = lane % SUB;
+    const bool mine = lane < SUB;
+    // acc[c] = sum_k A[k sa + row] B[c sb + k]
+    auto product = [&](const T *A, int sa, const T *B, int sb, T (&acc)[CB]) {
+#pragma unroll
+      for (int c = 0; c < CB; ++c) acc[c] = T(0);
+#pragma unroll 4
+      for (int kv = 0; kv < SUB / VW; ++kv) {
+        T x[VW];
+#pragma unroll
+        for (int u = 0; u < VW; ++u) x[u] = A[(kv * VW + u) * sa + row];
+#pragma unroll
+        for (int c = 0; c < CB; ++c) {
+          const V v = reinterpret_cast<const V *>(B + c * sb)[kv];
+          const T *vp = reinterpret_cast<const T *>(&v);
+#pragma unroll
+          for (int u = 0; u < VW; ++u) acc[c] += x[u] * vp[u];
+        }
+      }
+    };
+    T acc[CB];
+    __syncthreads();
+    for (int job = warp; job < 2 * SUB / CB; job += nw) {
+      const bool upper = job >= SUB / CB;
+      const int j = job % (SUB / CB) * CB;
+      T *A = upper ? Uk : Lk;
+      product(A + SUB, NB, inv + ((upper ? 2 : 0) * SUB + j) * LDI, LDI, acc);
+#pragma unroll
+      for (int c = 0; c < CB; ++c)
+        if (mine) A[(SUB + j + c) * NB + lane] = acc[c];
+    }
+    __syncthreads();
+    for (int job = warp; job < 2 * SUB / CB; job += nw) {
+      const bool upper = job >= SUB / CB;
+      const int j = job % (SUB / CB) * CB;
+      product(inv + (upper ? 3 : 1) * SUB * LDI, LDI, (upper ? Uk : Lk) + (SUB + j) * NB, NB, acc);
+#pragma unroll
+      for (int c = 0; c < CB; ++c) {
+        if (!mine) continue;
+        if (upper) {
+          Uout[SUB - 1 - lane + (size_t)(NB - 1 - j - c) * NB] = -acc[c];
+          Uout[NB - 1 - lane + (size_t)(SUB - 1 - j - c) * NB] = T(0);
+        } else {
+          Lout[SUB + lane + (size_t)(j + c) * NB] = -acc[c];
+          Lout[lane + (size_t)(SUB + j + c) * NB] = T(0);
         }
       }
     }
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (i < NB && j0 + cc < NB) Lout[i + (j0 + cc) * NB] = x[cc][r];
-      }
-    // U^{-1}: back substitution on e_j
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) x[cc][r] = (lane + 32 * r == j0 + cc) ? T(1) : T(0);
-#pragma unroll
-    for (int k = NB - 1; k >= 0; --k) {
-      T xk[4];
-      const T dk = udr[k];
-#pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
-        xk[cc] = __shfl_sync(0xffffffffu, x[cc][k / 32], k % 32) * dk;
-        if (lane == k % 32) x[cc][k / 32] = xk[cc];
-      }
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (i < k) {
-          const T u = Ur[i * LDL + k];
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) x[cc][r] -= u * xk[cc];
-        }
-      }
-    }
-#pragma unroll
-    for (int cc = 0; cc < 4; ++cc)
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        const int i = lane + 32 * r;
-        if (i < NB && j0 + cc < NB) Uout[i + (j0 + cc) * NB] = x[cc][r];
-      }
   }
 }
 
@@ -905,12 +859,6 @@ __global__ void __launch_bounds__(kInvThreads)
 
 }  // namespace
 
-template <int NB, typename T>
-size_t panel_smem(int ps) {
-  return (size_t)ps * NB * sizeof(T) + 2 * (size_t)NB * NB * sizeof(T) + 2 * NB * sizeof(int) +
-         16 * sizeof(T) + 32 * sizeof(int) + (size_t)ps * sizeof(int) + 64;
-}
-
 template <typename T>
 void launch_leaf_init(const LeafFactorTask<T> *tasks, int count, int *info, cudaStream_t s) {
   if (count <= 0) return;
@@ -918,24 +866,17 @@ void launch_leaf_init(const LeafFactorTask<T> *tasks, int count, int *info, cuda
   HODLR_LAUNCH_CHECK();
 }
 
-template <typename T, int NB>
-void launch_leaf_panel_nb(const LeafFactorTask<T> *tasks, int count, int max_n, int k0,
-                          int panel, int *info, cudaStream_t s) {
-  const int ps = (max_n - k0 + 3) & ~3;
-  // the panel buffer doubles as the inverses' output (2 NB^2 elements)
-  const int psz = ps < 2 * NB ? 2 * NB : ps;
-  const size_t smem = panel_smem<NB, T>(psz);
-  raise_smem_limit(reinterpret_cast<const void *>(leaf_panel_kernel<T, NB>), smem);
-  leaf_panel_kernel<T, NB><<<count, kThreads, smem, s>>>(tasks, k0, panel, psz, info);
-  HODLR_LAUNCH_CHECK();
-}
-
 template <typename T, int NB, int RPT>
 void launch_leaf_panel_reg(const LeafFactorTask<T> *tasks, int count, int rows, int k0,
                            int panel, int *info, cudaStream_t s) {
-  // one warp per 32 x RPT live rows of the largest leaf's panel
-  const int threads = std::min(kRegThreads, std::max(32, cdiv(cdiv(rows, RPT), 32) * 32));
-  leaf_panel_reg_kernel<T, NB, RPT><<<count, threads, 0, s>>>(tasks, k0, panel, info);
+  // one thread per RPT live rows of the largest leaf's panel, and a warp for
+  // each of the inverses' triangular blocks
+  constexpr int SUB = panel_sub<T, NB>(), blocks = 2 * NB / SUB;
+  const int threads = std::min(kRegThreads, std::max(32 * blocks, cdiv(cdiv(rows, RPT), 32) * 32));
+  // two blocks per triangle: their inverses
+  const size_t smem = blocks > 2 ? (size_t)blocks * SUB * (SUB * sizeof(T) + 16) : 0;
+  raise_smem_limit(reinterpret_cast<const void *>(leaf_panel_reg_kernel<T, NB, RPT>), smem);
+  leaf_panel_reg_kernel<T, NB, RPT><<<count, threads, smem, s>>>(tasks, k0, panel, info);
   HODLR_LAUNCH_CHECK();
 }
 
@@ -956,13 +897,7 @@ void launch_leaf_panel(const LeafFactorTask<T> *tasks, int count, int max_n, int
     if (nb == 16 && rows <= 2 * kRegThreads)
       return launch_leaf_panel_reg<T, 16, 2>(tasks, count, rows, k0, panel, info, s);
   }
-  if (sizeof(T) == 8) {
-    if (nb == 32) launch_leaf_panel_nb<T, 32>(tasks, count, max_n, k0, panel, info, s);
-    else launch_leaf_panel_nb<T, 16>(tasks, count, max_n, k0, panel, info, s);
-  } else {
-    if (nb == 64) launch_leaf_panel_nb<T, 64>(tasks, count, max_n, k0, panel, info, s);
-    else launch_leaf_panel_nb<T, 32>(tasks, count, max_n, k0, panel, info, s);
-  }
+  throw CudaError{cudaErrorInvalidValue};  // no such panel: leaves have at most 1024 rows
 }
 
 template <typename T>

@@ -231,3 +231,31 @@ def test_solve_refined_host_matches_device_path(fs, oracle, cuda, precision):
         np.testing.assert_array_equal(x3, x1)
     Xo, _ = oracle.bfs_solve(s, nthreads=8)
     assert relerr(x1, Xo[:, :m]) < 1e-11
+
+
+@pytest.mark.parametrize("n", [5, 20, 32, 33, 63, 100, 257, 511, 512, 513, 1024])
+def test_leaf_panels_ties_and_zero_columns(fs, cuda, n):
+    """The leaf panel LU at the edges of its sub-blocks, panels and threads, on
+    matrices full of equal pivot candidates, and its INFO for a zero column."""
+    rng = np.random.default_rng(n)
+    A = rng.integers(-1, 2, (n, n)).astype(np.float64) + 3 * np.eye(n) * rng.choice([-1, 1], n)
+    A = A[rng.permutation(n)]                    # pivots off the diagonal
+    B = rng.standard_normal((n, 3))
+    X = np.linalg.solve(A, B)
+    h = fs.HodlrMatrix(3, n, 1, 1024).create_tree()
+    h.set_matrix(A)
+    h.set_rhs(B)
+    solver = fs.FastSolver()
+    solver.bfs_solve(h)
+    cond = np.linalg.cond(A)
+    # both solvers: backward error of a few n u, growth of partial pivoting included
+    assert np.linalg.norm(h.solution() - X) <= 50 * n * cond * 2.0 ** -53 * np.linalg.norm(X)
+    it, rr = solver.solve_refined(h, fs.PREC_MIXED, tol=1e-12, maxiter=30)
+    assert rr <= 1e-12
+    j = int(rng.integers(0, n))
+    A[:, j] = 0.0
+    h.set_matrix(A)
+    for call in (lambda: solver.bfs_solve(h), lambda: solver.factor(h, fs.PREC_MIXED)):
+        with pytest.raises(fs.HodlrError) as e:
+            call()
+        assert e.value.status == j + 1
