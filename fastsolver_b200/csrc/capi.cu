@@ -3,14 +3,15 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <utility>
 #include <vector>
 
 #include "gemm_simt.cuh"
-#include "leaf.cuh"
 #include "node.cuh"
 #include "solver.h"
 #include "tc_gemm.cuh"
@@ -67,15 +68,59 @@ int device_ok() {
   return 0;
 }
 
-// Small stream-ordered device scratch for single-call task bodies.
+// The library's memory pool on the current device.  The device's default pool
+// gives all memory back at every synchronization, so that each task body paid
+// for mapping its scratch again (0.5 to 8 ms in the pass after a wait); this
+// one keeps up to 64 MB between calls.
+cudaMemPool_t scratch_pool() {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  HODLR_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  HODLR_CUDA_TRY(cudaMemPoolCreate(&pool, &props));
+  uint64_t keep = 64u << 20;
+  HODLR_CUDA_TRY(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  pools[dev] = pool;
+  return pool;
+}
+
+// Stream-ordered device scratch of one call.
 struct StreamScratch {
   void *p = nullptr;
   cudaStream_t s;
   explicit StreamScratch(size_t bytes, cudaStream_t st) : s(st) {
-    HODLR_CUDA_TRY(cudaMallocAsync(&p, bytes, s));
+    // a captured allocation belongs to its graph
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+      HODLR_CUDA_TRY(cudaMallocFromPoolAsync(&p, bytes, scratch_pool(), s));
+    else
+      HODLR_CUDA_TRY(cudaMallocAsync(&p, bytes, s));
   }
+  StreamScratch(const StreamScratch &) = delete;
+  StreamScratch &operator=(const StreamScratch &) = delete;
   ~StreamScratch() {
     if (p) cudaFreeAsync(p, s);
+  }
+};
+
+// Several of them, for callees that ask for scratch.
+struct ScratchList {
+  std::vector<std::unique_ptr<StreamScratch>> v;
+  cudaStream_t s;
+  explicit ScratchList(cudaStream_t st) : s(st) {}
+  std::function<void *(size_t)> taker() {
+    return [this](size_t bytes) {
+      v.push_back(std::make_unique<StreamScratch>(bytes, s));
+      return v.back()->p;
+    };
   }
 };
 
@@ -137,13 +182,13 @@ int hodlr_leaf_solve(int n, int nrhs, double *D, int ldd, double *X, int ldx, in
   return guarded([&]() -> int {
     cudaStream_t s = as_stream(stream);
     if (n == 0) return 0;
-    StreamScratch scr(sizeof(int), s);
-    int *info_dev = info ? info : static_cast<int *>(scr.p);
-    LeafTask<double> tk{};
-    tk.D = D; tk.ldd = ldd; tk.X = X; tk.ldx = ldx; tk.ipiv = ipiv; tk.perm = nullptr;
-    tk.n = n; tk.nrhs = nrhs; tk.info_slot = 0;
-    launch_getrf<double>(nullptr, tk, 1, n, info_dev, s);
-    if (nrhs > 0) launch_getrs<double>(nullptr, tk, 1, n, nrhs, s);
+    ScratchList scr(s);
+    const auto take = scr.taker();
+    int *info_dev = info ? info : static_cast<int *>(take(sizeof(int)));
+    LeafFactorTask<double> tk{};
+    tk.D = D; tk.ldd = ldd; tk.X = X; tk.ldx = ldx; tk.ipiv = ipiv;
+    tk.n = n; tk.ncols = nrhs; tk.info_slot = 0;
+    run_leaf_bodies({tk}, info_dev, s, take);
     return finish_info(info, info_dev, s);
   });
 }
@@ -156,31 +201,31 @@ int hodlr_leaf_solve_batched(int count, const hodlr_leaf_desc *descs, int max_n,
   if (max_nrhs < 0) return -4;
   if (!info && count > 0) return -5;
   if (int e = device_ok()) return e;
-  static_assert(sizeof(hodlr_leaf_desc) == sizeof(LeafTask<double>) - 2 * sizeof(int),
-                "descriptor layout");
   return guarded([&]() -> int {
     if (count == 0) return 0;
     cudaStream_t s = as_stream(stream);
-    // hodlr_leaf_desc has no info_slot: expand into LeafTask on the device
     std::vector<hodlr_leaf_desc> h(count);
     HODLR_CUDA_TRY(cudaMemcpyAsync(h.data(), descs, sizeof(hodlr_leaf_desc) * count,
                                    cudaMemcpyDeviceToHost, s));
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
-    std::vector<LeafTask<double>> t(count);
-    for (int i = 0; i < count; ++i) {
-      t[i].D = h[i].D; t[i].X = h[i].X; t[i].ipiv = h[i].ipiv; t[i].perm = h[i].perm;
-      t[i].ldd = h[i].ldd; t[i].ldx = h[i].ldx; t[i].n = h[i].n; t[i].nrhs = h[i].nrhs;
-      t[i].info_slot = i;
-      if (h[i].n > max_n || h[i].nrhs > max_nrhs || h[i].ldd < h[i].n || h[i].ldx < h[i].n)
-        return -2;
+    for (const hodlr_leaf_desc &d : h)
+      if (d.n > max_n || d.nrhs > max_nrhs || d.ldd < d.n || d.ldx < d.n) return -2;
+    // groups of leaves whose scratch (the inverses of their diagonal blocks)
+    // stays within 64 MB, and of at least enough leaves to fill the GPU
+    const size_t per = (size_t)std::max(max_n, 16) * 1024;
+    const int group = (int)std::max<size_t>(296, ((size_t)64 << 20) / per);
+    for (int i0 = 0; i0 < count; i0 += group) {
+      std::vector<LeafFactorTask<double>> t;
+      for (int i = i0; i < std::min(count, i0 + group); ++i) {
+        LeafFactorTask<double> k{};
+        k.D = h[i].D; k.X = h[i].X; k.ipiv = h[i].ipiv; k.perm = h[i].perm;
+        k.ldd = h[i].ldd; k.ldx = h[i].ldx; k.n = h[i].n; k.ncols = h[i].nrhs;
+        k.info_slot = i;
+        t.push_back(k);
+      }
+      ScratchList scr(s);
+      run_leaf_bodies(std::move(t), info, s, scr.taker());
     }
-    StreamScratch scr(sizeof(LeafTask<double>) * count, s);
-    HODLR_CUDA_TRY(cudaMemcpyAsync(scr.p, t.data(), sizeof(LeafTask<double>) * count,
-                                   cudaMemcpyHostToDevice, s));
-    LeafTask<double> none{};
-    auto *tp = static_cast<LeafTask<double> *>(scr.p);
-    launch_getrf<double>(tp, none, count, max_n, info, s);
-    launch_getrs<double>(tp, none, count, max_n, max_nrhs, s);
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
     return 0;
   });
@@ -203,40 +248,40 @@ int hodlr_gemm_reduce(double alpha, int k, int r, int ncol, const double *V, int
   return guarded([&]() -> int {
     if (r == 0 || ncol == 0) return 0;
     cudaStream_t s = as_stream(stream);
-    // split K into row chunks: partials in scratch, then W += sum (fixed order)
-    const int chunk = 4096;
-    const int nsl = k > 0 ? cdiv(k, chunk) : 0;
-    if (nsl == 0) return 0;
-    std::vector<GemmItem<double, double>> it(nsl);
-    std::vector<GemmSeg<double>> sg(nsl);
+    // Split K into row chunks: partials in scratch, then W += sum (fixed
+    // order).  The result is a few tiles (6 of 64 x 64 for 64 x 336), so the
+    // chunks fill the GPU: three resident CTAs per SM, at least 128 rows each.
+    // 16384 rows at r = 64, 336 columns in chunks of 4096 rows (24 CTAs): 140 us.
+    if (k == 0) return 0;
+    const long long tiles = (long long)cdiv(r, 64) * cdiv(ncol, 64);
+    const long long want = std::max<long long>(1, 444 / tiles);
+    const int chunk = cdiv(std::max(128, (int)cdiv<long long>(k, want)), 64) * 64;
+    const int nsl = cdiv(k, chunk);
     const size_t slot = (size_t)r * ncol;
-    StreamScratch part(sizeof(double) * slot * nsl, s);
-    double *pp = static_cast<double *>(part.p);
+    StreamScratch part(sizeof(double) * slot * (nsl + 1), s);
+    double *pp = static_cast<double *>(part.p), *sum = pp + slot * nsl;
+    using Item = GemmItem<double, double>;
+    using Seg = GemmSeg<double>;
+    const size_t o_seg = sizeof(Item) * nsl, o_sum = o_seg + sizeof(Seg) * nsl;
+    std::vector<char> blob(o_sum + sizeof(SumTask<double>));
+    auto *it = reinterpret_cast<Item *>(blob.data());
+    auto *sg = reinterpret_cast<Seg *>(blob.data() + o_seg);
     for (int q = 0; q < nsl; ++q) {
       const int rb = q * chunk, rows = std::min(chunk, k - rb);
-      sg[q] = GemmSeg<double>{V + rb, U + rb + (long long)col_beg * ldu, ldv, ldu, rows, 0};
-      it[q] = GemmItem<double, double>{pp + q * slot, nullptr, r, 0, r, ncol, q, 1};
+      sg[q] = Seg{V + rb, U + rb + (long long)col_beg * ldu, ldv, ldu, rows, 0};
+      it[q] = Item{pp + q * slot, nullptr, r, 0, r, ncol, q, 1};
     }
-    StreamScratch desc(sizeof(GemmItem<double, double>) * nsl + sizeof(GemmSeg<double>) * nsl +
-                           2 * sizeof(GemmItem<double, double>) + sizeof(SumTask<double>) + 256,
-                       s);
-    auto *di = static_cast<GemmItem<double, double> *>(desc.p);
-    auto *ds = reinterpret_cast<GemmSeg<double> *>(di + nsl);
-    HODLR_CUDA_TRY(cudaMemcpyAsync(di, it.data(), sizeof(it[0]) * nsl, cudaMemcpyHostToDevice, s));
-    HODLR_CUDA_TRY(cudaMemcpyAsync(ds, sg.data(), sizeof(sg[0]) * nsl, cudaMemcpyHostToDevice, s));
-    launch_gemm_items<double, double, double>(di, ds, nsl, r, ncol, true, alpha, 0.0, s);
-    // W += fixed-order sum of the partials
-    SumTask<double> st{};
-    StreamScratch tmp(sizeof(double) * slot, s);
-    st.dst = static_cast<double *>(tmp.p);
-    st.src = pp;
-    st.len = (long long)slot;
-    st.stride = (long long)slot;
-    st.nslots = nsl;
-    auto *dst = reinterpret_cast<SumTask<double> *>(ds + nsl);
-    HODLR_CUDA_TRY(cudaMemcpyAsync(dst, &st, sizeof(st), cudaMemcpyHostToDevice, s));
-    launch_sum_slots<double>(dst, 1, st.len, s);
-    launch_add2d<double>(W, ldw, static_cast<double *>(tmp.p), r, r, ncol, s);
+    *reinterpret_cast<SumTask<double> *>(blob.data() + o_sum) =
+        SumTask<double>{sum, pp, (long long)slot, (long long)slot, nsl, 0};
+    StreamScratch desc(blob.size(), s);
+    char *dev = static_cast<char *>(desc.p);
+    launch_param_copy(dev, blob.data(), blob.size(), s);
+    launch_gemm_items<double, double, double>(reinterpret_cast<Item *>(dev),
+                                              reinterpret_cast<Seg *>(dev + o_seg), nsl, r, ncol,
+                                              true, alpha, 0.0, s);
+    launch_sum_slots<double>(reinterpret_cast<SumTask<double> *>(dev + o_sum), 1,
+                             (long long)slot, s);
+    launch_add2d<double>(W, ldw, sum, r, r, ncol, s);
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
     return 0;
   });
@@ -314,66 +359,49 @@ static int node_solve_common(int form, int r0, int r1, int c, const double *V0Tu
   if (int e = device_ok()) return e;
   return guarded([&]() -> int {
     cudaStream_t s = as_stream(stream);
-    // scratch: task | S (r0 x r0) | F (r1 x r0) | I (r0 x r0) | M (s2 x s2) | eta (s2 x c)
-    //          | info | gram item + segment | apply item + 2 segments
-    const int s2 = r0 + r1;
+    // scratch: descriptors | S (r0 x r0) | F (r1 x r0) | M (s2 x s2) | eta (s2 x c) | info
+    using Item = GemmItem<double, double>;
+    using Seg = GemmSeg<double>;
+    struct Desc {
+      NodeTask<double, double> task;
+      Item gram, apply;
+      Seg gseg, aseg[2];
+    } h{};
+    const int s2 = r0 + r1, max_r = std::max(r0, r1);
     const size_t nR = (size_t)r0 * r0, nF = (size_t)r1 * r0, nM = (size_t)s2 * s2;
-    const size_t nE = (size_t)s2 * (c > 0 ? c : 1);
-    const size_t need = 256 + sizeof(double) * (2 * nR + nF + nM + nE) + 8 * sizeof(int) + 1024;
-    StreamScratch scr(need, s);
-    char *base = static_cast<char *>(scr.p);
-    auto *task = reinterpret_cast<NodeTask<double, double> *>(base);
-    double *S = reinterpret_cast<double *>(base + 256);
-    double *F = S + nR;
-    double *ident = F + nF;
-    double *M = ident + nR;
-    double *eta = M + nM;
+    const size_t nE = (size_t)s2 * std::max(c, 1), head = (sizeof(Desc) + 255) / 256 * 256;
+    StreamScratch scr(head + sizeof(double) * (nR + nF + nM + nE + 1), s);
+    auto *d = static_cast<Desc *>(scr.p);
+    double *S = reinterpret_cast<double *>(static_cast<char *>(scr.p) + head);
+    double *F = S + nR, *M = F + nF, *eta = M + nM;
     int *info_dev = reinterpret_cast<int *>(eta + nE);
-    auto *gitem = reinterpret_cast<GemmItem<double, double> *>(
-        (reinterpret_cast<uintptr_t>(info_dev + 8) + 15) & ~uintptr_t(15));
-    auto *gseg = reinterpret_cast<GemmSeg<double> *>(gitem + 1);
-    auto *aitem = reinterpret_cast<GemmItem<double, double> *>(gseg + 1);
-    auto *aseg = reinterpret_cast<GemmSeg<double> *>(aitem + 1);
-    NodeTask<double, double> k{};
-    k.W0u = V0Tu0; k.W1u = V1Tu1; k.ldw0u = ld00; k.ldw1u = ld11;
-    k.S = S; k.F = F; k.M = M;
-    k.r0 = r0; k.r1 = r1; k.info_slot = 0;
-    HODLR_CUDA_TRY(cudaMemcpyAsync(task, &k, sizeof(k), cudaMemcpyHostToDevice, s));
-    std::vector<double> I(nR, 0.0);
-    for (int i = 0; i < r0; ++i) I[(size_t)i * r0 + i] = 1.0;
-    GemmSeg<double> g{V1Tu1, V0Tu0, ld11, ld00, r1, 0};
-    GemmItem<double, double> git{S, ident, r0, r0, r0, r0, 0, 1};
-    GemmSeg<double> a2[2] = {{M, V0Td0, s2, ld0d, r1, 0},
-                             {M + (size_t)r1 * s2, V1Td1, s2, ld1d, r0, 0}};
-    GemmItem<double, double> ait{eta, nullptr, s2, 0, s2, c, 0, 2};
-    if (form == 0) {
-      // S = I - V1Tu1 V0Tu0 (the dgemm at solver_tasks.cc:261)
-      HODLR_CUDA_TRY(cudaMemcpyAsync(ident, I.data(), sizeof(double) * nR, cudaMemcpyHostToDevice, s));
-      HODLR_CUDA_TRY(cudaMemcpyAsync(gitem, &git, sizeof(git), cudaMemcpyHostToDevice, s));
-      HODLR_CUDA_TRY(cudaMemcpyAsync(gseg, &g, sizeof(g), cudaMemcpyHostToDevice, s));
-      launch_gemm_items<double, double, double>(gitem, gseg, 1, r0, r0, false, -1.0, 1.0, s);
+    h.task.W0u = V0Tu0; h.task.W1u = V1Tu1; h.task.ldw0u = ld00; h.task.ldw1u = ld11;
+    h.task.S = S; h.task.F = F; h.task.M = M;
+    h.task.r0 = r0; h.task.r1 = r1; h.task.info_slot = 0;
+    h.gseg = Seg{V1Tu1, V0Tu0, ld11, ld00, r1, 0};
+    h.gram = Item{S, S, r0, r0, r0, r0, 0, 1};
+    h.aseg[0] = Seg{M, V0Td0, s2, ld0d, r1, 0};
+    h.aseg[1] = Seg{M + (size_t)r1 * s2, V1Td1, s2, ld1d, r0, 0};
+    h.apply = Item{eta, nullptr, s2, 0, s2, c, 0, 2};
+    launch_param_copy(d, &h, sizeof(h), s);
+    const int max_s = form == 0 ? r0 : s2;
+    if (form == 0 && !node_factor_stages(max_s, max_r)) {
+      // S = I - V1Tu1 V0Tu0 (the dgemm at solver_tasks.cc:261) on the identity
+      launch_identity(S, r0, s);
+      launch_gemm_items<double, double, double>(&d->gram, &d->gseg, 1, r0, r0, false, -1.0, 1.0, s);
     }
-    HODLR_CUDA_TRY(cudaMemcpyAsync(aitem, &ait, sizeof(ait), cudaMemcpyHostToDevice, s));
-    HODLR_CUDA_TRY(cudaMemcpyAsync(aseg, a2, sizeof(a2), cudaMemcpyHostToDevice, s));
-    launch_node_factor<double, double>(task, 1, form == 0 ? r0 : s2, r0 > r1 ? r0 : r1, form,
-                                       info_dev, s);
-    int hinfo = 0;
-    HODLR_CUDA_TRY(cudaMemcpyAsync(&hinfo, info_dev, sizeof(int), cudaMemcpyDeviceToHost, s));
-    HODLR_CUDA_TRY(cudaStreamSynchronize(s));  // also ends the host staging buffers' use
-    if (info) HODLR_CUDA_TRY(cudaMemcpyAsync(info, info_dev, sizeof(int), cudaMemcpyDeviceToDevice, s));
-    if (hinfo == 0 && c > 0) {
-      launch_gemm_items<double, double, double>(aitem, aseg, 1, s2, c, false, 1.0, 0.0, s);
-      // outputs in place: form 0 writes eta0 over V1Td1, eta1 over V0Td0
-      // (fast_solver.cc:238-240); form 1 eta0 over V0Td0, eta1 over V1Td1.
-      double *o0 = form == 0 ? V1Td1 : V0Td0;
-      double *o1 = form == 0 ? V0Td0 : V1Td1;
-      const int l0 = form == 0 ? ld1d : ld0d, l1 = form == 0 ? ld0d : ld1d;
-      HODLR_CUDA_TRY(cudaMemcpy2DAsync(o0, sizeof(double) * l0, eta, sizeof(double) * s2,
-                                       sizeof(double) * r0, c, cudaMemcpyDeviceToDevice, s));
-      HODLR_CUDA_TRY(cudaMemcpy2DAsync(o1, sizeof(double) * l1, eta + r0, sizeof(double) * s2,
-                                       sizeof(double) * r1, c, cudaMemcpyDeviceToDevice, s));
+    launch_node_factor<double, double>(&d->task, 1, max_s, max_r, form, info_dev, s);
+    if (c > 0) {
+      launch_gemm_items<double, double, double>(&d->apply, d->aseg, 1, s2, c, false, 1.0, 0.0, s);
+      // outputs in place unless the system was singular: form 0 writes eta0
+      // over V1Td1, eta1 over V0Td0 (fast_solver.cc:238-240); form 1 eta0
+      // over V0Td0, eta1 over V1Td1
+      launch_node_output(eta, r0, r1, c, form == 0 ? V1Td1 : V0Td0, form == 0 ? ld1d : ld0d,
+                         form == 0 ? V0Td0 : V1Td1, form == 0 ? ld0d : ld1d, info_dev, s);
     }
-    HODLR_CUDA_TRY(cudaStreamSynchronize(s));  // scratch lifetime
+    if (info)
+      HODLR_CUDA_TRY(cudaMemcpyAsync(info, info_dev, sizeof(int), cudaMemcpyDeviceToDevice, s));
+    const int hinfo = finish_info(nullptr, info_dev, s);
     return info ? 0 : hinfo;  // with a device INFO pointer the value goes there
   });
 }
@@ -412,11 +440,14 @@ int hodlr_gemm_broadcast(double alpha, double beta, int k, int r, int c, double 
     GemmSeg<double> sg{X + (long long)u_col_beg * ldx, eta, ldx, lde, r, 0};
     double *Cp = X + (long long)d_col_beg * ldx;
     GemmItem<double, double> it{Cp, Cp, ldx, ldx, k, c, 0, 1};
-    StreamScratch scr(sizeof(sg) + sizeof(it) + 64, s);
+    struct {
+      GemmItem<double, double> it;
+      GemmSeg<double> sg;
+    } h{it, sg};
+    StreamScratch scr(sizeof(h), s);
     auto *di = static_cast<GemmItem<double, double> *>(scr.p);
     auto *ds = reinterpret_cast<GemmSeg<double> *>(di + 1);
-    HODLR_CUDA_TRY(cudaMemcpyAsync(di, &it, sizeof(it), cudaMemcpyHostToDevice, s));
-    HODLR_CUDA_TRY(cudaMemcpyAsync(ds, &sg, sizeof(sg), cudaMemcpyHostToDevice, s));
+    launch_param_copy(di, &h, sizeof(h), s);
     launch_gemm_items<double, double, double>(di, ds, 1, k, c, false, alpha, beta, s);
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
     return 0;

@@ -63,21 +63,6 @@ __host__ __device__ inline T cdiv(T a, T b) {
 // Task descriptors (device-resident arrays, one launch per level)
 // ---------------------------------------------------------------------------
 
-// Leaf LU + solve.  T is the factor precision.
-template <typename T>
-struct LeafTask {
-  T *D;          // n x n, ldd (overwritten by the LU factors)
-  T *X;          // n x nrhs, ldx (overwritten by the solution)
-  int *ipiv;     // n, LAPACK 1-based pivots
-  int *perm;     // n, final row order
-  long long ldd;
-  long long ldx;
-  int n;
-  int nrhs;      // columns solved by getrs (0..nrhs-1 of X)
-  int info_slot; // index into the info array
-  int pad;
-};
-
 // One operand pair of a GEMM item: op(A) (M x K) times B (K x N).
 //   TRANS (reduce):        A is K x M column-major (lda), op(A) = A^T
 //   not TRANS (broadcast): A is M x K column-major (lda)

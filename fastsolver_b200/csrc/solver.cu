@@ -21,7 +21,6 @@
 #include <cstring>
 
 #include "gemm_simt.cuh"
-#include "leaf.cuh"
 #include "leaf_blocked.cuh"
 #include "node.cuh"
 #include "solver.h"
@@ -93,10 +92,173 @@ void path_need(const Tree &t, bool factor, int chunk, size_t &part, size_t &wfin
 }
 
 
-// Step lists of the two-level blocked leaf factorization (see LeafPlan and
-// leaf_blocked.cu): forward steps on [D | X], then the backward solve on X.
-// Every step is one merged launch over all leaves; a leaf without work in a
-// step contributes no item.
+// One step of the two-level blocked leaf factorization (see LeafPlan and
+// leaf_blocked.cu) with its GEMM items on the host.
+template <typename T>
+struct HostStep {
+  using Kind = typename LeafPlan<T>::Kind;
+  Kind kind;
+  int k0 = 0, panel = 0, block = 0, np = 0;
+  int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+  bool with_x = false;
+  std::vector<GemmItem<T, T>> it;
+  std::vector<GemmSeg<T>> sg;
+  void add(T *C, long long ldc, int M, int N, const T *A, long long lda, const T *B,
+           long long ldb, int K, bool inplace) {
+    if (M <= 0 || N <= 0 || K <= 0) return;
+    GemmSeg<T> g{A, B, lda, ldb, K, 0};
+    GemmItem<T, T> i{C, inplace ? C : nullptr, ldc, inplace ? ldc : 0, M, N, (int)sg.size(), 1};
+    sg.push_back(g);
+    it.push_back(i);
+  }
+};
+
+// The steps of the blocked factorization of `tasks` (panels of NB columns in
+// outer blocks of OB, a multiple of NB): forward steps on [D | X], then the
+// backward solve on X, each one merged launch over all leaves; a leaf without
+// work in a step contributes no item.  binv: block-row solves by the inverses
+// of the outer diagonal blocks, in place on the block's rows, which one GEMM
+// tile row (128) covers (the GEMM launchers run launches of items of at most
+// 128 rows as one tile row).
+template <typename T>
+void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int nblocks, bool binv,
+                std::vector<HostStep<T>> &fwd, std::vector<HostStep<T>> &bwd) {
+  using Plan = LeafPlan<T>;
+  const int P = OB / NB;
+  auto step = [](typename Plan::Kind kind) {
+    HostStep<T> st;
+    st.kind = kind;
+    return st;
+  };
+  auto laswp_step = [&](int p0, int np, int a0, int a1, int b0, int b1, bool with_x) {
+    HostStep<T> st = step(Plan::kLaswp);
+    st.panel = p0;
+    st.np = np;
+    st.a0 = a0; st.a1 = a1; st.b0 = b0; st.b1 = b1;
+    st.with_x = with_x;
+    return st;
+  };
+  constexpr int kAll = 1 << 30;
+  for (int J = 0; J < nblocks; ++J) {
+    const int j0 = J * OB;
+    // the block's panels: factor, interchange and update inside the block columns
+    for (int p = 0; p < P; ++p) {
+      const int pi = J * P + p, k0 = pi * NB;
+      HostStep<T> pan = step(Plan::kPanel);
+      pan.k0 = k0;
+      pan.panel = pi;
+      fwd.push_back(pan);
+      fwd.push_back(laswp_step(pi, 1, j0, k0, k0 + NB, j0 + OB, false));
+      HostStep<T> tr = step(Plan::kTrsm), up = step(Plan::kUpdate);
+      for (const LeafFactorTask<T> &k : tasks) {
+        if (k0 >= k.n) continue;
+        const int kb = std::min(NB, k.n - k0);
+        const int N = std::min(j0 + OB, k.n) - (k0 + kb);
+        const int rest = k.n - k0 - kb;
+        const T *Li = k.Linv + (size_t)pi * NB * NB;
+        T *U12 = k.D + k0 + (long long)(k0 + kb) * k.ldd;
+        tr.add(U12, k.ldd, kb, N, Li, NB, U12, k.ldd, kb, false);
+        up.add(k.D + (k0 + kb) + (long long)(k0 + kb) * k.ldd, k.ldd, rest, N,
+               k.D + (k0 + kb) + (long long)k0 * k.ldd, k.ldd, U12, k.ldd, kb, true);
+      }
+      fwd.push_back(std::move(tr));
+      fwd.push_back(std::move(up));
+    }
+    // the block's interchanges on the columns left and right of it and on X
+    fwd.push_back(laswp_step(J * P, P, 0, j0, j0 + OB, kAll, true));
+    if (binv) {
+      // block rows: U12 = L11^{-1} A12 on R = (D right of the block | X), one
+      // product with the inverse of the block's unit-lower triangle
+      HostStep<T> inv = step(Plan::kBlockInv);
+      inv.block = J;
+      fwd.push_back(inv);
+      HostStep<T> tr = step(Plan::kTrsm);
+      for (const LeafFactorTask<T> &k : tasks) {
+        if (j0 >= k.n) continue;
+        const int obe = std::min(OB, k.n - j0);
+        const T *Li = k.LinvB + (size_t)J * OB * OB;
+        T *Dr = k.D + j0 + (long long)(j0 + obe) * k.ldd;
+        T *Xr = k.X + j0;
+        tr.add(Dr, k.ldd, obe, k.n - j0 - obe, Li, OB, Dr, k.ldd, obe, false);
+        tr.add(Xr, k.ldx, obe, k.ncols, Li, OB, Xr, k.ldx, obe, false);
+      }
+      fwd.push_back(std::move(tr));
+    }
+    // block rows: U12 = L11^{-1} A12 by panels on R = (D right of the block | X)
+    for (int p = 0; p < (binv ? 0 : P); ++p) {
+      const int pi = J * P + p, k0 = pi * NB;
+      HostStep<T> tr = step(Plan::kTrsm), up = step(Plan::kUpdate);
+      for (const LeafFactorTask<T> &k : tasks) {
+        if (k0 >= k.n) continue;
+        const int kb = std::min(NB, k.n - k0);
+        const int obe = std::min(OB, k.n - j0);
+        const int nd = k.n - j0 - obe;           // D columns right of the block
+        const int below = j0 + obe - k0 - kb;    // block rows below this panel
+        const T *Li = k.Linv + (size_t)pi * NB * NB;
+        T *Dr = k.D + k0 + (long long)(j0 + obe) * k.ldd;
+        T *Xr = k.X + k0;
+        tr.add(Dr, k.ldd, kb, nd, Li, NB, Dr, k.ldd, kb, false);
+        tr.add(Xr, k.ldx, kb, k.ncols, Li, NB, Xr, k.ldx, kb, false);
+        const T *L = k.D + (k0 + kb) + (long long)k0 * k.ldd;
+        up.add(Dr + kb, k.ldd, below, nd, L, k.ldd, Dr, k.ldd, kb, true);
+        up.add(Xr + kb, k.ldx, below, k.ncols, L, k.ldd, Xr, k.ldx, kb, true);
+      }
+      fwd.push_back(std::move(tr));
+      fwd.push_back(std::move(up));
+    }
+    // trailing update of depth OB: A22 -= L21 U12 on R, rows below the block
+    HostStep<T> big = step(Plan::kUpdate);
+    for (const LeafFactorTask<T> &k : tasks) {
+      if (j0 >= k.n) continue;
+      const int obe = std::min(OB, k.n - j0);
+      const int rest = k.n - j0 - obe;
+      const T *L21 = k.D + (j0 + obe) + (long long)j0 * k.ldd;
+      big.add(k.D + (j0 + obe) + (long long)(j0 + obe) * k.ldd, k.ldd, rest, rest, L21, k.ldd,
+              k.D + j0 + (long long)(j0 + obe) * k.ldd, k.ldd, obe, true);
+      big.add(k.X + (j0 + obe), k.ldx, rest, k.ncols, L21, k.ldd, k.X + j0, k.ldx, obe, true);
+    }
+    fwd.push_back(std::move(big));
+  }
+  // backward solve on X, last block first
+  for (int J = nblocks - 1; J >= 0; --J) {
+    const int j0 = J * OB;
+    if (binv) {
+      // X[block] = U11^{-1} X[block]: one product with the block's upper inverse
+      HostStep<T> tr = step(Plan::kTrsm);
+      for (const LeafFactorTask<T> &k : tasks) {
+        if (j0 >= k.n) continue;
+        const int obe = std::min(OB, k.n - j0);
+        T *Xk = k.X + j0;
+        tr.add(Xk, k.ldx, obe, k.ncols, k.UinvB + (size_t)J * OB * OB, OB, Xk, k.ldx, obe, false);
+      }
+      bwd.push_back(std::move(tr));
+    }
+    for (int p = binv ? -1 : P - 1; p >= 0; --p) {
+      const int pi = J * P + p, k0 = pi * NB;
+      HostStep<T> tr = step(Plan::kTrsm), up = step(Plan::kUpdate);
+      for (const LeafFactorTask<T> &k : tasks) {
+        if (k0 >= k.n) continue;
+        const int kb = std::min(NB, k.n - k0);
+        T *Xk = k.X + k0;
+        tr.add(Xk, k.ldx, kb, k.ncols, k.Uinv + (size_t)pi * NB * NB, NB, Xk, k.ldx, kb, false);
+        up.add(k.X + j0, k.ldx, k0 - j0, k.ncols, k.D + j0 + (long long)k0 * k.ldd, k.ldd, Xk,
+               k.ldx, kb, true);
+      }
+      bwd.push_back(std::move(tr));
+      bwd.push_back(std::move(up));
+    }
+    HostStep<T> big = step(Plan::kUpdate);
+    for (const LeafFactorTask<T> &k : tasks) {
+      if (j0 >= k.n) continue;
+      const int obe = std::min(OB, k.n - j0);
+      big.add(k.X, k.ldx, j0, k.ncols, k.D + (long long)j0 * k.ldd, k.ldd, k.X + j0, k.ldx, obe,
+              true);
+    }
+    bwd.push_back(std::move(big));
+  }
+}
+
+// The blocked factorization of every leaf of a tree as uploaded steps.
 template <typename T>
 void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long ldx,
                      int *ipiv, int *perm, bool factor_cols_all, int m, LeafPlan<T> &lp,
@@ -114,9 +276,6 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
   lp.nblocks = cdiv(lp.max_n, OB);
   lp.Linv.ensure((size_t)nleaf * max_panels * NB * NB);
   lp.Uinv.ensure((size_t)nleaf * max_panels * NB * NB);
-  // block-row solves by the inverses of the outer diagonal blocks: in place
-  // on the block's rows, which one GEMM tile row (128) covers (the GEMM
-  // launchers run launches of items of at most 128 rows as 128-row tiles)
   const bool binv = P > 1 && OB <= 128;
   lp.binv = binv;
   if (binv) {
@@ -150,154 +309,25 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
   lp.nleaf = nleaf;
   lp.fwd.clear();
   lp.bwd.clear();
-  // item lists of one GEMM step, filled leaf by leaf
-  struct Acc {
-    std::vector<GemmItem<T, T>> it;
-    std::vector<GemmSeg<T>> sg;
-    void add(T *C, long long ldc, int M, int N, const T *A, long long lda, const T *B,
-             long long ldb, int K, bool inplace) {
-      if (M <= 0 || N <= 0 || K <= 0) return;
-      GemmSeg<T> g{A, B, lda, ldb, K, 0};
-      GemmItem<T, T> i{C, inplace ? C : nullptr, ldc, inplace ? ldc : 0, M, N, (int)sg.size(), 1};
-      sg.push_back(g);
-      it.push_back(i);
+  std::vector<HostStep<T>> fwd, bwd;
+  leaf_steps<T>(tasks, NB, OB, lp.nblocks, binv, fwd, bwd);
+  auto upload = [](const std::vector<HostStep<T>> &src, std::vector<std::unique_ptr<Step>> &dst) {
+    for (const HostStep<T> &h : src) {
+      auto st = std::make_unique<Step>();
+      st->kind = h.kind;
+      st->k0 = h.k0;
+      st->panel = h.panel;
+      st->block = h.block;
+      st->np = h.np;
+      st->a0 = h.a0; st->a1 = h.a1; st->b0 = h.b0; st->b1 = h.b1;
+      st->with_x = h.with_x;
+      if (h.kind == LeafPlan<T>::kTrsm || h.kind == LeafPlan<T>::kUpdate) st->g.set(h.it, h.sg);
+      dst.push_back(std::move(st));
     }
   };
-  auto gemm_step = [&](typename LeafPlan<T>::Kind kind, const Acc &a) {
-    auto st = std::make_unique<Step>();
-    st->kind = kind;
-    st->g.set(a.it, a.sg);
-    return st;
-  };
-  auto laswp_step = [&](int p0, int np, int a0, int a1, int b0, int b1, bool with_x) {
-    auto st = std::make_unique<Step>();
-    st->kind = LeafPlan<T>::kLaswp;
-    st->panel = p0;
-    st->np = np;
-    st->a0 = a0; st->a1 = a1; st->b0 = b0; st->b1 = b1;
-    st->with_x = with_x;
-    return st;
-  };
-  constexpr int kAll = 1 << 30;
-  for (int J = 0; J < lp.nblocks; ++J) {
-    const int j0 = J * OB;
-    // the block's panels: factor, interchange and update inside the block columns
-    for (int p = 0; p < P; ++p) {
-      const int pi = J * P + p, k0 = pi * NB;
-      auto pan = std::make_unique<Step>();
-      pan->kind = LeafPlan<T>::kPanel;
-      pan->k0 = k0;
-      pan->panel = pi;
-      lp.fwd.push_back(std::move(pan));
-      lp.fwd.push_back(laswp_step(pi, 1, j0, k0, k0 + NB, j0 + OB, false));
-      Acc tr, up;
-      for (const LeafFactorTask<T> &k : tasks) {
-        if (k0 >= k.n) continue;
-        const int kb = std::min(NB, k.n - k0);
-        const int N = std::min(j0 + OB, k.n) - (k0 + kb);
-        const int rest = k.n - k0 - kb;
-        const T *Li = k.Linv + (size_t)pi * NB * NB;
-        T *U12 = k.D + k0 + (long long)(k0 + kb) * ldd;
-        tr.add(U12, ldd, kb, N, Li, NB, U12, ldd, kb, false);
-        up.add(k.D + (k0 + kb) + (long long)(k0 + kb) * ldd, ldd, rest, N,
-               k.D + (k0 + kb) + (long long)k0 * ldd, ldd, U12, ldd, kb, true);
-      }
-      lp.fwd.push_back(gemm_step(LeafPlan<T>::kTrsm, tr));
-      lp.fwd.push_back(gemm_step(LeafPlan<T>::kUpdate, up));
-    }
-    // the block's interchanges on the columns left and right of it and on X
-    lp.fwd.push_back(laswp_step(J * P, P, 0, j0, j0 + OB, kAll, true));
-    if (binv) {
-      // block rows: U12 = L11^{-1} A12 on R = (D right of the block | X), one
-      // product with the inverse of the block's unit-lower triangle
-      auto inv = std::make_unique<Step>();
-      inv->kind = LeafPlan<T>::kBlockInv;
-      inv->block = J;
-      lp.fwd.push_back(std::move(inv));
-      Acc tr;
-      for (const LeafFactorTask<T> &k : tasks) {
-        if (j0 >= k.n) continue;
-        const int obe = std::min(OB, k.n - j0);
-        const T *Li = k.LinvB + (size_t)J * OB * OB;
-        T *Dr = k.D + j0 + (long long)(j0 + obe) * ldd;
-        T *Xr = k.X + j0;
-        tr.add(Dr, ldd, obe, k.n - j0 - obe, Li, OB, Dr, ldd, obe, false);
-        tr.add(Xr, ldx, obe, k.ncols, Li, OB, Xr, ldx, obe, false);
-      }
-      lp.fwd.push_back(gemm_step(LeafPlan<T>::kTrsm, tr));
-    }
-    // block rows: U12 = L11^{-1} A12 by panels on R = (D right of the block | X)
-    for (int p = 0; p < (binv ? 0 : P); ++p) {
-      const int pi = J * P + p, k0 = pi * NB;
-      Acc tr, up;
-      for (const LeafFactorTask<T> &k : tasks) {
-        if (k0 >= k.n) continue;
-        const int kb = std::min(NB, k.n - k0);
-        const int obe = std::min(OB, k.n - j0);
-        const int nd = k.n - j0 - obe;           // D columns right of the block
-        const int below = j0 + obe - k0 - kb;    // block rows below this panel
-        const T *Li = k.Linv + (size_t)pi * NB * NB;
-        T *Dr = k.D + k0 + (long long)(j0 + obe) * ldd;
-        T *Xr = k.X + k0;
-        tr.add(Dr, ldd, kb, nd, Li, NB, Dr, ldd, kb, false);
-        tr.add(Xr, ldx, kb, k.ncols, Li, NB, Xr, ldx, kb, false);
-        const T *L = k.D + (k0 + kb) + (long long)k0 * ldd;
-        up.add(Dr + kb, ldd, below, nd, L, ldd, Dr, ldd, kb, true);
-        up.add(Xr + kb, ldx, below, k.ncols, L, ldd, Xr, ldx, kb, true);
-      }
-      lp.fwd.push_back(gemm_step(LeafPlan<T>::kTrsm, tr));
-      lp.fwd.push_back(gemm_step(LeafPlan<T>::kUpdate, up));
-    }
-    // trailing update of depth OB: A22 -= L21 U12 on R, rows below the block
-    Acc big;
-    for (const LeafFactorTask<T> &k : tasks) {
-      if (j0 >= k.n) continue;
-      const int obe = std::min(OB, k.n - j0);
-      const int rest = k.n - j0 - obe;
-      const T *L21 = k.D + (j0 + obe) + (long long)j0 * ldd;
-      big.add(k.D + (j0 + obe) + (long long)(j0 + obe) * ldd, ldd, rest, rest, L21, ldd,
-              k.D + j0 + (long long)(j0 + obe) * ldd, ldd, obe, true);
-      big.add(k.X + (j0 + obe), ldx, rest, k.ncols, L21, ldd, k.X + j0, ldx, obe, true);
-    }
-    lp.fwd.push_back(gemm_step(LeafPlan<T>::kUpdate, big));
-  }
+  upload(fwd, lp.fwd);
+  upload(bwd, lp.bwd);
   lp.fwd_per_block = binv ? 4 * P + 4 : 6 * P + 2;
-  // backward solve on X, last block first
-  for (int J = lp.nblocks - 1; J >= 0; --J) {
-    const int j0 = J * OB;
-    if (binv) {
-      // X[block] = U11^{-1} X[block]: one product with the block's upper inverse
-      Acc tr;
-      for (const LeafFactorTask<T> &k : tasks) {
-        if (j0 >= k.n) continue;
-        const int obe = std::min(OB, k.n - j0);
-        T *Xk = k.X + j0;
-        tr.add(Xk, ldx, obe, k.ncols, k.UinvB + (size_t)J * OB * OB, OB, Xk, ldx, obe, false);
-      }
-      lp.bwd.push_back(gemm_step(LeafPlan<T>::kTrsm, tr));
-    }
-    for (int p = binv ? -1 : P - 1; p >= 0; --p) {
-      const int pi = J * P + p, k0 = pi * NB;
-      Acc tr, up;
-      for (const LeafFactorTask<T> &k : tasks) {
-        if (k0 >= k.n) continue;
-        const int kb = std::min(NB, k.n - k0);
-        T *Xk = k.X + k0;
-        tr.add(Xk, ldx, kb, k.ncols, k.Uinv + (size_t)pi * NB * NB, NB, Xk, ldx, kb, false);
-        up.add(k.X + j0, ldx, k0 - j0, k.ncols, k.D + j0 + (long long)k0 * ldd, ldd, Xk, ldx,
-               kb, true);
-      }
-      lp.bwd.push_back(gemm_step(LeafPlan<T>::kTrsm, tr));
-      lp.bwd.push_back(gemm_step(LeafPlan<T>::kUpdate, up));
-    }
-    Acc big;
-    for (const LeafFactorTask<T> &k : tasks) {
-      if (j0 >= k.n) continue;
-      const int obe = std::min(OB, k.n - j0);
-      big.add(k.X, ldx, j0, k.ncols, k.D + (long long)j0 * ldd, ldd, k.X + j0, ldx, obe, true);
-    }
-    lp.bwd.push_back(gemm_step(LeafPlan<T>::kUpdate, big));
-  }
   lp.bwd_per_block = binv ? 2 : 2 * P + 1;
 }
 
@@ -354,31 +384,12 @@ template <typename T, typename TE>
 void build_path(const Tree &t, const PathSpec<T, TE> &sp, PathPlan<T, TE> &plan, int form) {
   plan.levels.clear();
   plan.factor = sp.factor;
+  plan.nleaf = (int)t.leaves.size();
   const int m = t.nrhs;
-  std::vector<LeafTask<T>> lt;
-  plan.max_n = plan.max_nrhs = 0;
-  for (size_t q = 0; q < t.leaves.size(); ++q) {
-    const Node &n = t.nodes[t.leaves[q]];
-    LeafTask<T> k{};
-    k.D = sp.D + n.row_beg;
-    k.ldd = sp.ldd;
-    k.X = sp.X + n.row_beg;
-    k.ldx = sp.ldx;
-    k.ipiv = sp.ipiv + n.row_beg;
-    k.perm = sp.perm + n.row_beg;
-    k.n = n.nrow;
-    k.nrhs = sp.factor ? n.col_beg + n.ncol : m;
-    k.info_slot = (int)q;
-    plan.max_n = std::max(plan.max_n, k.n);
-    plan.max_nrhs = std::max(plan.max_nrhs, k.nrhs);
-    lt.push_back(k);
-  }
-  plan.nleaf = (int)lt.size();
-  plan.leaf_tasks.upload(lt);
   if (sp.factor) {
     build_leaf_plan<T>(t, sp.D, sp.ldd, sp.X, sp.ldx, sp.ipiv, sp.perm, true, m, plan.leaf,
                        sp.nb_force, sp.ob);
-  } else if (sp.factors) {
+  } else {
     std::vector<LeafFactorTask<T>> at = sp.factors->host_tasks;
     for (size_t q = 0; q < at.size(); ++q) {
       const Node &n = t.nodes[t.leaves[q]];
@@ -599,46 +610,59 @@ struct PhaseScope {
   }
 };
 
+// What a step of the leaf factorization launches over.
+template <typename T>
+struct LeafSet {
+  const LeafFactorTask<T> *tasks;
+  int nleaf, max_n, laswp_cols, nb, ob;
+};
+
+// Enqueues one step (a plan's Step or a HostStep) with its GEMM items on the
+// device (n of them, at most max_m x max_n).
+template <typename T, typename S>
+void run_leaf_step(Profiler &pf, const LeafSet<T> &L, const S &st, const GemmItem<T, T> *items,
+                   const GemmSeg<T> *segs, int n, int max_m, int max_n, int *info,
+                   cudaStream_t s) {
+  using Plan = LeafPlan<T>;
+  const bool solve = st.kind == Plan::kTrsm;
+  switch (st.kind) {
+    case Plan::kPanel: {
+      PhaseScope pp(pf, PH_LEAF_PANEL, s);
+      launch_leaf_panel<T>(L.tasks, L.nleaf, L.max_n, L.nb, st.k0, st.panel, info, s);
+      break;
+    }
+    case Plan::kLaswp: {
+      if (st.a1 <= st.a0 && st.b1 <= st.b0 && !st.with_x) break;  // no columns
+      PhaseScope pp(pf, PH_LEAF_PANEL, s);
+      launch_leaf_laswp<T>(L.tasks, L.nleaf, L.laswp_cols, L.nb, st.panel, st.np, st.a0, st.a1,
+                           st.b0, st.b1, st.with_x, s);
+      break;
+    }
+    case Plan::kBlockInv: {
+      PhaseScope pt(pf, PH_LEAF_TRSM, s);
+      launch_leaf_block_inverse<T>(L.tasks, L.nleaf, L.nb, L.ob, st.block, false, 0, s);
+      break;
+    }
+    case Plan::kTrsm:
+    case Plan::kUpdate: {
+      if (n == 0) break;
+      PhaseScope pg(pf, solve ? PH_LEAF_TRSM : PH_LEAF_UPDATE, s);
+      launch_gemm_items<T, T, T>(items, segs, n, max_m, max_n, false, solve ? T(1) : T(-1),
+                                 solve ? T(0) : T(1), s);
+      break;
+    }
+  }
+}
+
 template <typename T>
 void run_leaf_plan(Profiler &pf, const LeafPlan<T> &lp, int *info, cudaStream_t s) {
-  using Step = typename LeafPlan<T>::Step;
-  auto run_step = [&](const Step &st) {
-    switch (st.kind) {
-      case LeafPlan<T>::kPanel: {
-        PhaseScope pp(pf, PH_LEAF_PANEL, s);
-        launch_leaf_panel<T>(lp.tasks.p, lp.nleaf, lp.max_n, lp.nb, st.k0, st.panel, info, s);
-        break;
-      }
-      case LeafPlan<T>::kLaswp: {
-        if (st.a1 <= st.a0 && st.b1 <= st.b0 && !st.with_x) break;  // no columns
-        PhaseScope pp(pf, PH_LEAF_PANEL, s);
-        launch_leaf_laswp<T>(lp.tasks.p, lp.nleaf, lp.laswp_cols, lp.nb, st.panel, st.np, st.a0,
-                             st.a1, st.b0, st.b1, st.with_x, s);
-        break;
-      }
-      case LeafPlan<T>::kBlockInv: {
-        PhaseScope pt(pf, PH_LEAF_TRSM, s);
-        launch_leaf_block_inverse<T>(lp.tasks.p, lp.nleaf, lp.nb, lp.ob, st.block, false, 0, s);
-        break;
-      }
-      case LeafPlan<T>::kTrsm: {
-        if (st.g.n == 0) break;
-        PhaseScope pt(pf, PH_LEAF_TRSM, s);
-        run_gemm<T, T, T>(st.g, false, T(1), T(0), s);
-        break;
-      }
-      case LeafPlan<T>::kUpdate: {
-        if (st.g.n == 0) break;
-        PhaseScope pu(pf, PH_LEAF_UPDATE, s);
-        run_gemm<T, T, T>(st.g, false, T(-1), T(1), s);
-        break;
-      }
-    }
-  };
+  const LeafSet<T> L{lp.tasks.p, lp.nleaf, lp.max_n, lp.laswp_cols, lp.nb, lp.ob};
   {
     PhaseScope ps(pf, PH_GETRF, s);
     launch_leaf_init<T>(lp.tasks.p, lp.nleaf, info, s);
-    for (const auto &st : lp.fwd) run_step(*st);
+    for (const auto &st : lp.fwd)
+      run_leaf_step<T>(pf, L, *st, st->g.items.p, st->g.segs.p, st->g.n, st->g.max_m, st->g.max_n,
+                       info, s);
     if (lp.binv) {  // the upper block inverses of every block, for the backward solve
       PhaseScope pt(pf, PH_LEAF_TRSM, s);
       launch_leaf_block_inverse<T>(lp.tasks.p, lp.nleaf, lp.nb, lp.ob, 0, true, lp.nblocks, s);
@@ -659,17 +683,13 @@ void run_leaf_plan(Profiler &pf, const LeafPlan<T> &lp, int *info, cudaStream_t 
 template <typename T, typename TE>
 void run_path(Profiler &pf, const PathPlan<T, TE> &plan, int form, int *info, cudaStream_t s,
               int parts = kPathLeaves | kPathLevels, const LevelHook *hook = nullptr) {
-  LeafTask<T> none{};
   if (!(parts & kPathLeaves)) {
   } else if (plan.factor) {
     run_leaf_plan<T>(pf, plan.leaf, info, s);
-  } else if (plan.apply_nb > 0) {
+  } else {
     PhaseScope ps(pf, PH_GETRS, s);
     launch_leaf_apply<T>(plan.apply_tasks.p, plan.nleaf, plan.apply_max_n, plan.apply_max_cols,
                          plan.apply_nb, s);
-  } else {
-    PhaseScope ps(pf, PH_GETRS, s);
-    launch_getrs<T>(plan.leaf_tasks.p, none, plan.nleaf, plan.max_n, plan.max_nrhs, s);
   }
   if (!(parts & kPathLevels)) return;
   if (!plan.factor && plan.sweep_ok && sweep_persistent_enabled()) {
@@ -938,7 +958,6 @@ void merge_paths(const std::vector<const PathPlan<T, TE> *> &src, const std::vec
   dst.levels.clear();
   dst.factor = src[0]->factor;
   dst.nleaf = 0;
-  dst.max_n = dst.max_nrhs = 0;
   dst.apply_nb = dst.apply_max_n = dst.apply_max_cols = 0;
   if (dst.factor) {
     std::vector<const LeafPlan<T> *> lps;
@@ -1030,7 +1049,97 @@ void matvec_launches(Profiler &pf, const MatvecPlan &p, double alpha, double bet
                                             p.ap_max_n, false, alpha, beta, s);
 }
 
+// Bytes of a vector, rounded up so that what follows stays 16-byte aligned.
+template <typename E>
+size_t padded_bytes(const std::vector<E> &v) {
+  return (v.size() * sizeof(E) + 15) & ~size_t(15);
+}
+
 }  // namespace
+
+void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaStream_t s,
+                     const std::function<void *(size_t)> &scratch) {
+  using T = double;
+  using Item = GemmItem<T, T>;
+  using Seg = GemmSeg<T>;
+  if (tasks.empty()) return;
+  int max_n = 0, cols = 0;
+  for (const auto &k : tasks) {
+    max_n = std::max(max_n, k.n);
+    cols = std::max(cols, k.n + k.ncols);
+  }
+  const int NB = leaf_nb<T>(max_n);
+  // Few leaves are bound by the chain of panels and launches, which outer
+  // blocks only lengthen (their triangles' inverses): one leaf of 512 rows and
+  // 592 columns takes 0.93 ms on one level, 1.05 ms with blocks of 64, 1.07 ms
+  // with 128.  Many are bound by the updates' traffic: 512 such leaves (the
+  // FP64 solve at N = 262144) take 17.6 ms on one level, 13.9 ms with blocks
+  // of 128; 16 leaves of 256 rows 0.74 / 0.85 ms, 128 of 469 rows 3.61 / 3.38.
+  const int OB = tasks.size() >= 64 && max_n > 128 ? 128 : NB;
+  const int P = OB / NB, nblocks = cdiv(max_n, OB), np = nblocks * P;
+  const bool binv = P > 1;
+  // per leaf: panel inverses, block inverses, row order, interchange flags
+  const size_t w_inv = (size_t)np * NB * NB, w_blk = binv ? (size_t)nblocks * OB * OB : 0;
+  // (in doubles; even, so that every leaf's inverses start on 16 bytes)
+  const size_t ints = ((size_t)max_n + np + 3) / 4 * 2;
+  const size_t per = 2 * w_inv + 2 * w_blk + ints;
+  double *w = static_cast<double *>(scratch(sizeof(double) * per * tasks.size()));
+  for (size_t q = 0; q < tasks.size(); ++q) {
+    LeafFactorTask<T> &k = tasks[q];
+    double *b = w + q * per;
+    k.Linv = b;
+    k.Uinv = b + w_inv;
+    k.LinvB = binv ? b + 2 * w_inv : nullptr;
+    k.UinvB = binv ? b + 2 * w_inv + w_blk : nullptr;
+    int *ip = reinterpret_cast<int *>(b + 2 * w_inv + 2 * w_blk);
+    if (!k.perm) k.perm = ip;
+    k.swapflag = ip + max_n;
+  }
+  std::vector<HostStep<T>> fwd, bwd;
+  leaf_steps<T>(tasks, NB, OB, nblocks, binv, fwd, bwd);
+  // one block of descriptors: tasks | items | segments
+  std::vector<Item> items;
+  std::vector<Seg> segs;
+  for (auto *v : {&fwd, &bwd})
+    for (const HostStep<T> &h : *v) {
+      items.insert(items.end(), h.it.begin(), h.it.end());
+      segs.insert(segs.end(), h.sg.begin(), h.sg.end());
+    }
+  const size_t o_items = padded_bytes(tasks), o_segs = o_items + padded_bytes(items);
+  std::vector<char> blob(o_segs + padded_bytes(segs));
+  std::memcpy(blob.data(), tasks.data(), sizeof(tasks[0]) * tasks.size());
+  if (!items.empty()) {
+    std::memcpy(blob.data() + o_items, items.data(), sizeof(Item) * items.size());
+    std::memcpy(blob.data() + o_segs, segs.data(), sizeof(Seg) * segs.size());
+  }
+  char *dev = static_cast<char *>(scratch(blob.size()));
+  if (blob.size() <= 64 * 1024)
+    launch_param_copy(dev, blob.data(), blob.size(), s);
+  else
+    HODLR_CUDA_TRY(cudaMemcpyAsync(dev, blob.data(), blob.size(), cudaMemcpyHostToDevice, s));
+  Profiler off;
+  const LeafSet<T> L{reinterpret_cast<const LeafFactorTask<T> *>(dev), (int)tasks.size(), max_n,
+                     cols, NB, OB};
+  const Item *di = reinterpret_cast<const Item *>(dev + o_items);
+  const Seg *ds = reinterpret_cast<const Seg *>(dev + o_segs);
+  auto run = [&](const std::vector<HostStep<T>> &steps) {
+    for (const HostStep<T> &h : steps) {
+      int mm = 0, mn = 0;
+      for (const Item &x : h.it) {
+        mm = std::max(mm, x.M);
+        mn = std::max(mn, x.N);
+      }
+      run_leaf_step<T>(off, L, h, di, ds, (int)h.it.size(), mm, mn, info, s);
+      di += h.it.size();
+      ds += h.sg.size();
+    }
+  };
+  launch_leaf_init<T>(L.tasks, L.nleaf, info, s);
+  run(fwd);
+  if (bwd.empty() || max_n == 0) return;
+  if (binv) launch_leaf_block_inverse<T>(L.tasks, L.nleaf, NB, OB, 0, true, nblocks, s);
+  run(bwd);
+}
 
 void Profiler::begin(int ph, cudaStream_t s, cudaEvent_t &a) {
   HODLR_CUDA_TRY(cudaEventCreate(&a));

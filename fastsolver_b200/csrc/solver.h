@@ -141,8 +141,7 @@ template <typename T, typename TE>
 struct PathPlan {
   bool built = false;
   bool factor = false;  // getrf + node factor (fused) vs getrs + node apply only
-  DevBuf<LeafTask<T>> leaf_tasks;
-  int nleaf = 0, max_n = 0, max_nrhs = 0;
+  int nleaf = 0;
   LeafPlan<T> leaf;     // factor paths: the blocked leaf factorization
   DevBuf<LeafFactorTask<T>> apply_tasks;  // apply paths: the factors' tasks on X
   int apply_nb = 0, apply_max_n = 0, apply_max_cols = 0;
@@ -389,6 +388,13 @@ struct Batch {
     ::hodlr::run_graph(g, !use_graphs || prof.on, s, fn);
   }
 };
+
+// The leaf task body on `tasks` (D, X, ipiv, perm or null, ldd, ldx, n, ncols
+// and info_slot set; n <= 1024) by the blocked factorization of
+// leaf_blocked.cu: `scratch(b)` returns b bytes of device scratch, 256-byte
+// aligned, that live until the work enqueued on s is done.
+void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaStream_t s,
+                     const std::function<void *(size_t)> &scratch);
 
 }  // namespace hodlr
 

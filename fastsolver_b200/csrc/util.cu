@@ -1,4 +1,6 @@
 // util.cu -- element-wise kernels and device-side generators.
+#include <cstring>
+
 #include "common.cuh"
 #include "util.cuh"
 
@@ -195,6 +197,33 @@ __global__ void colratio_batched_kernel(const RatioTask *__restrict__ tasks) {
 // dst[t][e] = sum_q src[t] + q * stride, fixed order (deterministic)
 // (the slot values are loaded four at a time ahead of the adds, which keep
 // the order q = 0, 1, 2, ...: the same sums)
+constexpr int kParamWords = 496;  // 8-byte words per launch, below the 4 KB parameter space
+struct ParamBlock {
+  unsigned long long w[kParamWords];
+};
+__global__ void param_copy_kernel(unsigned long long *dst, int words,
+                                  const __grid_constant__ ParamBlock b) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = b.w[i];
+}
+
+__global__ void identity_kernel(double *A, int n) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x)
+    A[e] = e % (n + 1) == 0 ? 1.0 : 0.0;
+}
+
+__global__ void node_output_kernel(const double *eta, int r0, int r1, int c, double *o0,
+                                   long long l0, double *o1, long long l1, const int *info) {
+  if (*info != 0) return;
+  const int s2 = r0 + r1;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)s2 * c;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(e % s2);
+    const long long j = e / s2;
+    if (i < r0) o0[i + j * l0] = eta[e];
+    else o1[i - r0 + j * l1] = eta[e];
+  }
+}
+
 template <typename T>
 __global__ void sum_slots_kernel(const SumTask<T> *__restrict__ tasks) {
   const SumTask<T> tk = tasks[blockIdx.y];
@@ -431,6 +460,34 @@ template void launch_ew2d_batched<float, double>(const Ew2DTask<float, double> *
 void launch_colratio_batched(const RatioTask *tasks, int ntasks, int max_cols, cudaStream_t s) {
   if (ntasks <= 0 || max_cols <= 0) return;
   colratio_batched_kernel<<<dim3(max_cols, ntasks), 1024, 0, s>>>(tasks);
+  HODLR_LAUNCH_CHECK();
+}
+
+void launch_param_copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  auto *d = static_cast<unsigned long long *>(dst);
+  const char *h = static_cast<const char *>(src);
+  for (size_t left = bytes / 8; left > 0;) {
+    ParamBlock b;
+    const int n = (int)std::min<size_t>(left, kParamWords);
+    std::memcpy(b.w, h, (size_t)n * 8);
+    param_copy_kernel<<<1, 256, 0, s>>>(d, n, b);
+    HODLR_LAUNCH_CHECK();
+    d += n;
+    h += (size_t)n * 8;
+    left -= n;
+  }
+}
+
+void launch_identity(double *A, int n, cudaStream_t s) {
+  identity_kernel<<<(unsigned)cdiv(n * n, kThreads), kThreads, 0, s>>>(A, n);
+  HODLR_LAUNCH_CHECK();
+}
+
+void launch_node_output(const double *eta, int r0, int r1, int c, double *o0, long long l0,
+                        double *o1, long long l1, const int *info, cudaStream_t s) {
+  const long long total = (long long)(r0 + r1) * c;
+  const unsigned grid = (unsigned)std::min<long long>(cdiv<long long>(total, kThreads), 1184);
+  node_output_kernel<<<grid, kThreads, 0, s>>>(eta, r0, r1, c, o0, l0, o1, l1, info);
   HODLR_LAUNCH_CHECK();
 }
 

@@ -31,6 +31,16 @@ void launch_add2d(double *x, long long ldx, const TS *y, long long ldy, long lon
 constexpr int kRatioChunks = 64;
 void launch_colratio(const double *r, long long ldr, const double *b, long long ldb,
                      long long rows, int cols, double *part, double *out, cudaStream_t s);
+// Copies `bytes` (a multiple of 8) of host memory to `dst` through kernel
+// parameters: no staging copy to wait for, and a captured launch keeps the
+// bytes.  For launch descriptors of a few KB.
+void launch_param_copy(void *dst, const void *src, size_t bytes, cudaStream_t s);
+// A (n x n, ld n) = I
+void launch_identity(double *A, int n, cudaStream_t s);
+// Unless *info != 0: o0 (r0 x c, ld l0) and o1 (r1 x c, ld l1) = the rows of
+// eta (r0 + r1 x c, ld r0 + r1).
+void launch_node_output(const double *eta, int r0, int r1, int c, double *o0, long long l0,
+                        double *o1, long long l1, const int *info, cudaStream_t s);
 template <typename T>
 void launch_sum_slots(const SumTask<T> *tasks, int ntasks, long long max_len, cudaStream_t s);
 void launch_scale_cols(double *a, long long lda, long long rows, int cols, const double *s_dev,

@@ -150,3 +150,66 @@ def test_dmma_tiles_elementwise(fs, cuda, k, r, c, odd):
     fs.gemm_reduce(0.75, dev(V, k + odd), dev(X, k + 2 * odd), 0, c, Wg)
     err = np.abs(host(Wg) - (W0 + 0.75 * (V.T @ d)))
     assert (err <= _gemm_bound(k, 0.75 * (np.abs(V).T @ np.abs(d)), np.abs(W0))).all()
+
+
+@pytest.mark.parametrize("count,n,c", [(1, 512, 40), (5, 33, 40), (70, 130, 1), (300, 250, 3)])
+def test_leaf_solve_batched_groups(fs, cuda, count, n, c):
+    """Batched leaves of uneven sizes and leading dimensions, one-level and
+    blocked, and more than one group of them."""
+    import ctypes
+    import torch
+    from fastsolver_b200 import _lib
+
+    class Desc(ctypes.Structure):
+        _fields_ = [("D", ctypes.c_void_p), ("X", ctypes.c_void_p), ("ipiv", ctypes.c_void_p),
+                    ("perm", ctypes.c_void_p), ("ldd", ctypes.c_longlong),
+                    ("ldx", ctypes.c_longlong), ("n", ctypes.c_int), ("nrhs", ctypes.c_int)]
+
+    rng = np.random.default_rng(count + n)
+    arr = (Desc * count)()
+    keep = []
+    for q in range(count):
+        nq = n - q % 7 if n > 7 else n
+        A, B = rng.standard_normal((nq, nq)) + 4 * np.eye(nq), rng.standard_normal((nq, c))
+        D, X, piv, perm = dev(A, n + q % 2), dev(B, n + 1), ivec(nq), ivec(nq)
+        keep.append((A, B, D, X, perm))
+        arr[q] = Desc(D.data_ptr(), X.data_ptr(), piv.data_ptr(), perm.data_ptr() if q % 3 else None,
+                      n + q % 2, n + 1, nq, c)
+        keep[-1] += (piv,)
+    raw = torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8).cuda()
+    info = torch.full((count,), -1, dtype=torch.int32, device="cuda")
+    assert _lib.lib.hodlr_leaf_solve_batched(count, raw.data_ptr(), n, c, info.data_ptr(), None) == 0
+    assert (info == 0).all()
+    for q, (A, B, D, X, perm, piv) in enumerate(keep):
+        nq = A.shape[0]
+        x = np.linalg.solve(A, B)
+        # two backward-stable solves: a few n u of the condition number each
+        assert relerr(host(X), x) <= 20 * nq * np.linalg.cond(A) * 2.0 ** -53
+        if q % 3:
+            LU, p = host(D), perm.cpu().numpy()[:nq]
+            L = np.tril(LU, -1) + np.eye(nq)
+            assert np.abs(L @ np.triu(LU) - A[p]).max() <= 4 * nq * 2.0 ** -53 * (
+                np.abs(L) @ np.abs(np.triu(LU))).max()
+
+
+def test_leaf_solve_captured(fs, cuda):
+    """With a device INFO pointer the call enqueues only: a captured one replays
+    on what the buffers then hold."""
+    import torch
+    rng = np.random.default_rng(8)
+    n, c = 300, 20
+    D, X, piv, info = dev(np.eye(n)), dev(np.ones((n, c))), ivec(n), ivec(1)
+    st = torch.cuda.Stream()
+    fs.leaf_solve(D, X, piv, info=info, stream=st)
+    st.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        fs.leaf_solve(D, X, piv, info=info, stream=torch.cuda.current_stream())
+    for _ in range(2):
+        A, B = rng.standard_normal((n, n)) + 4 * np.eye(n), rng.standard_normal((n, c))
+        D.copy_(dev(A))
+        X.copy_(dev(B))
+        g.replay()
+        torch.cuda.synchronize()
+        assert int(info[0]) == 0
+        assert relerr(host(X), np.linalg.solve(A, B)) <= 20 * n * np.linalg.cond(A) * 2.0 ** -53
