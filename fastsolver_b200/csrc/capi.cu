@@ -359,38 +359,30 @@ static int node_solve_common(int form, int r0, int r1, int c, const double *V0Tu
   if (int e = device_ok()) return e;
   return guarded([&]() -> int {
     cudaStream_t s = as_stream(stream);
-    // scratch: descriptors | S (r0 x r0) | F (r1 x r0) | M (s2 x s2) | eta (s2 x c) | info
+    // scratch: descriptors | F (r1 x r0) | M (s2 x s2) | eta (s2 x c) | info
     using Item = GemmItem<double, double>;
     using Seg = GemmSeg<double>;
     struct Desc {
       NodeTask<double, double> task;
-      Item gram, apply;
-      Seg gseg, aseg[2];
+      Item apply;
+      Seg aseg[2];
     } h{};
     const int s2 = r0 + r1, max_r = std::max(r0, r1);
-    const size_t nR = (size_t)r0 * r0, nF = (size_t)r1 * r0, nM = (size_t)s2 * s2;
+    const size_t nF = (size_t)r1 * r0, nM = (size_t)s2 * s2;
     const size_t nE = (size_t)s2 * std::max(c, 1), head = (sizeof(Desc) + 255) / 256 * 256;
-    StreamScratch scr(head + sizeof(double) * (nR + nF + nM + nE + 1), s);
+    StreamScratch scr(head + sizeof(double) * (nF + nM + nE + 1), s);
     auto *d = static_cast<Desc *>(scr.p);
-    double *S = reinterpret_cast<double *>(static_cast<char *>(scr.p) + head);
-    double *F = S + nR, *M = F + nF, *eta = M + nM;
+    double *F = reinterpret_cast<double *>(static_cast<char *>(scr.p) + head);
+    double *M = F + nF, *eta = M + nM;
     int *info_dev = reinterpret_cast<int *>(eta + nE);
     h.task.W0u = V0Tu0; h.task.W1u = V1Tu1; h.task.ldw0u = ld00; h.task.ldw1u = ld11;
-    h.task.S = S; h.task.F = F; h.task.M = M;
+    h.task.F = F; h.task.M = M;
     h.task.r0 = r0; h.task.r1 = r1; h.task.info_slot = 0;
-    h.gseg = Seg{V1Tu1, V0Tu0, ld11, ld00, r1, 0};
-    h.gram = Item{S, S, r0, r0, r0, r0, 0, 1};
     h.aseg[0] = Seg{M, V0Td0, s2, ld0d, r1, 0};
     h.aseg[1] = Seg{M + (size_t)r1 * s2, V1Td1, s2, ld1d, r0, 0};
     h.apply = Item{eta, nullptr, s2, 0, s2, c, 0, 2};
     launch_param_copy(d, &h, sizeof(h), s);
-    const int max_s = form == 0 ? r0 : s2;
-    if (form == 0 && !node_factor_stages(max_s, max_r)) {
-      // S = I - V1Tu1 V0Tu0 (the dgemm at solver_tasks.cc:261) on the identity
-      launch_identity(S, r0, s);
-      launch_gemm_items<double, double, double>(&d->gram, &d->gseg, 1, r0, r0, false, -1.0, 1.0, s);
-    }
-    launch_node_factor<double, double>(&d->task, 1, max_s, max_r, form, info_dev, s);
+    launch_node_factor<double, double>(&d->task, 1, form == 0 ? r0 : s2, max_r, form, info_dev, s);
     if (c > 0) {
       launch_gemm_items<double, double, double>(&d->apply, d->aseg, 1, s2, c, false, 1.0, 0.0, s);
       // outputs in place unless the system was singular: form 0 writes eta0

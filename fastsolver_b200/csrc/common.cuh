@@ -107,7 +107,6 @@ struct NodeTask {
   const TW *W0u;      // V0^T u0: r1 x r0, ld ldw0u
   const TW *W1u;      // V1^T u1: r0 x r1, ld ldw1u
   long long ldw0u, ldw1u;
-  const double *S;    // form 0: S = I - V1Tu1 V0Tu0 (r0 x r0, ld r0), FP64
   double *F;          // form 0: r1 x r0 FP64 work (-V0Tu0 S^{-1})
   TE *M;              // out: (r0 + r1)^2, ld r0 + r1
   int r0, r1;

@@ -412,8 +412,6 @@ void build_path(const Tree &t, const PathSpec<T, TE> &sp, PathPlan<T, TE> &plan,
     std::vector<GemmSeg<T>> rs, bs;
     std::vector<NodeTask<T, TE>> nt[2];
     std::vector<SumTask<T>> su;
-    std::vector<GemmItem<T, double>> gi;
-    std::vector<GemmSeg<T>> gs;
     std::vector<GemmItem<T, T>> ai;
     std::vector<GemmSeg<T>> as;
     size_t poff = 0, woff = 0, eoff = 0;
@@ -487,33 +485,12 @@ void build_path(const Tree &t, const PathSpec<T, TE> &sp, PathPlan<T, TE> &plan,
       // eta = [eta0; eta1] (s2 x cw, ld s2): eta0 feeds child 0, eta1 child 1
       TE *eta = sp.eta + eoff;
       eoff += (size_t)s2 * cw;
-      k.S = sp.ns->S.p + (size_t)p * sp.ns->rr;
       k.F = sp.ns->F.p + (size_t)p * sp.ns->rr;
       k.M = sp.M + (size_t)p * sp.ns->mm;
       k.info_slot = nleaf + p;
       // the node's form: 1 everywhere when asked for, else 1 inside a Legion leaf
       const int nform = (form == 1 || inside_legion_leaf(t, p, sp.leaf_size)) ? 1 : 0;
       nt[nform].push_back(k);
-      if (sp.factor && nform == 0) {
-        // S = I - V1Tu1 V0Tu0 (r0 x r0, ld r0): the dgemm at solver_tasks.cc:261
-        GemmSeg<T> g{};
-        g.A = k.W1u;
-        g.lda = k.ldw1u;
-        g.B = k.W0u;
-        g.ldb = k.ldw0u;
-        g.K = r1;
-        GemmItem<T, double> it{};
-        it.C = sp.ns->S.p + (size_t)p * sp.ns->rr;
-        it.ldc = r0;
-        it.Cin = sp.ns->ident.p;
-        it.ldcin = t.rank;
-        it.M = it.N = r0;
-        it.seg_begin = (int)gs.size();
-        it.seg_count = 1;
-        gs.push_back(g);
-        gi.push_back(it);
-        L->gram_max = std::max(L->gram_max, r0);
-      }
       const int s = nform == 0 ? r0 : s2;
       L->max_s[nform] = std::max(L->max_s[nform], s);
       L->max_r[nform] = std::max(L->max_r[nform], std::max(r0, r1));
@@ -576,13 +553,9 @@ void build_path(const Tree &t, const PathSpec<T, TE> &sp, PathPlan<T, TE> &plan,
     L->n_red = (int)ri.size();
     L->sums.upload(su);
     L->n_sums = (int)su.size();
-    L->gram_items.upload(gi);
-    L->gram_segs.upload(gs);
-    L->n_gram = (int)gi.size();
     for (int f = 0; f < 2; ++f) {
       L->node_tasks[f].upload(nt[f]);
       L->n_nodes[f] = (int)nt[f].size();
-      L->g_alias[f] = node_g_alias(nt[f]);
     }
     L->ap_items.upload(ai);
     L->ap_segs.upload(as);
@@ -711,15 +684,10 @@ void run_path(Profiler &pf, const PathPlan<T, TE> &plan, int form, int *info, cu
     }
     if (plan.factor) {
       PhaseScope ps(pf, PH_NODE_FACTOR, s);
-      // S = I - V1Tu1 V0Tu0 for the form-0 nodes, unless the node kernel stages
-      // its inputs and forms S itself
-      if (L.n_gram > 0 && !(L.n_nodes[0] > 0 && node_factor_stages(L.max_s[0], L.max_r[0])))
-        launch_gemm_items<T, double, double>(L.gram_items.p, L.gram_segs.p, L.n_gram, L.gram_max,
-                                             L.gram_max, false, -1.0, 1.0, s);
       for (int f = 0; f < 2; ++f)
         if (L.n_nodes[f] > 0)
           launch_node_factor<T, TE>(L.node_tasks[f].p, L.n_nodes[f], L.max_s[f], L.max_r[f], f,
-                                    info, s, L.g_alias[f]);
+                                    info, s);
     }
     {
       PhaseScope ps(pf, PH_NODE_APPLY, s);
@@ -739,13 +707,9 @@ void alloc_node_store(NodeStore &ns, const Tree &t, bool fp64) {
   ns.rr = r * r;
   ns.mm = 4 * r * r;
   const size_t nn = t.nodes.size();
-  ns.S.ensure(nn * ns.rr);
   ns.F.ensure(nn * ns.rr);
   if (fp64) ns.M64.ensure(nn * ns.mm);
   else ns.M32.ensure(nn * ns.mm);
-  std::vector<double> I((size_t)r * r, 0.0);
-  for (int i = 0; i < r; ++i) I[(size_t)i * r + i] = 1.0;
-  ns.ident.upload(I);
 }
 
 void build_matvec(System &S, const double *x, MatvecPlan &mv) {
@@ -981,14 +945,12 @@ void merge_paths(const std::vector<const PathPlan<T, TE> *> &src, const std::vec
   for (size_t j = 0; j < nlev; ++j) {
     auto L = std::make_unique<LevelPlan<T, TE>>();
     ItemAcc<T, T> red, ap, bc;
-    ItemAcc<T, double> gram;
     std::vector<SumTask<T>> su;
     std::vector<NodeTask<T, TE>> nt[2];
     for (size_t k = 0; k < src.size(); ++k) {
       if (j >= src[k]->levels.size()) continue;
       const LevelPlan<T, TE> &S = *src[k]->levels[j];
       red.add(S.red_items.h, S.red_segs.h);
-      gram.add(S.gram_items.h, S.gram_segs.h);
       ap.add(S.ap_items.h, S.ap_segs.h);
       bc.add(S.bc_items.h, S.bc_segs.h);
       su.insert(su.end(), S.sums.h.begin(), S.sums.h.end());
@@ -1004,9 +966,6 @@ void merge_paths(const std::vector<const PathPlan<T, TE> *> &src, const std::vec
       }
     }
     red.store(L->red_items, L->red_segs, L->n_red, L->red_max_m, L->red_max_n);
-    int gm = 0, gn = 0;
-    gram.store(L->gram_items, L->gram_segs, L->n_gram, gm, gn);
-    L->gram_max = std::max(gm, gn);
     ap.store(L->ap_items, L->ap_segs, L->n_ap, L->ap_max_m, L->ap_max_n);
     bc.store(L->bc_items, L->bc_segs, L->n_bc, L->bc_max_m, L->bc_max_n);
     L->sums.upload(su);
@@ -1014,7 +973,6 @@ void merge_paths(const std::vector<const PathPlan<T, TE> *> &src, const std::vec
     for (int f = 0; f < 2; ++f) {
       L->node_tasks[f].upload(nt[f]);
       L->n_nodes[f] = (int)nt[f].size();
-      L->g_alias[f] = node_g_alias(nt[f]);
     }
     dst.levels.push_back(std::move(L));
   }

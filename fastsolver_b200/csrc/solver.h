@@ -51,9 +51,7 @@ struct DevBuf {
 
 // Per-node factorization data kept for solves with the same factors.
 struct NodeStore {
-  DevBuf<double> S;      // form 0, per node: S = I - V1Tu1 V0Tu0 (r x r)
   DevBuf<double> F;      // per node: r x r FP64 work of the factor kernel
-  DevBuf<double> ident;  // r x r identity (the I of S)
   DevBuf<double> M64;    // per node: (2r)^2 solve matrix, FP64 path
   DevBuf<float> M32;     // per node: (2r)^2 solve matrix, mixed path
   int rr = 0, mm = 0;
@@ -69,14 +67,10 @@ struct LevelPlan {
   int n_sums = 0;
   int sum_max_slots = 0;             // most partial slots of one of its tasks
   long long sum_max_len = 0;
-  DevBuf<GemmItem<T, double>> gram_items;  // S = I - V1Tu1 V0Tu0, FP64 result
-  DevBuf<GemmSeg<T>> gram_segs;
-  int n_gram = 0, gram_max = 0;
   // node factorization tasks by form (0: r x r reduced system, 1: 2r x 2r
   // permuted Schur system of the nodes inside a Legion leaf)
   DevBuf<NodeTask<T, TE>> node_tasks[2];
   int n_nodes[2] = {0, 0}, max_s[2] = {0, 0}, max_r[2] = {0, 0};
-  bool g_alias[2] = {false, false};  // node_g_alias of each form's tasks
   DevBuf<GemmItem<T, T>> ap_items;  // [eta0; eta1] = M [V0Td0; V1Td1] per node
   DevBuf<GemmSeg<T>> ap_segs;
   int n_ap = 0, ap_max_m = 0, ap_max_n = 0;

@@ -206,11 +206,6 @@ __global__ void param_copy_kernel(unsigned long long *dst, int words,
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = b.w[i];
 }
 
-__global__ void identity_kernel(double *A, int n) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * n; e += gridDim.x * blockDim.x)
-    A[e] = e % (n + 1) == 0 ? 1.0 : 0.0;
-}
-
 __global__ void node_output_kernel(const double *eta, int r0, int r1, int c, double *o0,
                                    long long l0, double *o1, long long l1, const int *info) {
   if (*info != 0) return;
@@ -476,11 +471,6 @@ void launch_param_copy(void *dst, const void *src, size_t bytes, cudaStream_t s)
     h += (size_t)n * 8;
     left -= n;
   }
-}
-
-void launch_identity(double *A, int n, cudaStream_t s) {
-  identity_kernel<<<(unsigned)cdiv(n * n, kThreads), kThreads, 0, s>>>(A, n);
-  HODLR_LAUNCH_CHECK();
 }
 
 void launch_node_output(const double *eta, int r0, int r1, int c, double *o0, long long l0,

@@ -35,8 +35,6 @@ void launch_colratio(const double *r, long long ldr, const double *b, long long 
 // parameters: no staging copy to wait for, and a captured launch keeps the
 // bytes.  For launch descriptors of a few KB.
 void launch_param_copy(void *dst, const void *src, size_t bytes, cudaStream_t s);
-// A (n x n, ld n) = I
-void launch_identity(double *A, int n, cudaStream_t s);
 // Unless *info != 0: o0 (r0 x c, ld l0) and o1 (r1 x c, ld l1) = the rows of
 // eta (r0 + r1 x c, ld r0 + r1).
 void launch_node_output(const double *eta, int r0, int r1, int c, double *o0, long long l0,

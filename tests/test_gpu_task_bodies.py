@@ -213,3 +213,26 @@ def test_leaf_solve_captured(fs, cuda):
         torch.cuda.synchronize()
         assert int(info[0]) == 0
         assert relerr(host(X), np.linalg.solve(A, B)) <= 20 * n * np.linalg.cond(A) * 2.0 ** -53
+
+
+@pytest.mark.parametrize("r0,r1", [(1, 1), (8, 8), (9, 9), (16, 17), (40, 25), (56, 56), (57, 57),
+                                   (72, 72), (73, 73), (104, 104), (105, 105), (144, 144),
+                                   (10, 300), (144, 9)])
+def test_node_elimination_edges(fs, cuda, r0, r1):
+    """The blocked elimination at the edges of its panels, tiles and shared-memory
+    layouts, unequal ranks included, with pivots off the diagonal."""
+    rng = np.random.default_rng(r0 * 1000 + r1)
+    V0Tu0 = rng.standard_normal((r1, r0)) / np.sqrt(r1)
+    V1Tu1 = 2 * rng.standard_normal((r0, r1)) / np.sqrt(r0)
+    V0Td0, V1Td1 = rng.standard_normal((r1, 5)), rng.standard_normal((r0, 5))
+    S = np.eye(r0) - V1Tu1 @ V0Tu0
+    eta0 = np.linalg.solve(S, V1Td1 - V1Tu1 @ V0Td0)
+    eta1 = V0Td0 - V0Tu0 @ eta0
+    g = [dev(V0Tu0, r1 + 1), dev(V1Tu1), dev(V0Td0, r1 + 2), dev(V1Td1)]
+    assert fs.node_lu_solve(*g) == 0
+    # the solve and the products around it: a few s u of S's condition number
+    # and of the blocks' norms each
+    lim = 50 * max(r0, r1) * np.linalg.cond(S) * 2.0 ** -53 * (
+        1 + np.linalg.norm(V0Tu0, 2)) ** 2 * (1 + np.linalg.norm(V1Tu1, 2)) ** 2
+    assert np.linalg.norm(host(g[3]) - eta0) <= lim * np.linalg.norm(eta0)
+    assert np.linalg.norm(host(g[2]) - eta1) <= lim * np.linalg.norm(eta1)
