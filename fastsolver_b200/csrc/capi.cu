@@ -1103,7 +1103,7 @@ int tune_search(hodlr_schedule &best, double &best_ms, int precision,
   if (!(best_ms >= 0)) return HODLR_ERR_CUDA;
   const std::vector<int> rows = {256, 512, 1024, 2048};
   const std::vector<int> ob32 = {0, 128, 256};
-  const std::vector<int> ob64 = {0, 64, 128};
+  const std::vector<int> ob64 = {0, 16, 64, 128};  // 0: by the leaves, 16: one level
   const int nfields = 4;
   for (int pass = 0; pass < 2; ++pass) {
     bool changed = false;

@@ -725,62 +725,114 @@ __global__ void __launch_bounds__(kApplyThreads)
 
 // ---- inverses of the outer diagonal blocks (two-level factorization).
 //
-// For outer block J (rows / columns j0 .. j0 + obe of a leaf) with panels
-// p = 0 .. P-1 of width NB, the unit-lower block inverse is built by block
-// forward substitution from the panels' own inverses Linv_p:
-//   X[p][p] = Linv_p,  X[p][q] = -Linv_p sum_{s=q}^{p-1} L[p][s] X[s][q]  (q < p),
-// and the upper one by block back substitution from Uinv_p:
-//   Y[p][p] = Uinv_p,  Y[q][p] = -Uinv_q sum_{s=q+1}^{p} U[q][s] Y[s][p]  (q < p).
-// Lower: CTA (256 threads) = one leaf, for one block; upper: one leaf x one
-// block, all blocks in one launch.  The ob x ob result, an NB x NB product
-// tile and one staged NB x NB block of D live in shared memory (padded leading
-// dimensions; the panel inverses are read from global memory), so two CTAs
-// fit on an SM; products are 16 x 16 thread grids of R x R outputs.
+// Outer block J (rows / columns j0 .. j0 + obe of a leaf) starts as its
+// panels' own inverses on the diagonal and L's (U's) blocks beside them, and
+// diagonal blocks are merged pairwise, in place:
+//   lower: X21 = -X22 (L21 X11),    upper: Y12 = -Y11 (U12 Y22),
+// with blocks of NB, 2 NB, ... columns: two products and two barriers per
+// doubling.  One CTA per leaf, block and triangle; the matrix (column-major,
+// padded), and the inner product live in shared memory, FP64 products on the
+// DMMA pipe, tiles skipping the triangular operand's zeros.  Built panel by
+// panel, with P (P - 1) (P + 1) / 3 products one after another and a staged
+// block for each, the five launches of an FP64 solve (N = 262144, 512 leaves
+// of 512 rows, blocks of four panels) took 1.64 ms; this takes 0.8 ms.  FP32
+// blocks are two panels, two products either way (0.47 -> 0.45 ms).
 constexpr int kInvThreads = 256;
 
-template <typename T, int NB>
-__device__ inline void tile_mm(const T *A, int lda, const T *B, int ldb, T *C, int ldc,
-                               T alpha, bool acc) {
-  constexpr int R = NB / 16;
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  T c[R][R];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int q = 0; q < R; ++q) c[r][q] = T(0);
-#pragma unroll 4
-  for (int k = 0; k < NB; ++k) {
-    T a[R], b[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = A[(ty * R + r) + k * lda];
-#pragma unroll
-    for (int q = 0; q < R; ++q) b[q] = B[k + (tx * R + q) * ldb];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if constexpr (sizeof(T) == 4 && R % 2 == 0) {
-        // packed two-wide FMAs, each half rounded as c + a b
-#pragma unroll
-        for (int q = 0; q < R; q += 2) {
-          const float2 v = __ffma2_rn(make_float2(a[r], a[r]), make_float2(b[q], b[q + 1]),
-                                      make_float2(c[r][q], c[r][q + 1]));
-          c[r][q] = v.x;
-          c[r][q + 1] = v.y;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < R; ++q) c[r][q] += a[r] * b[q];
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      T *cp = C + (ty * R + r) + (tx * R + q) * ldc;
-      *cp = (acc ? *cp : T(0)) + alpha * c[r][q];
-    }
+// Which operand of a product is triangular: the lower or the upper one of A or
+// B.  A tile of C skips the k for which that operand's rows (columns) of the
+// tile are zero.
+enum Tri { kLowerA, kUpperA, kLowerB, kUpperB };
+template <Tri TRI>
+__device__ inline void tri_range(int m0, int m1, int n0, int n1, int K, int &k0, int &k1) {
+  k0 = TRI == kUpperA ? m0 : TRI == kLowerB ? n0 : 0;
+  k1 = TRI == kLowerA ? m1 : TRI == kUpperB ? n1 : K;
 }
 
+// C (M x N) = alpha A B (A M x K, B K x N), all column-major in shared memory,
+// M and N multiples of 16 R
+template <int R, Tri TRI>
+__device__ inline void block_mm(int M, int N, int K, const float *A, int lda, const float *B,
+                                int ldb, float *C, int ldc, float alpha) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  for (int m0 = 0; m0 < M; m0 += 16 * R)
+    for (int n0 = 0; n0 < N; n0 += 16 * R) {
+      int k0, k1;
+      tri_range<TRI>(m0, m0 + 16 * R, n0, n0 + 16 * R, K, k0, k1);
+      float c[R][R];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < R; ++q) c[r][q] = 0.f;
+#pragma unroll 8
+      for (int k = k0; k < k1; ++k) {
+        float a[R], b[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[r] = A[(m0 + ty * R + r) + k * lda];
+#pragma unroll
+        for (int q = 0; q < R; ++q) b[q] = B[k + (n0 + tx * R + q) * ldb];
+        // packed two-wide FMAs, each half rounded as c + a b
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int q = 0; q < R; q += 2) {
+            const float2 v = __ffma2_rn(make_float2(a[r], a[r]), make_float2(b[q], b[q + 1]),
+                                        make_float2(c[r][q], c[r][q + 1]));
+            c[r][q] = v.x;
+            c[r][q + 1] = v.y;
+          }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          C[(m0 + ty * R + r) + (n0 + tx * R + q) * ldc] = alpha * c[r][q];
+    }
+}
+template <Tri TRI>
+__device__ inline void block_product(int M, int N, int K, const float *A, int lda, const float *B,
+                                     int ldb, float *C, int ldc, float alpha) {
+  block_mm<2, TRI>(M, N, K, A, lda, B, ldb, C, ldc, alpha);
+}
+// FP64: warps take 16 x 8 tiles in turn (fragments as in gemm_dmma.cu)
+template <Tri TRI>
+__device__ inline void block_product(int M, int N, int K, const double *A, int lda,
+                                     const double *B, int ldb, double *C, int ldc, double alpha) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int tm = M / 16, tn = N / 8;
+  for (int tile = threadIdx.x >> 5; tile < tm * tn; tile += kInvThreads / 32) {
+    const int m = (tile % tm) * 16 + g, n = (tile / tm) * 8;
+    int k0, k1;
+    tri_range<TRI>(m - g, m - g + 16, n, n + 8, K, k0, k1);
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int k = k0 + t; k < k1; k += 4) {
+      const double a0 = A[m + k * lda], a1 = A[m + 8 + k * lda], b = B[k + (n + g) * ldb];
+      asm volatile(
+          "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+          "{%0, %1, %2, %3};\n"
+          : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+          : "d"(a0), "d"(a1), "d"(b));
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      C[m + (v >> 1) * 8 + (n + 2 * t + (v & 1)) * ldc] = alpha * c[v];
+  }
+}
+
+// column strides: FP64 4 modulo 16 (conflict-free DMMA fragments), FP32 odd
+template <typename T>
+__host__ __device__ constexpr int inv_ld(int n) { return n + (sizeof(T) == 8 ? 4 : 1); }
+// largest inner product: a block of half the next power of two's size
+template <typename T>
+__host__ __device__ inline size_t inv_words(int ob, int nb) {
+  int h = nb;
+  while (2 * h < ob) h *= 2;
+  return (size_t)inv_ld<T>(ob) * ob + (size_t)inv_ld<T>(h) * h;
+}
+
+// grid (leaf, 1): block J0's lower triangle; grid (leaf, blocks) with upper:
+// every block's upper one
 template <typename T, int NB>
 __global__ void __launch_bounds__(kInvThreads)
     leaf_block_inverse_kernel(const LeafFactorTask<T> *__restrict__ tasks, int ob, int J0,
@@ -792,69 +844,58 @@ __global__ void __launch_bounds__(kInvThreads)
   const int j0 = J * ob;
   if (j0 >= n) return;
   const int obe = min(ob, n - j0);
-  const int P = (obe + NB - 1) / NB;
-  const int pbase = j0 / NB;
-  constexpr int LT = NB + 1;  // padded ld of the NB x NB tiles
-  const int LX = ob + 1;      // padded ld of the block inverse
-  T *X = reinterpret_cast<T *>(smem_raw);  // ob x ob
-  T *Tt = X + (size_t)ob * LX;             // product tile
-  T *Bs = Tt + NB * LT;                    // staged L / U block of D
+  const int pbase = j0 / NB, live = (obe + NB - 1) / NB * NB;  // whole panels
+  const int ld = inv_ld<T>(ob);
+  T *X = reinterpret_cast<T *>(smem_raw);
+  T *Tt = X + (size_t)ld * ob;
   const int tid = threadIdx.x;
-  for (int e = tid; e < ob * ob; e += kInvThreads) X[(e % ob) + (e / ob) * LX] = T(0);
-  // panel pi's inverse (NB x NB, ld NB; identity beyond the leaf), read from
-  // global memory (L1 / L2) by the products
-  auto inv_of = [&](int pi) { return (upper ? tk.Uinv : tk.Linv) + (size_t)pi * NB * NB; };
-  // stage the NB x NB block of D at block panels (pr, pc), zero outside the block
-  auto stage_d = [&](int pr, int pc) {
-    for (int e = tid; e < NB * NB; e += kInvThreads) {
-      const int i = e % NB, c = e / NB;
-      const int gi = pr * NB + i, gc = pc * NB + c;
-      Bs[i + c * LT] = (gi < obe && gc < obe) ? tk.D[(j0 + gi) + (long long)(j0 + gc) * tk.ldd] : T(0);
+  const T *inv = upper ? tk.Uinv : tk.Linv;
+  const int lane = tid & 31, warp = tid >> 5;
+  // a warp per column, every load unconditional (an address inside the leaf's
+  // own data), so that a thread's loads overlap
+  const T *safe = tk.D + j0 + (long long)j0 * tk.ldd;
+  constexpr int kAhead = sizeof(T) == 8 ? 2 : 4;  // columns whose loads overlap
+#pragma unroll kAhead
+  for (int c = warp; c < ob; c += kInvThreads / 32) {
+    const int pc = c / NB;
+    const T *dcol = tk.D + j0 + (long long)(j0 + c) * tk.ldd;
+    const T *icol = inv + (size_t)(pbase + pc) * NB * NB + (c - pc * NB) * NB - pc * NB;
+    T v[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = lane + 32 * q, pi = i / NB;
+      const bool diag = pi == pc;
+      in[q] = diag ? i < live : (upper ? pi < pc : pi > pc) && i < obe && c < obe;
+      v[q] = *(in[q] ? (diag ? icol : dcol) + i : safe);
     }
-  };
-  auto Xb = [&](int pr, int pc) { return X + pr * NB + (size_t)pc * NB * LX; };
-  for (int p = 0; p < P; ++p) {
-    __syncthreads();
-    {
-      const T *src = inv_of(pbase + p);
-      for (int e = tid; e < NB * NB; e += kInvThreads) {
-        const int i = e % NB, c = e / NB;
-        Xb(p, p)[i + c * LX] = src[e];
-      }
-    }
-    if (!upper) {
-      for (int q = 0; q < p; ++q) {
-        // Tt = sum_{s=q}^{p-1} L[p][s] X[s][q];  X[p][q] = -Linv_p Tt
-        for (int s2 = q; s2 < p; ++s2) {
-          __syncthreads();
-          stage_d(p, s2);
-          __syncthreads();
-          tile_mm<T, NB>(Bs, LT, Xb(s2, q), LX, Tt, LT, T(1), s2 > q);
-        }
-        __syncthreads();
-        tile_mm<T, NB>(inv_of(pbase + p), NB, Tt, LT, Xb(p, q), LX, T(-1), false);
-      }
-    } else {
-      for (int q = p - 1; q >= 0; --q) {
-        // Tt = sum_{s=q+1}^{p} U[q][s] Y[s][p];  Y[q][p] = -Uinv_q Tt
-        for (int s2 = q + 1; s2 <= p; ++s2) {
-          __syncthreads();
-          stage_d(q, s2);
-          __syncthreads();
-          tile_mm<T, NB>(Bs, LT, Xb(s2, p), LX, Tt, LT, T(1), s2 > q + 1);
-        }
-        __syncthreads();
-        tile_mm<T, NB>(inv_of(pbase + q), NB, Tt, LT, Xb(q, p), LX, T(-1), false);
-      }
-    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (lane + 32 * q < ob) X[lane + 32 * q + c * ld] = in[q] ? v[q] : T(0);
   }
   __syncthreads();
+  for (int b = NB; b < ob; b *= 2) {
+    for (int o = 0; o + b < live; o += 2 * b) {
+      const int h = min(b, ob - o - b);  // the second block's size
+      T *X11 = X + o + o * ld, *X22 = X + (o + b) + (o + b) * ld;
+      T *off = upper ? X + o + (o + b) * ld : X + (o + b) + o * ld;
+      const int lt = inv_ld<T>(upper ? b : h);
+      if (upper) block_product<kUpperB>(b, h, h, off, ld, X22, ld, Tt, lt, T(1));
+      else block_product<kLowerB>(h, b, b, off, ld, X11, ld, Tt, lt, T(1));
+      __syncthreads();
+      if (upper) block_product<kUpperA>(b, h, b, X11, ld, Tt, lt, off, ld, T(-1));
+      else block_product<kLowerA>(h, b, h, X22, ld, Tt, lt, off, ld, T(-1));
+      __syncthreads();
+    }
+  }
   // zero outside the leaf's part of the block (rows / columns >= obe)
   T *dst = (upper ? tk.UinvB : tk.LinvB) + (size_t)J * ob * ob;
-  for (int e = tid; e < ob * ob; e += kInvThreads) {
-    const int i = e % ob, c = e / ob;
-    dst[e] = (i < obe && c < obe) ? X[i + c * LX] : T(0);
-  }
+  for (int c = warp; c < ob; c += kInvThreads / 32)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = lane + 32 * q;
+      if (i < ob) dst[i + c * ob] = (i < obe && c < obe) ? X[i + c * ld] : T(0);
+    }
 }
 
 }  // namespace
@@ -940,14 +981,14 @@ void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb
   if (count <= 0 || (upper && nblocks <= 0)) return;
   if (ob > 128 || ob % nb) throw CudaError{cudaErrorInvalidValue};
   dim3 grid(count, upper ? nblocks : 1);
-  auto go = [&](auto kern, int NBv) {
-    const size_t smem = ((size_t)ob * (ob + 1) + 2 * (size_t)NBv * (NBv + 1)) * sizeof(T);
+  const size_t smem = inv_words<T>(ob, nb) * sizeof(T);
+  auto go = [&](auto kern) {
     raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
     kern<<<grid, kInvThreads, smem, s>>>(tasks, ob, J, upper ? 1 : 0);
   };
-  if (nb == 64) go(leaf_block_inverse_kernel<T, 64>, 64);
-  else if (nb == 32) go(leaf_block_inverse_kernel<T, 32>, 32);
-  else if (nb == 16) go(leaf_block_inverse_kernel<T, 16>, 16);
+  if (nb == 64) go(leaf_block_inverse_kernel<T, 64>);
+  else if (nb == 32) go(leaf_block_inverse_kernel<T, 32>);
+  else if (nb == 16) go(leaf_block_inverse_kernel<T, 16>);
   else throw CudaError{cudaErrorInvalidValue};
   HODLR_LAUNCH_CHECK();
 }

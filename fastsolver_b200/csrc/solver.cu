@@ -258,6 +258,19 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
   }
 }
 
+// FP64 outer block width without a request, for `rows` rows in leaves of at
+// most max_n: 0 (one level) or 128.  Blocks of 128 read and write the trailing
+// matrix a quarter as often but lengthen the chain of launches by the blocks'
+// triangular inverses, so they pay once a factorization is bound by its
+// updates: whole FP64 solves on one level / with 128, in ms: 4096 rows in
+// leaves of 256 0.60 / 0.65, of 512 0.96 / 1.04; 12000 rows in leaves of 375
+// 1.25 / 1.29; 16384 rows of 512 1.68 / 1.62; 60001 rows of 469 4.18 / 3.76;
+// 262144 rows of 512 27.5 / 22.0.  Above 512 rows panels are 16 wide, and one
+// level means 16-deep updates: 6000 rows in leaves of 750 2.02 / 1.89.
+int leaf_ob_auto64(long long rows, int max_n) {
+  return max_n > 512 || (max_n > 128 && rows * max_n >= (8 << 20)) ? 128 : 0;
+}
+
 // The blocked factorization of every leaf of a tree as uploaded steps.
 template <typename T>
 void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long ldx,
@@ -1027,13 +1040,7 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
     cols = std::max(cols, k.n + k.ncols);
   }
   const int NB = leaf_nb<T>(max_n);
-  // Few leaves are bound by the chain of panels and launches, which outer
-  // blocks only lengthen (their triangles' inverses): one leaf of 512 rows and
-  // 592 columns takes 0.93 ms on one level, 1.05 ms with blocks of 64, 1.07 ms
-  // with 128.  Many are bound by the updates' traffic: 512 such leaves (the
-  // FP64 solve at N = 262144) take 17.6 ms on one level, 13.9 ms with blocks
-  // of 128; 16 leaves of 256 rows 0.74 / 0.85 ms, 128 of 469 rows 3.61 / 3.38.
-  const int OB = tasks.size() >= 64 && max_n > 128 ? 128 : NB;
+  const int OB = std::max(NB, leaf_ob_auto64((long long)tasks.size() * max_n, max_n));
   const int P = OB / NB, nblocks = cdiv(max_n, OB), np = nblocks * P;
   const bool binv = P > 1;
   // per leaf: panel inverses, block inverses, row order, interchange flags
@@ -1181,7 +1188,8 @@ void System::ensure_fp64() {
     f.X = X64.p; f.ldx = N; f.Usrc = X64.p; f.ldu = N;
     f.D = DLU64.p; f.ldd = N; f.ipiv = ipiv64.p; f.perm = perm64.p;
     f.V = V.p; f.ldv = N; f.part = part64.p; f.wfin = wfin64.p; f.eta = eta64.p; f.M = ns64.M64.p; f.ns = &ns64;
-    f.factor = true; f.red_chunk = red_chunk; f.bc_chunk = bc_chunk; f.ob = ob64;
+    f.factor = true; f.red_chunk = red_chunk; f.bc_chunk = bc_chunk;
+    f.ob = ob64 > 0 ? ob64 : leaf_ob_auto64(N, nmax);
     f.leaf_size = leaf_size;
     build_path(tree, f, fused64[form], form);
     PathSpec<double, double> a = f;

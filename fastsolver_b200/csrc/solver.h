@@ -291,7 +291,8 @@ struct System {
   int factored_form = 0;
   int red_chunk = 512;
   int nb32 = 0;  // forced FP32 leaf panel width (0: by the largest leaf)
-  int ob32 = 128, ob64 = 0;  // leaf outer block width per path (0: one level)
+  // leaf outer block width per path (0: FP32 one level, FP64 by the leaves)
+  int ob32 = 128, ob64 = 0;
   int bc_chunk = 512;
   int n_info = 0;
   // granularity of the reference's tasks (HodlrMatrix leafSize): the FP64
