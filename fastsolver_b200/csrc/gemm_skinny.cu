@@ -207,21 +207,34 @@ __device__ inline void dmma(double (&c)[4], double a0, double a1, double b) {
       : "d"(a0), "d"(a1), "d"(b));
 }
 
-constexpr int kDmmaRows = 512;          // NN: 8 warps x 64 rows
-constexpr int kDmmaKT = 8;              // NN: K per stage
 constexpr int kDmmaStages = 3;
-constexpr int kDmmaAP = kDmmaRows + 8;  // padded k-row stride (doubles)
 
 // NN: C (M x N) = beta Cin + alpha sum_s A_s B_s, A_s column-major; one CTA
-// per (item, 512-row block, block of 8 NT8 columns)
-template <int NT8>
-__global__ void __launch_bounds__(kSkThreads, 2)
+// per (item, ROWS-row block, block of 8 NT8 columns), KT k-values per stage.
+// Large: 512 rows, 8 warps, 8 k (133 KB of A in flight per SM); small: 128
+// rows, 4 warps, 16 k, for launches that leave SMs without a large block and
+// for items that fill a quarter of one.
+template <bool SMALL>
+struct NnDmma {
+  static constexpr int ROWS = SMALL ? 128 : 512, THREADS = SMALL ? 128 : 256;
+  static constexpr int KT = SMALL ? 16 : 8;
+  static constexpr int AP = ROWS + 8;  // padded k-row stride (doubles)
+  static constexpr size_t smem(int ncs) {
+    return (size_t)kDmmaStages * KT * (AP + ncs + 4) * sizeof(double);
+  }
+};
+
+template <int NT8, bool SMALL>
+__global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
     skinny_nn_dmma_kernel(const GemmItem<double, double> *__restrict__ items,
                           const GemmSeg<double> *__restrict__ segs, double alpha, double beta) {
-  constexpr int KT = kDmmaKT, ROWS = kDmmaRows, AP = kDmmaAP, NCS = 8 * NT8;
+  using Cfg = NnDmma<SMALL>;
+  constexpr int KT = Cfg::KT, ROWS = Cfg::ROWS, AP = Cfg::AP, THREADS = Cfg::THREADS;
+  constexpr int NCS = 8 * NT8, BP = NCS + 4;  // conflict-free fragments
+  constexpr int MT = ROWS / (THREADS / 32) / 16;  // 16-row fragments per warp
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *As = reinterpret_cast<double *>(smem_raw);      // [stage][KT][AP]
-  double *Bs = As + (size_t)kDmmaStages * KT * AP;         // [stage][KT][NCS]
+  double *Bs = As + (size_t)kDmmaStages * KT * AP;         // [stage][KT][BP]
   const GemmItem<double, double> it = items[blockIdx.x];
   const int row0 = blockIdx.y * ROWS;
   const int n0 = blockIdx.z * NCS;  // column block of this CTA
@@ -234,10 +247,10 @@ __global__ void __launch_bounds__(kSkThreads, 2)
     if (p.valid) {
       const GemmSeg<double> &sg = p.sg;
       double *a = As + (size_t)st * KT * AP;
-      double *b = Bs + (size_t)st * KT * NCS;
+      double *b = Bs + (size_t)st * KT * BP;
       const double *abase = sg.A + row0 + (long long)p.k0 * sg.lda;
       const bool vec = ((reinterpret_cast<uintptr_t>(abase) & 15) == 0) && ((sg.lda & 1) == 0);
-      for (int e = tid; e < KT * (ROWS / 2); e += kSkThreads) {
+      for (int e = tid; e < KT * (ROWS / 2); e += THREADS) {
         const int k = e / (ROWS / 2), rv = e % (ROWS / 2);
         const int r = row0 + 2 * rv;
         const bool kin = p.k0 + k < sg.K;
@@ -253,19 +266,19 @@ __global__ void __launch_bounds__(kSkThreads, 2)
           }
         }
       }
-      for (int e = tid; e < KT * NCS; e += kSkThreads) {
+      for (int e = tid; e < KT * NCS; e += THREADS) {
         const int k = e % KT, n = e / KT;
         const bool ok = (p.k0 + k < sg.K) && n < N;
-        cpa(b + k * NCS + n, ok ? sg.B + (p.k0 + k) + (long long)(n0 + n) * sg.ldb : sg.B, 8,
+        cpa(b + k * BP + n, ok ? sg.B + (p.k0 + k) + (long long)(n0 + n) * sg.ldb : sg.B, 8,
             ok);
       }
     }
     cpa_commit();
   };
 
-  double acc[4][NT8][4];
+  double acc[MT][NT8][4];
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
@@ -279,7 +292,7 @@ __global__ void __launch_bounds__(kSkThreads, 2)
     if (ld.valid) ld.next(KT);
   }
   int st = 0, lst = kDmmaStages - 1;
-  const int wrow = warp * 64;
+  const int wrow = warp * 16 * MT;
   while (cp.valid) {
     load(ld, lst);
     if (ld.valid) ld.next(KT);
@@ -287,15 +300,15 @@ __global__ void __launch_bounds__(kSkThreads, 2)
     cpa_wait<kDmmaStages - 1>();
     __syncthreads();
     const double *a = As + (size_t)st * KT * AP;
-    const double *b = Bs + (size_t)st * KT * NCS;
+    const double *b = Bs + (size_t)st * KT * BP;
 #pragma unroll
     for (int ks = 0; ks < KT; ks += 4) {
       const double *ak = a + (ks + t) * AP + wrow + g;
       double bv[NT8];
 #pragma unroll
-      for (int nt = 0; nt < NT8; ++nt) bv[nt] = b[(ks + t) * NCS + nt * 8 + g];
+      for (int nt = 0; nt < NT8; ++nt) bv[nt] = b[(ks + t) * BP + nt * 8 + g];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         const double a0 = ak[mt * 16], a1 = ak[mt * 16 + 8];
 #pragma unroll
         for (int nt = 0; nt < NT8; ++nt) dmma(acc[mt][nt], a0, a1, bv[nt]);
@@ -309,7 +322,7 @@ __global__ void __launch_bounds__(kSkThreads, 2)
   // per 16-row fragment: its Cin values before its stores (C may alias Cin,
   // so a load after a store would wait for it)
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {
+  for (int mt = 0; mt < MT; ++mt) {
     double cin[NT8][4];
 #pragma unroll
     for (int nt = 0; nt < NT8; ++nt)
@@ -449,15 +462,27 @@ void launch_skinny(const GemmItem<T, T> *items, const GemmSeg<T> *segs, int nite
       dim3 grid(nitems, cdiv(max_m, 64), cdiv(max_n, 16));
       skinny_tn_dmma_kernel<<<grid, kTNThreads, smem, s>>>(items, segs, alpha, beta);
     } else {
-      // 8 columns per CTA when every item has at most 8, else 16-column blocks
-      dim3 grid(nitems, cdiv(max_m, kDmmaRows), max_n <= 8 ? 1 : cdiv(max_n, 16));
-      auto go = [&](auto kern, int ncs) {
-        const size_t smem = (size_t)kDmmaStages * kDmmaKT * (kDmmaAP + ncs) * sizeof(double);
+      // 8 columns per CTA when every item has at most 8, else 16-column blocks.
+      // Small blocks where large ones would leave SMs idle or mostly empty:
+      // matvec of 4096 rows 88 -> 36 us, 60001 rows 201 -> 184 us, node
+      // products of 128 rows 233 -> 129 us per solve; above, large ones stream
+      // faster (131072 rows: 346 us large, 404 us small).
+      const int nz = max_n <= 8 ? 1 : cdiv(max_n, 16);
+      const bool small = max_m <= 256 || (long long)nitems * cdiv(max_m, 512) * nz < 148;
+      auto go = [&](auto kern, auto cfg) {
+        using Cfg = decltype(cfg);
+        const size_t smem = Cfg::smem(max_n <= 8 ? 8 : 16);
         raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-        kern<<<grid, kSkThreads, smem, s>>>(items, segs, alpha, beta);
+        const dim3 grid(nitems, cdiv(max_m, Cfg::ROWS), nz);
+        kern<<<grid, Cfg::THREADS, smem, s>>>(items, segs, alpha, beta);
       };
-      if (max_n <= 8) go(skinny_nn_dmma_kernel<1>, 8);
-      else go(skinny_nn_dmma_kernel<2>, 16);
+      if (max_n <= 8) {
+        if (small) go(skinny_nn_dmma_kernel<1, true>, NnDmma<true>{});
+        else go(skinny_nn_dmma_kernel<1, false>, NnDmma<false>{});
+      } else {
+        if (small) go(skinny_nn_dmma_kernel<2, true>, NnDmma<true>{});
+        else go(skinny_nn_dmma_kernel<2, false>, NnDmma<false>{});
+      }
     }
     HODLR_LAUNCH_CHECK();
     return;

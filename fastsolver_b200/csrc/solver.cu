@@ -729,7 +729,9 @@ void build_matvec(System &S, const double *x, MatvecPlan &mv) {
   const Tree &t = S.tree;
   const int m = S.m;
   const long long N = S.N;
-  const int chunk = 1024;
+  // rows per split-K slot: 1024, fewer where that would leave the reduce of
+  // all levels below four CTAs per SM
+  const int chunk = std::min(1024, std::max(128, (int)((long long)N * t.max_depth / 592 / 64 * 64)));
   std::vector<GemmItem<double, double>> ri, ai;
   std::vector<GemmSeg<double>> rs, as;
   std::vector<SumTask<double>> su;

@@ -128,7 +128,11 @@ def _gemm_bound(K, AB, C):
 @pytest.mark.parametrize("k,r,c", [(1, 1, 33), (31, 5, 63), (32, 16, 64), (33, 17, 65),
                                    (63, 15, 100), (64, 32, 128), (65, 33, 129), (127, 48, 40),
                                    (128, 100, 190), (129, 31, 64), (1000, 64, 257),
-                                   (20011, 37, 129)])
+                                   (20011, 37, 129),
+                                   # at most 32 columns: blocks of 128 rows, and of 512
+                                   (1, 1, 1), (127, 15, 8), (128, 16, 9), (129, 17, 16),
+                                   (513, 64, 17), (5000, 33, 32), (75777, 20, 8),
+                                   (80001, 33, 16), (76000, 7, 31)])
 def test_dmma_tiles_elementwise(fs, cuda, k, r, c, odd):
     """The FP64 tile GEMM at the edges of its tiles and K stages, with operands
     on and off 16-byte boundaries, C added in front (beta = 1) and behind."""
