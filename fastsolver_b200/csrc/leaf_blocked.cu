@@ -23,6 +23,7 @@
 // the batched GEMM engine (gemm_simt.cu), one launch per step for all leaves.
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "leaf_blocked.cuh"
@@ -32,6 +33,17 @@ namespace hodlr {
 namespace {
 
 constexpr int kThreads = 256;
+
+// Fragments of m16n8k4 .f64 (g = lane / 4, t = lane % 4): A a0 = A[g][t],
+// a1 = A[g + 8][t]; B b = B[t][g]; C c0..c3 = C[g][2t], C[g][2t + 1],
+// C[g + 8][2t], C[g + 8][2t + 1].
+__device__ inline void dmma64(double (&c)[4], double a0, double a1, double b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+      "{%0, %1, %2, %3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b));
+}
 
 // 16-byte vector of T
 template <typename T>
@@ -543,184 +555,327 @@ __global__ void leaf_init_kernel(const LeafFactorTask<T> *__restrict__ tasks, in
 
 // ---- apply: X <- U^{-1} L^{-1} P X with the stored blocked factors.
 //
-// One CTA per (column chunk of MC right-hand sides, leaf).  The chunk of P X
-// lives in shared memory (row-major, padded rows); per panel the diagonal
-// block is applied with its explicit inverse and the rest of the block
-// column of L (forward) or U (backward) is streamed from global memory once,
-// coalesced along the rows, into register accumulators.  Every element of the
-// factors is read once per chunk.
-constexpr int kApplyThreads = 512;
-
+// One CTA per (column chunk of MC right-hand sides, leaf).  The rows of P X
+// live in registers for the whole solve; panel by panel (forward with L, then
+// backward with U) the owners of the panel's rows publish them, they are
+// multiplied by the diagonal block's explicit inverse, and every row still to
+// come subtracts its row of the block column, streamed from global memory
+// once, coalesced along the rows and loaded ahead of the barriers it does not
+// depend on.  Two barriers per panel.
+//
+// FP32: rows in threads, two per thread, so that a broadcast read of the
+// panel's values feeds two rows (with the chunk of X in shared memory and one
+// row per thread the kernel was bound by those reads).  FP64: 16-row tiles in
+// warps on the DMMA pipe.
+//   FP32, 512 leaves of 512 rows, 16 columns: 407 -> 320 us;
+//   FP32, 128 leaves of 512 rows, 8 columns: 172 -> 78 us;
+//   FP64, 256 leaves of 512 rows, 16 columns: 587 -> 251 us.
 
 // Stage the diagonal-block inverse Ainv (kb x kb, column-major, ld nb) into
 // shared memory `As` (ld kb + 1) with asynchronous copies (one commit group).
-template <typename T>
-__device__ inline void stage_inverse(const T *__restrict__ Ainv, int nb, int kb, T *As) {
+__device__ inline void stage_inverse(const float *__restrict__ Ainv, int nb, int kb, float *As) {
   const int lds = kb + 1;
-  for (int e = threadIdx.x; e < kb * kb; e += kApplyThreads) {
+  for (int e = threadIdx.x; e < kb * kb; e += blockDim.x) {
     const int i = e % kb, k = e / kb;
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(As + i + k * lds));
-    if (sizeof(T) == 8)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(Ainv + i + (size_t)k * nb));
-    else
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(Ainv + i + (size_t)k * nb));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(Ainv + i + (size_t)k * nb));
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// y (kb x MC in shared memory, row stride XS) <- As y, As the staged inverse.
-template <typename T, int MC, int XS>
-__device__ inline void apply_diag(T *y, int kb, const T *As) {
-  constexpr int VW = 16 / sizeof(T);
-  constexpr int NV = MC / VW;
-  constexpr int OUT = (64 * NV + kApplyThreads - 1) / kApplyThreads;
-  using V = typename Vec16<T>::V;
-  const int tid = threadIdx.x;
-  const int lds = kb + 1;
-  T acc[OUT][VW];
-#pragma unroll
-  for (int o = 0; o < OUT; ++o) {
-#pragma unroll
-    for (int v = 0; v < VW; ++v) acc[o][v] = T(0);
-    const int e = tid + o * kApplyThreads;
-    if (e < kb * NV) {
-      const int i = e % kb, jv = e / kb;
-#pragma unroll 8
-      for (int k = 0; k < kb; ++k) {
-        const T a = As[i + k * lds];
-        const V x = *reinterpret_cast<const V *>(y + k * XS + jv * VW);
-        const T *xp = reinterpret_cast<const T *>(&x);
-#pragma unroll
-        for (int v = 0; v < VW; ++v) acc[o][v] += a * xp[v];
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int o = 0; o < OUT; ++o) {
-    const int e = tid + o * kApplyThreads;
-    if (e < kb * NV) {
-      const int i = e % kb, jv = e / kb;
-      V out;
-      T *op = reinterpret_cast<T *>(&out);
-#pragma unroll
-      for (int v = 0; v < VW; ++v) op[v] = acc[o][v];
-      *reinterpret_cast<V *>(y + i * XS + jv * VW) = out;
-    }
-  }
-  __syncthreads();
+constexpr int kApplyNB = 64;  // largest panel
+
+template <int MC>
+constexpr int apply32_smem() {
+  return (2 * kApplyNB * (kApplyNB + 1) + 2 * kApplyNB * MC) * (int)sizeof(float);
 }
 
-// dst (rows x MC, shared, stride XS) -= A (rows x kb, global, ld lda) y (kb x MC, shared)
-template <typename T, int MC, int XS>
-__device__ inline void apply_block(const T *__restrict__ A, long long lda, T *dst, int rows,
-                                   const T *y, int kb) {
-  constexpr int VW = 16 / sizeof(T);
-  using V = typename Vec16<T>::V;
-  for (int i = threadIdx.x; i < rows; i += kApplyThreads) {
-    T acc[MC];
-#pragma unroll
-    for (int j = 0; j < MC; j += VW) {
-      const V x = *reinterpret_cast<const V *>(dst + i * XS + j);
-      const T *xp = reinterpret_cast<const T *>(&x);
-#pragma unroll
-      for (int v = 0; v < VW; ++v) acc[j + v] = xp[v];
-    }
-    const T *Ai = A + i;
-    constexpr int LB = sizeof(T) == 4 ? 64 : 32;  // loads in flight per row
-    int k = 0;
-    for (; k + LB <= kb; k += LB) {
-      T a[LB];
-#pragma unroll
-      for (int u = 0; u < LB; ++u) a[u] = Ai[(long long)(k + u) * lda];
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const T *yk = y + (k + u) * XS;
-#pragma unroll
-        for (int j = 0; j < MC; j += VW) {
-          const V x = *reinterpret_cast<const V *>(yk + j);
-          const T *xp = reinterpret_cast<const T *>(&x);
-#pragma unroll
-          for (int v = 0; v < VW; ++v) acc[j + v] -= a[u] * xp[v];
-        }
-      }
-    }
-    for (; k < kb; ++k) {
-      const T a = Ai[(long long)k * lda];
-      const T *yk = y + k * XS;
-#pragma unroll
-      for (int j = 0; j < MC; ++j) acc[j] -= a * yk[j];
-    }
-#pragma unroll
-    for (int j = 0; j < MC; j += VW) {
-      V out;
-      T *op = reinterpret_cast<T *>(&out);
-#pragma unroll
-      for (int v = 0; v < VW; ++v) op[v] = acc[j + v];
-      *reinterpret_cast<V *>(dst + i * XS + j) = out;
-    }
-  }
-}
-
-template <typename T, int MC>
-__global__ void __launch_bounds__(kApplyThreads)
-    leaf_apply_kernel(const LeafFactorTask<T> *__restrict__ tasks, int nb, int max_n) {
+// THREADS >= half the rows of the largest leaf, a multiple of 4 kApplyNB
+template <int MC, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
+    leaf_apply32_kernel(const LeafFactorTask<float> *__restrict__ tasks, int nb) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int XS = MC + 16 / sizeof(T);  // padded row stride (16 bytes)
-  const LeafFactorTask<T> tk = tasks[blockIdx.y];
+  constexpr int CH = MC == 32 ? 8 : 16;            // k-values of a row loaded ahead
+  constexpr int CG = THREADS / kApplyNB, CW = MC / CG;  // column groups of the diagonal product
+  static_assert(CW * CG == MC, "whole column groups");
+  const LeafFactorTask<float> tk = tasks[blockIdx.y];
   const int n = tk.n;
   const int c0 = blockIdx.x * MC;
   if (c0 >= tk.ncols || n <= 0) return;
   const int mc = min(MC, tk.ncols - c0);
   const int tid = threadIdx.x;
-  T *xs = reinterpret_cast<T *>(smem_raw);
-  T *As0 = xs + (size_t)max_n * XS;  // two staged inverses, nb x (nb + 1) each
-  const int as_stride = nb * (nb + 1);
-  T *X = tk.X + (long long)c0 * tk.ldx;
+  float *As0 = reinterpret_cast<float *>(smem_raw);  // two staged inverses
+  const int as_stride = kApplyNB * (kApplyNB + 1);
+  float *ys = As0 + 2 * as_stride;                   // the panel's rows, published
+  float *yo = ys + kApplyNB * MC;                    // ... times the inverse
+  float *X = tk.X + (long long)c0 * tk.ldx;
   const long long ldx = tk.ldx, ldd = tk.ldd;
   const int np = (n + nb - 1) / nb;
-  // step s < np: forward panel s with Linv_s; step s >= np: backward panel
-  // 2 np - 1 - s with its Uinv.  The next step's inverse is staged while the
-  // current one is applied.
-  auto inv_of = [&](int st, int &k0, int &kb) -> const T * {
-    const int p = st < np ? st : 2 * np - 1 - st;
-    k0 = p * nb;
-    kb = min(nb, n - k0);
-    return (st < np ? tk.Linv : tk.Uinv) + (size_t)p * nb * nb;
+  // step st < np: forward panel st with Linv; else backward panel 2 np - 1 - st
+  // with Uinv
+  auto panel_of = [&](int st) { return st < np ? st : 2 * np - 1 - st; };
+  auto stage = [&](int st) {
+    const int p = panel_of(st), kb = min(nb, n - p * nb);
+    stage_inverse((st < np ? tk.Linv : tk.Uinv) + (size_t)p * nb * nb, nb, kb,
+                  As0 + (st & 1) * as_stride);
   };
-  {
-    int k0, kb;
-    const T *inv0 = inv_of(0, k0, kb);
-    stage_inverse<T>(inv0, nb, kb, As0);
-  }
-  for (int e = tid; e < n * MC; e += kApplyThreads) {
-    const int i = e % n, j = e / n;
-    xs[i * XS + j] = j < mc ? X[tk.perm[i] + (long long)j * ldx] : T(0);
+  stage(0);
+  float acc[2][MC];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float *x = X + tk.perm[min(tid + q * THREADS, n - 1)];
+#pragma unroll
+    for (int j = 0; j < MC; ++j) acc[q][j] = x[(long long)min(j, mc - 1) * ldx];
   }
   for (int st = 0; st < 2 * np; ++st) {
-    int k0, kb;
-    inv_of(st, k0, kb);
+    const int p = panel_of(st), k0 = p * nb, kb = min(nb, n - k0);
+    const bool fwd = st < np;
+    bool act[2];
+    const float *ap[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = tid + q * THREADS;
+      act[q] = fwd ? i >= k0 + kb && i < n : i < k0;
+      ap[q] = tk.D + min(i, n - 1) + (long long)k0 * ldd;
+    }
+    // the first k-values of this thread's rows, before the barriers
+    float a[2][CH];
+    auto load = [&](int q, int kk) {  // the next CH columns (the last one repeated)
+      const float *x = ap[q] + (long long)kk * ldd;
+      if (kk + CH <= kb) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u, x += ldd) a[q][u] = *x;
+      } else {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+          a[q][u] = *x;
+          if (kk + u + 1 < kb) x += ldd;
+        }
+      }
+    };
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (act[q]) load(q, 0);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = tid + q * THREADS - k0;
+      if (i >= 0 && i < kb) {
+#pragma unroll
+        for (int j = 0; j < MC; j += 4)
+          *reinterpret_cast<float4 *>(ys + i * MC + j) =
+              make_float4(acc[q][j], acc[q][j + 1], acc[q][j + 2], acc[q][j + 3]);
+      }
+    }
     if (st + 1 < 2 * np) {
-      int k1, kb1;
-      const T *inv1 = inv_of(st + 1, k1, kb1);
-      stage_inverse<T>(inv1, nb, kb1, As0 + ((st + 1) & 1) * as_stride);
+      stage(st + 1);
       asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
-    __syncthreads();  // this step's inverse and the previous step's updates visible
-    apply_diag<T, MC, XS>(xs + k0 * XS, kb, As0 + (st & 1) * as_stride);
-    if (st < np)
-      apply_block<T, MC, XS>(tk.D + (k0 + kb) + (long long)k0 * ldd, ldd, xs + (k0 + kb) * XS,
-                             n - k0 - kb, xs + k0 * XS, kb);
-    else
-      apply_block<T, MC, XS>(tk.D + (long long)k0 * ldd, ldd, xs, k0, xs + k0 * XS, kb);
     __syncthreads();
+    {
+      const int i = tid % kApplyNB, cg = tid / kApplyNB * CW;
+      const float *As = As0 + (st & 1) * as_stride;
+      float o[CW];
+#pragma unroll
+      for (int c = 0; c < CW; ++c) o[c] = 0.f;
+      if (i < kb) {
+#pragma unroll 8
+        for (int k = 0; k < kb; ++k) {
+          const float m = As[i + k * (kb + 1)];
+#pragma unroll
+          for (int c = 0; c < CW; ++c) o[c] += m * ys[k * MC + cg + c];
+        }
+      }
+      if (i < nb) {
+#pragma unroll
+        for (int c = 0; c < CW; ++c) yo[i * MC + cg + c] = o[c];  // 0 beyond kb
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = tid + q * THREADS - k0;
+      if (i >= 0 && i < kb) {
+#pragma unroll
+        for (int j = 0; j < MC; ++j) acc[q][j] = yo[i * MC + j];
+      }
+    }
+    // rows still to come: acc -= D[row][panel] y
+    auto update = [&](auto Q0, auto Q1) {
+      for (int kk = 0; kk < kb; kk += CH) {
+        float c[2][CH];
+#pragma unroll
+        for (int q = Q0; q < Q1; ++q)
+#pragma unroll
+          for (int u = 0; u < CH; ++u) c[q][u] = a[q][u];
+        if (kk + CH < kb) {
+#pragma unroll
+          for (int q = Q0; q < Q1; ++q) load(q, kk + CH);
+        }
+        const float *y = yo + kk * MC;
+#pragma unroll
+        for (int u = 0; u < CH; ++u)
+#pragma unroll
+          for (int j = 0; j < MC; j += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(y + u * MC + j);
+#pragma unroll
+            for (int q = Q0; q < Q1; ++q) {
+              acc[q][j] -= c[q][u] * v.x;
+              acc[q][j + 1] -= c[q][u] * v.y;
+              acc[q][j + 2] -= c[q][u] * v.z;
+              acc[q][j + 3] -= c[q][u] * v.w;
+            }
+          }
+      }
+    };
+    using std::integral_constant;
+    if (act[0] && act[1]) update(integral_constant<int, 0>{}, integral_constant<int, 2>{});
+    else if (act[0]) update(integral_constant<int, 0>{}, integral_constant<int, 1>{});
+    else if (act[1]) update(integral_constant<int, 1>{}, integral_constant<int, 2>{});
   }
-  for (int e = tid; e < n * mc; e += kApplyThreads) {
-    const int i = e % n, j = e / n;
-    X[i + (long long)j * ldx] = xs[i * XS + j];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int i = tid + q * THREADS;
+    if (i < n) {
+#pragma unroll
+      for (int j = 0; j < MC; ++j)
+        if (j < mc) X[i + (long long)j * ldx] = acc[q][j];
+    }
   }
+}
+
+// NT blocks of 8 columns; TPW 16-row tiles per warp (16 warps: 256 TPW rows)
+template <int NT, int TPW>
+__global__ void __launch_bounds__(512, 1)
+    leaf_apply64_kernel(const LeafFactorTask<double> *__restrict__ tasks, int nb) {
+  constexpr int MC = 8 * NT, XS = MC + 4, NBM = 32;  // row stride: conflict-free fragments
+  __shared__ __align__(16) double ys[NBM * XS], yo[NBM * XS];
+  const LeafFactorTask<double> tk = tasks[blockIdx.y];
+  const int n = tk.n;
+  const int c0 = blockIdx.x * MC;
+  if (c0 >= tk.ncols || n <= 0) return;
+  const int mc = min(MC, tk.ncols - c0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  double *X = tk.X + (long long)c0 * tk.ldx;
+  const long long ldx = tk.ldx, ldd = tk.ldd;
+  const int np = (n + nb - 1) / nb;
+  // tile j of this warp: rows 16 (warp + 16 j) .. + 15
+  double acc[TPW][NT][4];
+#pragma unroll
+  for (int j = 0; j < TPW; ++j)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const double *x = X + tk.perm[min(16 * (warp + 16 * j) + g + (v >> 1) * 8, n - 1)];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+        acc[j][nt][v] = x[(long long)min(8 * nt + 2 * t + (v & 1), mc - 1) * ldx];
+    }
+  for (int st = 0; st < 2 * np; ++st) {
+    const bool fwd = st < np;
+    const int p = fwd ? st : 2 * np - 1 - st, k0 = p * nb, kb = min(nb, n - k0);
+    const int t0 = k0 / 16, t1 = t0 + nb / 16;  // the panel's tiles
+    auto active = [&](int j) {
+      const int tile = warp + 16 * j;
+      return fwd ? tile >= t1 && 16 * tile < n : tile < t0;
+    };
+    // fragments of 16 of the panel's columns in the tile's rows; columns beyond
+    // the leaf meet zero rows of y
+    double a[4][2];
+    auto load = [&](int j, int h) {
+      const int r = 16 * (warp + 16 * j) + g;
+      const double *p0 = tk.D + min(r, n - 1), *p1 = tk.D + min(r + 8, n - 1);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const long long o = (long long)min(k0 + 16 * h + 4 * k + t, n - 1) * ldd;
+        a[k][0] = p0[o];
+        a[k][1] = p1[o];
+      }
+    };
+    // the diagonal product's tile of this warp, then the first block tile
+    const int dm = warp % 2, dn = warp / 2;  // 16-row and 8-column block
+    const bool diag = dm < nb / 16 && dn < NT;
+    double d[NBM / 4][2];
+    if (diag) {
+      const double *inv = (fwd ? tk.Linv : tk.Uinv) + (size_t)p * nb * nb + 16 * dm + g;
+#pragma unroll
+      for (int k = 0; k < NBM / 4; ++k) {
+        if (4 * k >= nb) break;
+        d[k][0] = inv[(4 * k + t) * nb];
+        d[k][1] = inv[(4 * k + t) * nb + 8];
+      }
+    }
+    int first = TPW;
+#pragma unroll
+    for (int j = TPW - 1; j >= 0; --j)
+      if (active(j)) first = j;
+    if (first < TPW) load(first, 0);
+#pragma unroll
+    for (int j = 0; j < TPW; ++j) {
+      const int tile = warp + 16 * j;
+      if (tile >= t0 && tile < t1) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int r = 16 * (tile - t0) + g + (v >> 1) * 8;
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            ys[r * XS + 8 * nt + 2 * t + (v & 1)] = r < kb ? acc[j][nt][v] : 0.0;
+        }
+      }
+    }
+    __syncthreads();
+    if (diag) {
+      double c[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < NBM / 4; ++k) {
+        if (4 * k >= nb) break;
+        dmma64(c, d[k][0], d[k][1], ys[(4 * k + t) * XS + 8 * dn + g]);
+      }
+#pragma unroll
+      for (int v = 0; v < 4; ++v)  // kept negated: the updates subtract
+        yo[(16 * dm + g + (v >> 1) * 8) * XS + 8 * dn + 2 * t + (v & 1)] = -c[v];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < TPW; ++j) {
+      const int tile = warp + 16 * j;
+      if (tile >= t0 && tile < t1) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            acc[j][nt][v] =
+                -yo[(16 * (tile - t0) + g + (v >> 1) * 8) * XS + 8 * nt + 2 * t + (v & 1)];
+      }
+      if (active(j)) {
+        for (int h = 0; h < nb / 16; ++h) {
+          double c[4][2];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) { c[k][0] = a[k][0]; c[k][1] = a[k][1]; }
+          if (16 * (h + 1) < nb) load(j, h + 1);
+          else if (j + 1 < TPW && active(j + 1)) load(j + 1, 0);
+          const double *y = yo + (16 * h + t) * XS + g;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+              dmma64(acc[j][nt], c[k][0], c[k][1], y[4 * k * XS + 8 * nt]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < TPW; ++j)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int r = 16 * (warp + 16 * j) + g + (v >> 1) * 8;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int c = 8 * nt + 2 * t + (v & 1);
+        if (r < n && c < mc) X[r + (long long)c * ldx] = acc[j][nt][v];
+      }
+    }
 }
 
 // ---- inverses of the outer diagonal blocks (two-level factorization).
@@ -794,7 +949,7 @@ __device__ inline void block_product(int M, int N, int K, const float *A, int ld
                                      int ldb, float *C, int ldc, float alpha) {
   block_mm<2, TRI>(M, N, K, A, lda, B, ldb, C, ldc, alpha);
 }
-// FP64: warps take 16 x 8 tiles in turn (fragments as in gemm_dmma.cu)
+// FP64: warps take 16 x 8 tiles in turn
 template <Tri TRI>
 __device__ inline void block_product(int M, int N, int K, const double *A, int lda,
                                      const double *B, int ldb, double *C, int ldc, double alpha) {
@@ -808,11 +963,7 @@ __device__ inline void block_product(int M, int N, int K, const double *A, int l
 #pragma unroll 4
     for (int k = k0 + t; k < k1; k += 4) {
       const double a0 = A[m + k * lda], a1 = A[m + 8 + k * lda], b = B[k + (n + g) * ldb];
-      asm volatile(
-          "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-          "{%0, %1, %2, %3};\n"
-          : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-          : "d"(a0), "d"(a1), "d"(b));
+      dmma64(c, a0, a1, b);
     }
 #pragma unroll
     for (int v = 0; v < 4; ++v)
@@ -951,28 +1102,34 @@ void launch_leaf_laswp(const LeafFactorTask<T> *tasks, int count, int max_cols, 
   HODLR_LAUNCH_CHECK();
 }
 
-template <typename T, int MC>
-void launch_leaf_apply_mc(const LeafFactorTask<T> *tasks, int count, int max_n, int max_cols,
-                          int nb, cudaStream_t s) {
-  constexpr int XS = MC + 16 / sizeof(T);
-  const size_t smem = ((size_t)max_n * XS + 2 * (size_t)nb * (nb + 1)) * sizeof(T);
-  raise_smem_limit(reinterpret_cast<const void *>(leaf_apply_kernel<T, MC>), smem);
-  dim3 grid(cdiv(max_cols, MC), count);
-  leaf_apply_kernel<T, MC><<<grid, kApplyThreads, smem, s>>>(tasks, nb, max_n);
-  HODLR_LAUNCH_CHECK();
-}
-
 template <typename T>
 void launch_leaf_apply(const LeafFactorTask<T> *tasks, int count, int max_n, int max_cols, int nb,
                        cudaStream_t s) {
   if (count <= 0 || max_cols <= 0 || max_n <= 0) return;
-  if (nb > 64) throw CudaError{cudaErrorInvalidValue};
-  // the chunk of P X is max_n x (MC + pad) in shared memory (<= 160 KB)
-  const bool wide_ok = ((size_t)max_n * (32 + 16 / sizeof(T)) + 2 * (size_t)nb * (nb + 1)) *
-                           sizeof(T) <= 180 * 1024;
-  if (max_cols <= 8) launch_leaf_apply_mc<T, 8>(tasks, count, max_n, max_cols, nb, s);
-  else if (max_cols <= 16 || !wide_ok) launch_leaf_apply_mc<T, 16>(tasks, count, max_n, max_cols, nb, s);
-  else launch_leaf_apply_mc<T, 32>(tasks, count, max_n, max_cols, nb, s);
+  if (max_n > 1024 || nb > (sizeof(T) == 8 ? 32 : kApplyNB) || nb % 16)
+    throw CudaError{cudaErrorInvalidValue};
+  auto go = [&](auto kern, int mc, int threads, size_t smem) {
+    raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+    kern<<<dim3(cdiv(max_cols, mc), count), threads, smem, s>>>(tasks, nb);
+  };
+  const bool tall = max_n > 512;
+  if constexpr (sizeof(T) == 4) {
+    auto pick = [&](auto mcv) {
+      constexpr int MC = decltype(mcv)::value;
+      if (tall) go(leaf_apply32_kernel<MC, 512>, MC, 512, apply32_smem<MC>());
+      else go(leaf_apply32_kernel<MC, 256>, MC, 256, apply32_smem<MC>());
+    };
+    if (max_cols <= 8) pick(std::integral_constant<int, 8>{});
+    else if (max_cols <= 16) pick(std::integral_constant<int, 16>{});
+    else pick(std::integral_constant<int, 32>{});
+  } else {
+    // 32 columns of a leaf above 512 rows do not fit the registers
+    if (max_cols <= 8) tall ? go(leaf_apply64_kernel<1, 4>, 8, 512, 0) : go(leaf_apply64_kernel<1, 2>, 8, 512, 0);
+    else if (tall) go(leaf_apply64_kernel<2, 4>, 16, 512, 0);
+    else if (max_cols <= 16) go(leaf_apply64_kernel<2, 2>, 16, 512, 0);
+    else go(leaf_apply64_kernel<4, 2>, 32, 512, 0);
+  }
+  HODLR_LAUNCH_CHECK();
 }
 
 template <typename T>

@@ -259,3 +259,27 @@ def test_leaf_panels_ties_and_zero_columns(fs, cuda, n):
         with pytest.raises(fs.HodlrError) as e:
             call()
         assert e.value.status == j + 1
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 17, 32, 40])
+@pytest.mark.parametrize("n", [3, 16, 17, 33, 64, 130, 255, 500, 512, 513, 700, 1024])
+def test_leaf_apply_edges(fs, cuda, n, m):
+    """Kept leaf factors applied to new right-hand sides, at the edges of the
+    panels, tiles and column chunks, FP64 and FP32."""
+    rng = np.random.default_rng(100 * n + m)
+    A = rng.standard_normal((n, n)) / np.sqrt(n) + 2 * np.eye(n)
+    A = A[rng.permutation(n)]
+    h = fs.HodlrMatrix(m, n, 1, 1024).create_tree()
+    h.set_matrix(A)
+    h.set_rhs(rng.standard_normal((n, m)))
+    solver = fs.FastSolver()
+    cond = np.linalg.cond(A)
+    for prec, u in ((fs.PREC_FP64, 2.0 ** -53), (fs.PREC_MIXED, 2.0 ** -15)):
+        # FP32 factors carry the split-BF16 updates' 2^-15 per product
+        solver.factor(h, prec)
+        B = rng.standard_normal((n, m))
+        h.set_rhs(B)
+        solver.solve(h)
+        X = np.linalg.solve(A, B)
+        lim = (50 * n if prec == fs.PREC_FP64 else 8) * cond * u
+        assert np.linalg.norm(h.solution() - X) <= lim * np.linalg.norm(X)
