@@ -3,19 +3,11 @@
 // HODLR matvec (gemm_simt.cu routes them here).
 //
 // These products stream a tall operand (V, U or D, up to a few GB per
-// launch) against a small one, so they are bound by HBM bandwidth; both
-// kernels keep every operand tile in flight with a 3-stage cp.async ring
-// (16-byte copies where the addresses allow) and compute from shared memory.
-//
-//   skinny_nn2: C (M x N) = beta Cin + alpha sum_s A_s B_s, A_s M x K column-
-//               major.  CTA = 512 rows of one item, thread = 2 rows, 2 x NC
-//               accumulators; per K tile the A tile (KT x 512) and the B tile
-//               (KT x NC) land in shared memory.
-//   skinny_tn2: C (M x N) = beta Cin + alpha sum_s A_s^T B_s, A_s K x M.
-//               CTA (128 threads) = 64 x 16 block of C of one item over all
-//               of K; thread = rows (m, m + 32) x 4 columns, the A and B tiles
-//               stored k-contiguous so each thread reads 16-byte vectors along k.
+// launch) against a small one, so they are bound by HBM bandwidth once their
+// shared-memory reads are: the FP32 units are those of skinny_units.cuh, the
+// FP64 kernels run on the DMMA pipe out of a 3-stage cp.async ring.
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_skinny.cuh"
@@ -26,170 +18,38 @@ namespace hodlr {
 namespace {
 
 using namespace sk;
-constexpr int kSkThreads = 256;
 
-// ---------------------------------------------------------------- NN (rows)
-// FP32 C (M x N <= NC) = beta Cin + alpha sum_s A_s B_s with one row per
-// thread: A is read straight from global memory (a warp reads 32 consecutive
-// rows of one column: 128 bytes), 32 (16 when NC = 32) k-values in flight
-// per thread, while the matching block of B sits in shared memory.  Small CTAs (128 rows)
-// and no A staging let many CTAs share an SM, which keeps enough loads in
-// flight for the short-K products of the refinement sweeps (K = r).
-// The CTAs (as many as are resident: three per SM at the kernel's 168
-// registers) take the units (item, 128-row block) u = blockIdx.x,
-// blockIdx.x + gridDim.x, ...: at N = 262144 the root's m-column broadcast
-// has 2048 units, which as one CTA each ran in 4.6 waves of short CTAs.
+// ---------------------------------------------------------------- FP32
+// The resident CTAs (three per SM) take the units (item, row block)
+// u = blockIdx.x, blockIdx.x + gridDim.x, ...: at N = 262144 the root's
+// m-column broadcast has 2048 blocks of 128 rows, which as one CTA each ran in
+// 4.6 waves of short CTAs.
 template <int NC>
-__global__ void __launch_bounds__(kRowThreads)
+__global__ void __launch_bounds__(kRowThreads, 3)
     skinny_nn_rows_kernel(const GemmItem<float, float> *__restrict__ items,
                           const GemmSeg<float> *__restrict__ segs, float alpha, float beta,
                           int nunits, int rbn) {
-  __shared__ __align__(16) float Bs[nn_rows_kc<NC>() * NC];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   for (int u = blockIdx.x; u < nunits; u += gridDim.x)
-    nn_rows_unit<NC>(items, segs, alpha, beta, u / rbn, u % rbn, Bs);
+    nn_rows_unit<NC>(items, segs, alpha, beta, u / rbn, u % rbn, reinterpret_cast<float *>(smem_raw));
+}
+template <int NC>
+__global__ void __launch_bounds__(kRowThreads, 3)
+    skinny_nn_ring_kernel(const GemmItem<float, float> *__restrict__ items,
+                          const GemmSeg<float> *__restrict__ segs, float alpha, float beta,
+                          int nunits, int rbn) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  for (int u = blockIdx.x; u < nunits; u += gridDim.x)
+    nn_ring_unit<NC>(items, segs, alpha, beta, u / rbn, u % rbn, smem_raw);
 }
 
-// ---------------------------------------------------------------- NN
-// CTA = 512 rows of one item, thread = rows (r, r + 256), 2 x NC accumulators,
-// so every broadcast read of B feeds two rows.
-constexpr int kNNRows = 2 * kSkThreads;
-template <typename T>
-__host__ __device__ constexpr int nn_kt() { return sizeof(T) == 4 ? 16 : 8; }
-
-// ring depth: FP64 runs one CTA per SM (register bound) and keeps five tiles
-// in flight; FP32 two CTAs per SM with two each
-template <typename T>
-__host__ __device__ constexpr int nn_stages() { return sizeof(T) == 4 ? 3 : 6; }
-
-template <typename T, int NC>
-__global__ void __launch_bounds__(kSkThreads)
-    skinny_nn2_kernel(const GemmItem<T, T> *__restrict__ items, const GemmSeg<T> *__restrict__ segs,
-                      T alpha, T beta) {
-  constexpr int KT = nn_kt<T>();
-  constexpr int STG = nn_stages<T>();
-  constexpr int ROWS = kNNRows;
-  constexpr int VW = Vec<T>::W;
-  using V = typename Vec<T>::V;
+// CTA per (item, 64-row block)
+template <int NC>
+__global__ void __launch_bounds__(kTNThreads, 3)
+    skinny_tn_kernel(const GemmItem<float, float> *__restrict__ items,
+                     const GemmSeg<float> *__restrict__ segs, float alpha, float beta) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *As = reinterpret_cast<T *>(smem_raw);             // [stage][KT][ROWS]
-  T *Bs = As + (size_t)STG * KT * ROWS;          // [stage][KT][NC]
-  const GemmItem<T, T> it = items[blockIdx.x];
-  const int row0 = blockIdx.y * ROWS;
-  if (row0 >= it.M) return;
-  const int tid = threadIdx.x;
-  const int N = it.N;
-
-  auto load = [&](const TileIter<T> &p, int st) {
-    if (p.valid) {
-      const GemmSeg<T> &sg = p.sg;
-      T *a = As + (size_t)st * KT * ROWS;
-      T *b = Bs + (size_t)st * KT * NC;
-      const T *abase = sg.A + row0 + (long long)p.k0 * sg.lda;
-      const bool vec = ((reinterpret_cast<uintptr_t>(abase) & 15) == 0) && ((sg.lda % VW) == 0);
-      if (vec) {
-        for (int e = tid; e < KT * (ROWS / VW); e += kSkThreads) {
-          const int k = e / (ROWS / VW), rv = e % (ROWS / VW);
-          const int r = row0 + rv * VW;
-          const bool kin = p.k0 + k < sg.K;
-          const T *src = abase + rv * VW + (long long)k * sg.lda;
-          if (kin && r + VW <= it.M) {
-            cpa(a + k * ROWS + rv * VW, src, 16, true);
-          } else {
-#pragma unroll
-            for (int u = 0; u < VW; ++u) {
-              const bool ok = kin && r + u < it.M;
-              cpa(a + k * ROWS + rv * VW + u, ok ? src + u : sg.A, sizeof(T), ok);
-            }
-          }
-        }
-      } else {
-        for (int e = tid; e < KT * ROWS; e += kSkThreads) {
-          const int k = e / ROWS, rr = e % ROWS;
-          const bool ok = (p.k0 + k < sg.K) && row0 + rr < it.M;
-          cpa(a + k * ROWS + rr, ok ? abase + rr + (long long)k * sg.lda : sg.A, sizeof(T), ok);
-        }
-      }
-      for (int e = tid; e < KT * NC; e += kSkThreads) {
-        const int k = e % KT, n = e / KT;
-        const bool ok = (p.k0 + k < sg.K) && n < N;
-        cpa(b + k * NC + n, ok ? sg.B + (p.k0 + k) + (long long)n * sg.ldb : sg.B, sizeof(T), ok);
-      }
-    }
-    cpa_commit();
-  };
-
-  T acc0[NC], acc1[NC];
-#pragma unroll
-  for (int n = 0; n < NC; ++n) { acc0[n] = T(0); acc1[n] = T(0); }
-  TileIter<T> ld, cp;
-  ld.init(segs, it.seg_begin, it.seg_count);
-  cp = ld;
-#pragma unroll
-  for (int i = 0; i < STG - 1; ++i) {
-    load(ld, i);
-    if (ld.valid) ld.next(KT);
-  }
-  int st = 0, lst = STG - 1;
-  while (cp.valid) {
-    load(ld, lst);
-    if (ld.valid) ld.next(KT);
-    lst = (lst + 1) % STG;
-    cpa_wait<STG - 1>();
-    __syncthreads();
-    const T *a = As + (size_t)st * KT * ROWS + tid;
-    const T *b = Bs + (size_t)st * KT * NC;
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-      const T a0 = a[k * ROWS], a1 = a[k * ROWS + kSkThreads];
-#pragma unroll
-      for (int n = 0; n < NC; n += VW) {
-        const V bv = *reinterpret_cast<const V *>(b + k * NC + n);
-        const T *bp = reinterpret_cast<const T *>(&bv);
-#pragma unroll
-        for (int u = 0; u < VW; ++u) {
-          acc0[n + u] += a0 * bp[u];
-          acc1[n + u] += a1 * bp[u];
-        }
-      }
-    }
-    __syncthreads();  // stage st is refilled STG - 1 tiles later
-    st = (st + 1) % STG;
-    cp.next(KT);
-  }
-  cpa_wait<0>();
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int row = row0 + tid + h * kSkThreads;
-    if (row < it.M) {
-      static_assert(NC % 8 == 0, "whole column groups");
-      // per 8 columns: their Cin values before their stores (C may alias
-      // Cin, so a load after a store would wait for it)
-#pragma unroll
-      for (int n8 = 0; n8 < NC; n8 += 8) {
-        T cin[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u)
-          cin[u] = (it.Cin && n8 + u < N) ? it.Cin[row + (long long)(n8 + u) * it.ldcin] : T(0);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int n = n8 + u;
-          if (n >= N) break;
-          T v = alpha * (h ? acc1[n] : acc0[n]);
-          if (it.Cin) v += beta * cin[u];
-          it.C[row + (long long)n * it.ldc] = v;
-        }
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------- TN
-template <typename T>
-__global__ void __launch_bounds__(kTNThreads)
-    skinny_tn2_kernel(const GemmItem<T, T> *__restrict__ items, const GemmSeg<T> *__restrict__ segs,
-                      T alpha, T beta) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  tn2_unit<T>(items, segs, alpha, beta, blockIdx.x, blockIdx.y, blockIdx.z, smem_raw);
+  tn_unit<NC>(items, segs, alpha, beta, blockIdx.x, blockIdx.y, smem_raw);
 }
 
 // ---------------------------------------------------------------- FP64 on the DMMA pipe
@@ -487,44 +347,41 @@ void launch_skinny(const GemmItem<T, T> *items, const GemmSeg<T> *segs, int nite
     HODLR_LAUNCH_CHECK();
     return;
   }
-  if (trans) {
-    constexpr int TM = 64, TN = 16;
-    const size_t smem = tn2_smem_bytes<T>();
-    raise_smem_limit(reinterpret_cast<const void *>(skinny_tn2_kernel<T>), smem);
-    dim3 grid(nitems, cdiv(max_m, TM), cdiv(max_n, TN));
-    skinny_tn2_kernel<T><<<grid, kTNThreads, smem, s>>>(items, segs, alpha, beta);
-  } else if constexpr (sizeof(T) == 4) {
-    const int rbn = cdiv(max_m, kRowThreads);
-    const long long nunits = (long long)nitems * rbn;
-    if (nunits > 0x7fffffffLL) throw CudaError{cudaErrorInvalidValue};
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess)
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaGetLastError();
-    const int grid = (int)std::min<long long>(nunits, 3LL * sms);
-    const int nu = (int)nunits;
-    const auto *fi = reinterpret_cast<const GemmItem<float, float> *>(items);
-    const auto *fs = reinterpret_cast<const GemmSeg<float> *>(segs);
-    if (max_n <= 8)
-      skinny_nn_rows_kernel<8><<<grid, kRowThreads, 0, s>>>(fi, fs, alpha, beta, nu, rbn);
-    else if (max_n <= 16)
-      skinny_nn_rows_kernel<16><<<grid, kRowThreads, 0, s>>>(fi, fs, alpha, beta, nu, rbn);
-    else
-      skinny_nn_rows_kernel<32><<<grid, kRowThreads, 0, s>>>(fi, fs, alpha, beta, nu, rbn);
-  } else {
-    constexpr int KT = nn_kt<T>();
-    dim3 grid(nitems, cdiv(max_m, kNNRows));
-    if (max_n <= 16) {
-      const size_t smem = (size_t)nn_stages<T>() * KT * (kNNRows + 16) * sizeof(T);
-      raise_smem_limit(reinterpret_cast<const void *>(skinny_nn2_kernel<T, 16>), smem);
-      skinny_nn2_kernel<T, 16><<<grid, kSkThreads, smem, s>>>(items, segs, alpha, beta);
-    } else {
-      const size_t smem = (size_t)nn_stages<T>() * KT * (kNNRows + 32) * sizeof(T);
-      raise_smem_limit(reinterpret_cast<const void *>(skinny_nn2_kernel<T, 32>), smem);
-      skinny_nn2_kernel<T, 32><<<grid, kSkThreads, smem, s>>>(items, segs, alpha, beta);
-    }
+  if constexpr (sizeof(T) == 4) {
+    auto by_width = [&](auto &&f) {
+      if (max_n <= 8) f(std::integral_constant<int, 8>{});
+      else if (max_n <= 16) f(std::integral_constant<int, 16>{});
+      else f(std::integral_constant<int, 32>{});
+    };
+    by_width([&](auto w) {
+      constexpr int NC = decltype(w)::value;
+      if (trans) {
+        auto kern = skinny_tn_kernel<NC>;
+        raise_smem_limit(reinterpret_cast<const void *>(kern), tn_smem<NC>());
+        kern<<<dim3(nitems, cdiv(max_m, 64)), kTNThreads, tn_smem<NC>(), s>>>(items, segs, alpha,
+                                                                              beta);
+        return;
+      }
+      int sms = 148, dev = 0;
+      if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaGetLastError();
+      auto units = [&](auto kern, int rows, size_t smem) {
+        const int rbn = cdiv(max_m, rows);
+        const long long nunits = (long long)nitems * rbn;
+        if (nunits > 0x7fffffffLL) throw CudaError{cudaErrorInvalidValue};
+        const int grid = (int)std::min<long long>(nunits, 3LL * sms);
+        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
+        kern<<<grid, kRowThreads, smem, s>>>(items, segs, alpha, beta, (int)nunits, rbn);
+      };
+      // short items (the node products) a row per thread, tall ones by the ring
+      if (max_m <= kRowThreads)
+        units(skinny_nn_rows_kernel<NC>, kRowThreads, (size_t)kNnSlab * NC * sizeof(float));
+      else
+        units(skinny_nn_ring_kernel<NC>, kRingRows, nn_ring_smem<NC>());
+    });
+    HODLR_LAUNCH_CHECK();
   }
-  HODLR_LAUNCH_CHECK();
 }
 
 template void launch_skinny<double>(const GemmItem<double, double> *, const GemmSeg<double> *,

@@ -370,7 +370,6 @@ void build_sweep(PathPlan<T, TE> &plan) {
       d.red_segs = L.red_segs.p;
       d.n_red = L.n_red;
       d.red_mt = cdiv(std::max(L.red_max_m, 1), 64);
-      d.red_nt = cdiv(std::max(L.red_max_n, 1), 16);
       d.sums = L.sums.p;
       d.n_sums = L.n_sums;
       d.sum_units = (int)cdiv<long long>(std::max<long long>(L.sum_max_len, 1), kSweepSumChunk);
@@ -382,8 +381,8 @@ void build_sweep(PathPlan<T, TE> &plan) {
       d.bc_items = L.bc_items.p;
       d.bc_segs = L.bc_segs.p;
       d.n_bc = L.n_bc;
-      d.bc_rb = cdiv(std::max(L.bc_max_m, 1), 128);
-      mx = std::max(mx, std::max(L.ap_max_n, L.bc_max_n));
+      d.bc_rb = cdiv(std::max(L.bc_max_m, 1), 256);
+      mx = std::max({mx, L.red_max_n, L.ap_max_n, L.bc_max_n});
       v.push_back(d);
     }
     plan.sweep.upload(v);

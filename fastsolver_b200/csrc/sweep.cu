@@ -8,8 +8,8 @@
 // launch per step (four per level) spends most of its time ramping up and
 // draining.  sweep_levels_kernel runs all of them: one cooperative launch of
 // as many 128-thread CTAs as fit on the GPU, every CTA taking work units of a
-// step by grid stride (a 64 x 16 block of a reduce item, 32 elements of a
-// slot sum, 128 rows of an apply or broadcast item -- the same CTA units as
+// step by grid stride (64 rows of a reduce item, 32 elements of a slot sum,
+// 128 rows of an apply item, 256 of a broadcast item -- the same CTA units as
 // the one-step kernels, skinny_units.cuh), and a grid barrier between steps.
 //
 // The grid barrier is a counter in global memory: each CTA adds one, and the
@@ -85,10 +85,9 @@ __device__ bool grid_sync(unsigned *bar, unsigned &gen, long long limit) {
   return s_ok != 0;
 }
 
-// 3 CTAs (12 warps) per SM: the units keep a chunk of A, their share of B
-// and a row's Cin values in registers (up to 168 per thread); measured at
-// N = 262144 (m = 16) the same sweep time as 4 CTAs per SM, where the
-// 128-register bound makes them spill
+// Three CTAs (12 warps) per SM at 168 registers: at 32 columns the units'
+// accumulators make the kernel spill a little, yet two CTAs without spills ran
+// the sweeps of N = 1048576 in 20.7 instead of 18.2 ms.
 template <int NC>
 __global__ void __launch_bounds__(kThreads, 3)
     sweep_levels_kernel(const SweepLevel *__restrict__ levels, int nlevels, unsigned *bar) {
@@ -106,13 +105,9 @@ __global__ void __launch_bounds__(kThreads, 3)
     const SweepLevel L = levels[l];
     // reduce: partial slots of V_c^T d_c
     {
-      const int per = L.red_mt * L.red_nt;
-      const int nu = L.n_red * per;
-      for (int u = blockIdx.x; u < nu; u += gridDim.x) {
-        const int item = u / per, rem = u - item * per;
-        tn2_unit<float, true>(L.red_items, L.red_segs, 1.f, 0.f, item, rem / L.red_nt,
-                              rem % L.red_nt, smem);
-      }
+      const int nu = L.n_red * L.red_mt;
+      for (int u = blockIdx.x; u < nu; u += gridDim.x)
+        tn_unit<NC, true>(L.red_items, L.red_segs, 1.f, 0.f, u / L.red_mt, u % L.red_mt, smem);
     }
     if (!grid_sync(bar, gen, limit)) return;
     // slot sums in a fixed order (the REDOP_ADD of gemm.cc:74-133,
@@ -166,24 +161,17 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (!grid_sync(bar, gen, limit)) return;
     // broadcast d_c -= u_c eta_c
     {
-      float *Bs = reinterpret_cast<float *>(smem);
       const int nu = L.n_bc * L.bc_rb;
       for (int u = blockIdx.x; u < nu; u += gridDim.x)
-        nn_rows_unit<NC, true>(L.bc_items, L.bc_segs, -1.f, 1.f, u / L.bc_rb, u % L.bc_rb, Bs);
+        nn_ring_unit<NC, true>(L.bc_items, L.bc_segs, -1.f, 1.f, u / L.bc_rb, u % L.bc_rb, smem);
     }
     if (l + 1 < nlevels && !grid_sync(bar, gen, limit)) return;
   }
 }
 
-size_t sweep_smem() {
-  const size_t rows_b = std::max({nn_rows_kc<8>() * 8, nn_rows_kc<16>() * 16, nn_rows_kc<32>() * 32}) *
-                       sizeof(float);
-  return std::max(tn2_smem_bytes<float>(), rows_b);
-}
-
 template <int NC>
 void launch_nc(const SweepLevel *levels, int nlevels, unsigned *bar, cudaStream_t s) {
-  const size_t smem = sweep_smem();
+  const size_t smem = std::max(tn_smem<NC>(), nn_ring_smem<NC>());
   auto kern = sweep_levels_kernel<NC>;
   raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
   // co-resident CTAs (cached per device: the occupancy query is not a stream

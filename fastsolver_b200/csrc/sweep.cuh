@@ -16,11 +16,11 @@ struct SweepLevel {
   const GemmSeg<float> *ap_segs;
   const GemmItem<float, float> *bc_items;
   const GemmSeg<float> *bc_segs;
-  int n_red, red_mt, red_nt;  // items, 64-row and 16-column blocks per item
+  int n_red, red_mt;          // items, 64-row blocks per item
   int n_sums, sum_units;      // tasks, kSweepSumChunk-element chunks per task
   int sum_max_slots;          // most partial slots of one task
   int n_ap, ap_rb;            // items, 128-row blocks per item
-  int n_bc, bc_rb;
+  int n_bc, bc_rb;            // items, 256-row blocks per item
 };
 
 // Slot-sum elements per work unit of the persistent kernel.

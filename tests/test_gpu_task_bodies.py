@@ -240,3 +240,35 @@ def test_node_elimination_edges(fs, cuda, r0, r1):
         1 + np.linalg.norm(V0Tu0, 2)) ** 2 * (1 + np.linalg.norm(V1Tu1, 2)) ** 2
     assert np.linalg.norm(host(g[3]) - eta0) <= lim * np.linalg.norm(eta0)
     assert np.linalg.norm(host(g[2]) - eta1) <= lim * np.linalg.norm(eta1)
+
+
+@pytest.mark.parametrize("odd", [0, 1])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (63, 7, 9), (64, 8, 128), (65, 9, 129), (100, 32, 100),
+                                   (127, 16, 8), (128, 17, 64), (129, 31, 7), (255, 8, 127),
+                                   (256, 16, 144), (257, 32, 16), (1000, 5, 300), (4000, 32, 100)])
+def test_fp32_skinny_elementwise(fs, cuda, m, n, k, odd):
+    """The FP32 products of at most 32 columns at the edges of their row, column
+    and K blocks, on and off 16-byte boundaries, both orientations."""
+    import torch
+    from fastsolver_b200 import _lib
+    rng = np.random.default_rng(m + 3 * n + 7 * k)
+
+    def put(a, ld):
+        t = torch.zeros((a.shape[1], ld), dtype=torch.float32, device="cuda")
+        t[:, :a.shape[0]] = torch.from_numpy(np.ascontiguousarray(a.T))
+        return t
+
+    for trans in (0, 1):
+        A = rng.standard_normal((k, m) if trans else (m, k)).astype(np.float32)
+        B = rng.standard_normal((k, n)).astype(np.float32)
+        C = rng.standard_normal((m, n)).astype(np.float32)
+        lda, ldb, ldc = ((x + 3) // 4 * 4 + odd for x in (A.shape[0], k, m))
+        for alpha, beta in ((1.0, 0.0), (-1.0, 1.0), (0.5, -2.0)):
+            Ag, Bg, Cg = put(A, lda), put(B, ldb), put(C, ldc)
+            assert _lib.lib.hodlr_gemm_f32(trans, m, n, k, alpha, Ag.data_ptr(), lda, Bg.data_ptr(),
+                                           ldb, beta, Cg.data_ptr(), ldc, 0, None) == 0
+            op = (A.T if trans else A).astype(np.float64)
+            Bd, Cd = B.astype(np.float64), C.astype(np.float64)
+            err = np.abs(Cg.cpu().numpy().T[:m].astype(np.float64) - (alpha * (op @ Bd) + beta * Cd))
+            lim = (k + 4) * 2.0 ** -24 * (abs(alpha) * (np.abs(op) @ np.abs(Bd)) + abs(beta * Cd))
+            assert (err <= lim).all()
