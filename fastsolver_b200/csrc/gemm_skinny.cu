@@ -67,41 +67,44 @@ __device__ inline void dmma(double (&c)[4], double a0, double a1, double b) {
       : "d"(a0), "d"(a1), "d"(b));
 }
 
-constexpr int kDmmaStages = 3;
-
 // NN: C (M x N) = beta Cin + alpha sum_s A_s B_s, A_s column-major; one CTA
-// per (item, ROWS-row block, block of 8 NT8 columns), KT k-values per stage.
-// Large: 512 rows, 8 warps, 8 k (133 KB of A in flight per SM); small: 128
-// rows, 4 warps, 16 k, for launches that leave SMs without a large block and
-// for items that fill a quarter of one.
-template <bool SMALL>
+// per (item, ROWS-row block) and all of an item's columns (8 NT8; with two
+// passes of 16 the tall operand, all of D and U in a matvec, was read twice
+// above 16 columns: 9.0 instead of 7.5 ms at N = 1048576, 32 columns, where
+// the DMMA pipe's floor is 4.9 ms), KT
+// k-values per stage.  Large: 512 rows (256 above 16 columns, for the
+// accumulators), 8 warps, 8 k; small: 128 rows, 4 warps, 16 k, for launches
+// that leave SMs without a large block and for items that fill a quarter of one.
+template <int NT8, bool SMALL>
 struct NnDmma {
-  static constexpr int ROWS = SMALL ? 128 : 512, THREADS = SMALL ? 128 : 256;
+  static constexpr int NCS = 8 * NT8;
+  static constexpr int ROWS = SMALL ? 128 : NT8 > 2 ? 256 : 512, THREADS = SMALL ? 128 : 256;
   static constexpr int KT = SMALL ? 16 : 8;
-  static constexpr int AP = ROWS + 8;  // padded k-row stride (doubles)
-  static constexpr size_t smem(int ncs) {
-    return (size_t)kDmmaStages * KT * (AP + ncs + 4) * sizeof(double);
+  static constexpr int AP = ROWS + 8;              // padded k-row stride (doubles)
+  static constexpr int BP = NCS + 4;              // conflict-free fragments
+  static constexpr int STAGES = 3;                // (five above 16 columns: no gain)
+  static constexpr size_t smem() {
+    return (size_t)STAGES * KT * (AP + BP) * sizeof(double);
   }
 };
 
 template <int NT8, bool SMALL>
-__global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
+__global__ void __launch_bounds__(NnDmma<NT8, SMALL>::THREADS, 2)
     skinny_nn_dmma_kernel(const GemmItem<double, double> *__restrict__ items,
                           const GemmSeg<double> *__restrict__ segs, double alpha, double beta) {
-  using Cfg = NnDmma<SMALL>;
+  using Cfg = NnDmma<NT8, SMALL>;
   constexpr int KT = Cfg::KT, ROWS = Cfg::ROWS, AP = Cfg::AP, THREADS = Cfg::THREADS;
-  constexpr int NCS = 8 * NT8, BP = NCS + 4;  // conflict-free fragments
+  constexpr int NCS = Cfg::NCS, BP = Cfg::BP, STAGES = Cfg::STAGES;
   constexpr int MT = ROWS / (THREADS / 32) / 16;  // 16-row fragments per warp
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *As = reinterpret_cast<double *>(smem_raw);      // [stage][KT][AP]
-  double *Bs = As + (size_t)kDmmaStages * KT * AP;         // [stage][KT][BP]
+  double *Bs = As + (size_t)STAGES * KT * AP;         // [stage][KT][BP]
   const GemmItem<double, double> it = items[blockIdx.x];
   const int row0 = blockIdx.y * ROWS;
-  const int n0 = blockIdx.z * NCS;  // column block of this CTA
-  if (row0 >= it.M || n0 >= it.N) return;
+  if (row0 >= it.M) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int N = it.N - n0;  // columns left from n0
+  const int N = it.N;
 
   auto load = [&](const TileIter<double> &p, int st) {
     if (p.valid) {
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
       for (int e = tid; e < KT * NCS; e += THREADS) {
         const int k = e % KT, n = e / KT;
         const bool ok = (p.k0 + k < sg.K) && n < N;
-        cpa(b + k * BP + n, ok ? sg.B + (p.k0 + k) + (long long)(n0 + n) * sg.ldb : sg.B, 8,
+        cpa(b + k * BP + n, ok ? sg.B + (p.k0 + k) + (long long)n * sg.ldb : sg.B, 8,
             ok);
       }
     }
@@ -147,17 +150,17 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
   ld.init(segs, it.seg_begin, it.seg_count);
   cp = ld;
 #pragma unroll
-  for (int i = 0; i < kDmmaStages - 1; ++i) {
+  for (int i = 0; i < STAGES - 1; ++i) {
     load(ld, i);
     if (ld.valid) ld.next(KT);
   }
-  int st = 0, lst = kDmmaStages - 1;
+  int st = 0, lst = STAGES - 1;
   const int wrow = warp * 16 * MT;
   while (cp.valid) {
     load(ld, lst);
     if (ld.valid) ld.next(KT);
-    lst = (lst + 1) % kDmmaStages;
-    cpa_wait<kDmmaStages - 1>();
+    lst = (lst + 1) % STAGES;
+    cpa_wait<STAGES - 1>();
     __syncthreads();
     const double *a = As + (size_t)st * KT * AP;
     const double *b = Bs + (size_t)st * KT * BP;
@@ -174,8 +177,8 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
         for (int nt = 0; nt < NT8; ++nt) dmma(acc[mt][nt], a0, a1, bv[nt]);
       }
     }
-    __syncthreads();  // stage st is refilled kDmmaStages - 1 tiles later
-    st = (st + 1) % kDmmaStages;
+    __syncthreads();  // stage st is refilled STAGES - 1 tiles later
+    st = (st + 1) % STAGES;
     cp.next(KT);
   }
   cpa_wait<0>();
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
       for (int v = 0; v < 4; ++v) {
         const int row = row0 + wrow + mt * 16 + g + (v >> 1) * 8;
         const int c = nt * 8 + 2 * t + (v & 1);
-        cin[nt][v] = (it.Cin && row < it.M && c < N) ? it.Cin[row + (n0 + c) * (long long)it.ldcin]
+        cin[nt][v] = (it.Cin && row < it.M && c < N) ? it.Cin[row + c * (long long)it.ldcin]
                                                       : 0.0;
       }
 #pragma unroll
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
         const int row = row0 + wrow + mt * 16 + g + (v >> 1) * 8;
         const int c = nt * 8 + 2 * t + (v & 1);
         if (row < it.M && c < N) {
-          const long long col = n0 + c;
+          const long long col = c;
           double val = alpha * acc[mt][nt][v];
           if (it.Cin) val += beta * cin[nt][v];
           it.C[row + col * it.ldc] = val;
@@ -209,20 +212,27 @@ __global__ void __launch_bounds__(NnDmma<SMALL>::THREADS, 2)
   }
 }
 
-// TN: C (64 x 16 block of an item, over all K) = beta Cin + alpha sum_s A_s^T B_s
+// TN: C (64 rows of an item and all of its 8 NT8 columns, over all K) =
+// beta Cin + alpha sum_s A_s^T B_s
 constexpr int kDmmaKC = 32;
 constexpr int kDmmaLDK = kDmmaKC + 4;  // padded k stride (doubles): conflict-free fragments
 
+template <int NT8>
+constexpr size_t tn_dmma_smem() {
+  return (size_t)kSkStages * (64 + 8 * NT8) * kDmmaLDK * sizeof(double);
+}
+
+template <int NT8>
 __global__ void __launch_bounds__(kTNThreads)
     skinny_tn_dmma_kernel(const GemmItem<double, double> *__restrict__ items,
                           const GemmSeg<double> *__restrict__ segs, double alpha, double beta) {
-  constexpr int TM = 64, TN = 16, KC = kDmmaKC, LDK = kDmmaLDK;
+  constexpr int TM = 64, TN = 8 * NT8, KC = kDmmaKC, LDK = kDmmaLDK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *As = reinterpret_cast<double *>(smem_raw);   // [stage][TM][LDK]
   double *Bs = As + (size_t)kSkStages * TM * LDK;      // [stage][TN][LDK]
   const GemmItem<double, double> it = items[blockIdx.x];
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.z * TN;
-  if (m0 >= it.M || n0 >= it.N) return;
+  const int m0 = blockIdx.y * TM;
+  if (m0 >= it.M) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
 
@@ -250,12 +260,16 @@ __global__ void __launch_bounds__(kTNThreads)
   auto load = [&](const TileIter<double> &p, int st) {
     if (p.valid) {
       load_block(As + (size_t)st * TM * LDK, p.sg.A, p.sg.lda, p.k0, p.sg.K, m0, TM, it.M);
-      load_block(Bs + (size_t)st * TN * LDK, p.sg.B, p.sg.ldb, p.k0, p.sg.K, n0, TN, it.N);
+      load_block(Bs + (size_t)st * TN * LDK, p.sg.B, p.sg.ldb, p.k0, p.sg.K, 0, TN, it.N);
     }
     cpa_commit();
   };
 
-  double acc[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+  double acc[NT8][4];
+#pragma unroll
+  for (int nt = 0; nt < NT8; ++nt)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[nt][v] = 0.0;
   TileIter<double> ld, cp;
   ld.init(segs, it.seg_begin, it.seg_count);
   cp = ld;
@@ -276,8 +290,8 @@ __global__ void __launch_bounds__(kTNThreads)
 #pragma unroll
     for (int ks = 0; ks < KC; ks += 4) {
       const double a0 = a[ks], a1 = a[8 * LDK + ks];
-      dmma(acc[0], a0, a1, b[ks]);
-      dmma(acc[1], a0, a1, b[8 * LDK + ks]);
+#pragma unroll
+      for (int nt = 0; nt < NT8; ++nt) dmma(acc[nt], a0, a1, b[8 * nt * LDK + ks]);
     }
     __syncthreads();
     st = (st + 1) % kSkStages;
@@ -285,27 +299,36 @@ __global__ void __launch_bounds__(kTNThreads)
   }
   cpa_wait<0>();
   // every Cin value before any store (C may alias Cin)
-  double cin[2][4];
+  double cin[NT8][4];
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
+  for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const int gm = m0 + warp * 16 + g + (v >> 1) * 8;
-      const int gn = n0 + nt * 8 + 2 * t + (v & 1);
+      const int gn = nt * 8 + 2 * t + (v & 1);
       cin[nt][v] = (it.Cin && gm < it.M && gn < it.N) ? it.Cin[gm + (long long)gn * it.ldcin] : 0.0;
     }
 #pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
+  for (int nt = 0; nt < NT8; ++nt)
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       const int gm = m0 + warp * 16 + g + (v >> 1) * 8;
-      const int gn = n0 + nt * 8 + 2 * t + (v & 1);
+      const int gn = nt * 8 + 2 * t + (v & 1);
       if (gm < it.M && gn < it.N) {
         double val = alpha * acc[nt][v];
         if (it.Cin) val += beta * cin[nt][v];
         it.C[gm + (long long)gn * it.ldc] = val;
       }
     }
+}
+
+// f(blocks of 8 columns of the widest item)
+template <typename F>
+void dmma_by_width(int max_n, F &&f) {
+  if (max_n <= 8) f(std::integral_constant<int, 1>{});
+  else if (max_n <= 16) f(std::integral_constant<int, 2>{});
+  else if (max_n <= 24) f(std::integral_constant<int, 3>{});
+  else f(std::integral_constant<int, 4>{});
 }
 
 }  // namespace
@@ -317,32 +340,30 @@ void launch_skinny(const GemmItem<T, T> *items, const GemmSeg<T> *segs, int nite
   if constexpr (sizeof(T) == 8) {
     // FP64 products run on the FP64 tensor pipe (DMMA)
     if (trans) {
-      const size_t smem = (size_t)kSkStages * (64 + 16) * kDmmaLDK * sizeof(double);
-      raise_smem_limit(reinterpret_cast<const void *>(skinny_tn_dmma_kernel), smem);
-      dim3 grid(nitems, cdiv(max_m, 64), cdiv(max_n, 16));
-      skinny_tn_dmma_kernel<<<grid, kTNThreads, smem, s>>>(items, segs, alpha, beta);
+      dmma_by_width(max_n, [&](auto w) {
+        constexpr int NT8 = decltype(w)::value;
+        auto kern = skinny_tn_dmma_kernel<NT8>;
+        raise_smem_limit(reinterpret_cast<const void *>(kern), tn_dmma_smem<NT8>());
+        kern<<<dim3(nitems, cdiv(max_m, 64)), kTNThreads, tn_dmma_smem<NT8>(), s>>>(items, segs,
+                                                                                  alpha, beta);
+      });
     } else {
-      // 8 columns per CTA when every item has at most 8, else 16-column blocks.
       // Small blocks where large ones would leave SMs idle or mostly empty:
       // matvec of 4096 rows 88 -> 36 us, 60001 rows 201 -> 184 us, node
       // products of 128 rows 233 -> 129 us per solve; above, large ones stream
       // faster (131072 rows: 346 us large, 404 us small).
-      const int nz = max_n <= 8 ? 1 : cdiv(max_n, 16);
-      const bool small = max_m <= 256 || (long long)nitems * cdiv(max_m, 512) * nz < 148;
+      const bool small = max_m <= 256 || (long long)nitems * cdiv(max_m, 512) < 148;
       auto go = [&](auto kern, auto cfg) {
         using Cfg = decltype(cfg);
-        const size_t smem = Cfg::smem(max_n <= 8 ? 8 : 16);
-        raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-        const dim3 grid(nitems, cdiv(max_m, Cfg::ROWS), nz);
-        kern<<<grid, Cfg::THREADS, smem, s>>>(items, segs, alpha, beta);
+        raise_smem_limit(reinterpret_cast<const void *>(kern), Cfg::smem());
+        const dim3 grid(nitems, cdiv(max_m, Cfg::ROWS));
+        kern<<<grid, Cfg::THREADS, Cfg::smem(), s>>>(items, segs, alpha, beta);
       };
-      if (max_n <= 8) {
-        if (small) go(skinny_nn_dmma_kernel<1, true>, NnDmma<true>{});
-        else go(skinny_nn_dmma_kernel<1, false>, NnDmma<false>{});
-      } else {
-        if (small) go(skinny_nn_dmma_kernel<2, true>, NnDmma<true>{});
-        else go(skinny_nn_dmma_kernel<2, false>, NnDmma<false>{});
-      }
+      dmma_by_width(max_n, [&](auto w) {
+        constexpr int NT8 = decltype(w)::value;
+        if (small) go(skinny_nn_dmma_kernel<NT8, true>, NnDmma<NT8, true>{});
+        else go(skinny_nn_dmma_kernel<NT8, false>, NnDmma<NT8, false>{});
+      });
     }
     HODLR_LAUNCH_CHECK();
     return;
