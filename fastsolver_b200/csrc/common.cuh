@@ -73,7 +73,10 @@ struct GemmSeg {
   long long lda;
   long long ldb;
   int K;
-  int pad;
+  // A's zero half, which the FP64 tile GEMM leaves out (no other kernel looks):
+  // 1 = A is lower triangular, 2 = upper; only where the segment is its item's
+  // only one, A is not transposed and M <= 128
+  int tri;
 };
 
 // C (M x N) = beta * Cin + alpha * sum_s op(A_s) B_s over segments

@@ -151,11 +151,13 @@ struct MCols {
           !one;
     p = base + m + (long long)k * ld;
   }
-  __device__ void copy(double *s, int left) {
+  // only the rows [lo, hi)
+  __device__ void copy(double *s, int left, int lo = 0, int hi = BM) {
     const int k = threadIdx.x / (BM / 2), mv = 2 * (threadIdx.x % (BM / 2));
     double *d = s + k * (BM + 4) + mv;
     const int u = one ? 0 : 1;
-    if (left >= BK) {
+    if (mv < lo || mv >= hi) {
+    } else if (left >= BK) {
       if (vec) {
 #pragma unroll
         for (int i = 0; i < NC; ++i) cpa16(d + i * STEP * (BM + 4), p + i * STEP * ld);
@@ -200,7 +202,14 @@ __global__ void __launch_bounds__(WM *WN * 32, WM * WN == 4 ? 3 : 2)
   if (m0 >= it.M || n0 >= it.N) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = (warp / WN) * (16 * MT), wn = (warp % WN) * 32;
+  const int wn = (warp % WN) * 32;
+  // tile row of the warp's row fragment mt: fragments w and 2 WM - 1 - w, so
+  // that a triangular A gives every warp (each on its own SM quarter) the same
+  // number of products
+  auto frow = [&](int mt) {
+    return 16 * (mt & 1 ? MT * WM - 1 - warp / WN : warp / WN);
+  };
+  static_assert(MT <= 2, "two fragments mirror each other");
 
   // the item's K stages, flattened over its segments
   KRows<BN, THREADS> cb;
@@ -219,12 +228,24 @@ __global__ void __launch_bounds__(WM *WN * 32, WM * WN == 4 ? 3 : 2)
       return;
     }
   };
+  // A's zero half (the leaf LU's block-row solves) is neither copied nor
+  // multiplied: stage i of a lower (upper) triangle holds values only in the
+  // rows from (up to) its 16-row fragment i.  N = 262144, leaf 512, r = 64,
+  // m = 16: block solves and inverses 2.76 -> 2.45 ms, the backward solve
+  // 3.60 -> 3.38 ms, the solve 21.9 -> 21.4 ms.
+  const int tri = !TRANS && it.seg_count == 1 ? segs[seg].tri : 0;
+  int copied = 0;  // stages
   int stages = 0;
   for (int s = seg; s < seg_end; ++s) stages += (max(segs[s].K, 0) + BK - 1) / BK;
   auto load = [&](int st) {
     if (left <= 0) settle();
     if (left > 0) {
-      ca.copy(As + (size_t)st * AS, left);
+      if constexpr (TRANS)
+        ca.copy(As + (size_t)st * AS, left);
+      else
+        ca.copy(As + (size_t)st * AS, left, tri == 1 ? BK * copied : 0,
+                tri == 2 ? BK * (copied + 1) : BM);
+      ++copied;
       cb.copy(Bs + (size_t)st * BS, left);
       left -= BK;
     }
@@ -239,7 +260,7 @@ __global__ void __launch_bounds__(WM *WN * 32, WM * WN == 4 ? 3 : 2)
   // any is used (rows and columns outside the item repeat its last ones, for
   // outputs that are not stored)
   auto load_cin = [&](int mt, double (&c)[4][4]) {
-    const int row = m0 + wm + mt * 16 + g;
+    const int row = m0 + frow(mt) + g;
     const double *c0 = it.Cin + min(row, it.M - 1), *c1 = it.Cin + min(row + 8, it.M - 1);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
@@ -270,29 +291,39 @@ __global__ void __launch_bounds__(WM *WN * 32, WM * WN == 4 ? 3 : 2)
         for (int v = 0; v < 4; ++v) acc[mt][nt][v] = 0.0;
   }
 
-  int st = 0, lst = kStages - 1;
-  for (int i = 0; i < stages; ++i) {
-    cpa_wait<kStages - 2>();  // this thread's copies of stage i have landed
-    __syncthreads();          // ... and everybody's; slot lst (stage i - 1) is free
-    load(lst);
-    lst = lst + 1 == kStages ? 0 : lst + 1;
-    const double *a = As + (size_t)st * AS;
-    const double *b = Bs + (size_t)st * BS;
+  auto run = [&](auto triangular) {
+    constexpr bool TRI = decltype(triangular)::value;
+    int st = 0, lst = kStages - 1;
+    for (int i = 0; i < stages; ++i) {
+      cpa_wait<kStages - 2>();  // this thread's copies of stage i have landed
+      __syncthreads();          // ... and everybody's; slot lst (stage i - 1) is free
+      load(lst);
+      lst = lst + 1 == kStages ? 0 : lst + 1;
+      const double *a = As + (size_t)st * AS;
+      const double *b = Bs + (size_t)st * BS;
 #pragma unroll
-    for (int ks = 0; ks < BK; ks += 4) {
-      double bv[4];
+      for (int ks = 0; ks < BK; ks += 4) {
+        double bv[4];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) bv[nt] = b[(wn + nt * 8 + g) * LDK + ks + t];
+        for (int nt = 0; nt < 4; ++nt) bv[nt] = b[(wn + nt * 8 + g) * LDK + ks + t];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const int mr = wm + mt * 16 + g;
-        const double a0 = TRANS ? a[mr * LDK + ks + t] : a[(ks + t) * AP + mr];
-        const double a1 = TRANS ? a[(mr + 8) * LDK + ks + t] : a[(ks + t) * AP + mr + 8];
+        for (int mt = 0; mt < MT; ++mt) {
+          if (TRI && (tri == 1 ? frow(mt) < BK * i : frow(mt) > BK * i)) continue;
+          const int mr = frow(mt) + g;
+          const double a0 = TRANS ? a[mr * LDK + ks + t] : a[(ks + t) * AP + mr];
+          const double a1 = TRANS ? a[(mr + 8) * LDK + ks + t] : a[(ks + t) * AP + mr + 8];
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], a0, a1, bv[nt]);
+          for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], a0, a1, bv[nt]);
+        }
       }
+      st = st + 1 == kStages ? 0 : st + 1;
     }
-    st = st + 1 == kStages ? 0 : st + 1;
+  };
+  if constexpr (TRANS) {
+    run(std::false_type{});
+  } else {
+    if (tri) run(std::true_type{});
+    else run(std::false_type{});
   }
   cpa_wait<0>();
 
@@ -312,7 +343,7 @@ __global__ void __launch_bounds__(WM *WN * 32, WM * WN == 4 ? 3 : 2)
 #pragma unroll
         for (int v = 0; v < 4; ++v) x[nt][v] += beta * c[nt][v];
     }
-    const int row = m0 + wm + mt * 16 + g;
+    const int row = m0 + frow(mt) + g;
     const bool ok0 = row < it.M, ok1 = row + 8 < it.M;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)

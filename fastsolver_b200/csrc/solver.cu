@@ -104,9 +104,9 @@ struct HostStep {
   std::vector<GemmItem<T, T>> it;
   std::vector<GemmSeg<T>> sg;
   void add(T *C, long long ldc, int M, int N, const T *A, long long lda, const T *B,
-           long long ldb, int K, bool inplace) {
+           long long ldb, int K, bool inplace, int tri = 0) {
     if (M <= 0 || N <= 0 || K <= 0) return;
-    GemmSeg<T> g{A, B, lda, ldb, K, 0};
+    GemmSeg<T> g{A, B, lda, ldb, K, tri};
     GemmItem<T, T> i{C, inplace ? C : nullptr, ldc, inplace ? ldc : 0, M, N, (int)sg.size(), 1};
     sg.push_back(g);
     it.push_back(i);
@@ -179,8 +179,8 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         const T *Li = k.LinvB + (size_t)J * OB * OB;
         T *Dr = k.D + j0 + (long long)(j0 + obe) * k.ldd;
         T *Xr = k.X + j0;
-        tr.add(Dr, k.ldd, obe, k.n - j0 - obe, Li, OB, Dr, k.ldd, obe, false);
-        tr.add(Xr, k.ldx, obe, k.ncols, Li, OB, Xr, k.ldx, obe, false);
+        tr.add(Dr, k.ldd, obe, k.n - j0 - obe, Li, OB, Dr, k.ldd, obe, false, 1);
+        tr.add(Xr, k.ldx, obe, k.ncols, Li, OB, Xr, k.ldx, obe, false, 1);
       }
       fwd.push_back(std::move(tr));
     }
@@ -229,7 +229,8 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         if (j0 >= k.n) continue;
         const int obe = std::min(OB, k.n - j0);
         T *Xk = k.X + j0;
-        tr.add(Xk, k.ldx, obe, k.ncols, k.UinvB + (size_t)J * OB * OB, OB, Xk, k.ldx, obe, false);
+        tr.add(Xk, k.ldx, obe, k.ncols, k.UinvB + (size_t)J * OB * OB, OB, Xk, k.ldx, obe, false,
+               2);
       }
       bwd.push_back(std::move(tr));
     }

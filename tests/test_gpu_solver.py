@@ -283,3 +283,22 @@ def test_leaf_apply_edges(fs, cuda, n, m):
         X = np.linalg.solve(A, B)
         lim = (50 * n if prec == fs.PREC_FP64 else 8) * cond * u
         assert np.linalg.norm(h.solution() - X) <= lim * np.linalg.norm(X)
+
+
+@pytest.mark.parametrize("ob64", [64, 128])
+@pytest.mark.parametrize("n", [15, 16, 17, 33, 64, 65, 100, 127, 128, 129, 177, 241, 300])
+def test_fp64_block_row_solves_edges(fs, cuda, n, ob64):
+    """The triangular products of the two-level FP64 leaf LU, whose zero half
+    is left out by 16-row fragments, at the remainders of blocks and fragments."""
+    rng = np.random.default_rng(10 * n + ob64)
+    A = rng.standard_normal((n, n)) / np.sqrt(n) + 2 * np.eye(n)
+    A = A[rng.permutation(n)]
+    B = rng.standard_normal((n, 40))
+    h = fs.HodlrMatrix(40, n, 1, 1024).create_tree()
+    h.schedule = dict(leaf_ob64=ob64)
+    h.set_matrix(A)
+    h.set_rhs(B)
+    fs.FastSolver().bfs_solve(h)
+    X = np.linalg.solve(A, B)
+    lim = 50 * n * np.linalg.cond(A) * 2.0 ** -53
+    assert np.linalg.norm(h.solution() - X) <= lim * np.linalg.norm(X)
