@@ -86,10 +86,10 @@ __device__ inline T tabs(T v) {
 // panel with its inverses 27 us (FP64, 32 columns) and 41 us (FP32, 64) where
 // it took 50 and 87 us.
 constexpr int kRegThreads = 512;
-// order of the triangular blocks that are inverted on their own
-template <typename T, int NB>
+// columns of a triangle's inverse per warp
+template <int NB>
 __host__ __device__ constexpr int panel_sub() {
-  return NB < 64 / (int)sizeof(T) * 2 ? NB : 64 / (int)sizeof(T) * 2;
+  return NB < 32 ? NB : 32;
 }
 
 // |a| as an integer that orders like it, plus one; 0 for a NaN (never a
@@ -400,106 +400,71 @@ __global__ void __launch_bounds__(kRegThreads, 1)
     if (info_local && info && info[tk.info_slot] == 0) info[tk.info_slot] = info_local;
   }
   __syncthreads();
-  // Inverses of the diagonal block's triangles, from those of their SUB x SUB
-  // diagonal blocks (SUB = 32, FP64 16: a lane's column in registers).  One warp
-  // per such block, a lane per column, the column in registers: after x_k,
-  // all later x_i -= A[i][k] x_k are independent, A[.][k] read as broadcasts.
-  // (With lanes as rows and x_k passed by shuffles the shuffles took 9.5 k
-  // cycles per 32 x 32 FP64 pair and 17.5 k per 64 x 64 FP32 pair.)
-  constexpr int SUB = panel_sub<T, NB>(), NT = NB / SUB, LDI = SUB + VW;
-  static_assert(NT <= 2, "two diagonal blocks at most");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *inv = reinterpret_cast<T *>(smem_raw);  // NT == 2: the four blocks' inverses, column-major
+  // Inverses of the diagonal block's triangles, every column by substitution: a
+  // warp per 32 columns of a triangle, a lane per column, RB rows at a time in
+  // registers; A's columns are read as broadcasts.  (With lanes as rows and x_k
+  // passed by shuffles the shuffles took 9.5 k cycles per 32 x 32 FP64 pair and
+  // 17.5 k per 64 x 64 FP32 pair; with all rows in registers the straight-line
+  // code's instruction fetches took 5 us per FP64 panel.)  The columns are not put
+  // together from the inverses of half blocks, -A22^{-1} (A21 A11^{-1}): that
+  // squares the triangle's condition number in the residual of a solve.
+  constexpr int CB = panel_sub<NB>(), NT = NB / CB, RB = 16;
   T *Lout = tk.Linv + (size_t)panel * NB * NB;
   T *Uout = tk.Uinv + (size_t)panel * NB * NB;
-  for (int tri = warp; tri < 2 * NT; tri += nw) {
-    const bool upper = tri >= NT;
-    const int o = tri % NT * SUB;
-    const T *A = (upper ? Uk : Lk) + o * NB + o;
-    T x[SUB];
+  for (int job = warp; job < 2 * NT; job += nw) {
+    const bool upper = job >= NT;
+    const int cb = job % NT * CB;  // the warp's columns cb, cb + 1, ..
+    const int j = cb + lane % CB;  // this lane's
+    T *A = upper ? Uk : Lk;
+    T *out = upper ? Uout + (NB - RB) + (size_t)(NB - 1 - j) * NB : Lout + (size_t)j * NB;
+#pragma unroll 1
+    for (int o = 0; o < NB; o += RB) {
+      T x[RB];
 #pragma unroll
-    for (int i = 0; i < SUB; ++i) x[i] = lane == i ? T(1) : T(0);
-#pragma unroll
-    for (int k = 0; k < SUB; ++k) {
-      __syncwarp();  // A's columns are read as needed (read ahead, they spill)
-      if (upper) x[k] *= udr[o + k];
-#pragma unroll
-      for (int cv = (k + 1) / VW; cv < SUB / VW; ++cv) {
-        const V v = reinterpret_cast<const V *>(A + k * NB)[cv];
-        const T *vp = reinterpret_cast<const T *>(&v);
-#pragma unroll
-        for (int u = 0; u < VW; ++u)
-          if (cv * VW + u > k) x[cv * VW + u] -= vp[u] * x[k];
-      }
-    }
-    if (lane < SUB) {
-      T *out = upper ? Uout + (NB - SUB - o) + (size_t)(NB - 1 - o - lane) * NB
-                     : Lout + o + (size_t)(o + lane) * NB;
-#pragma unroll
-      for (int cv = 0; cv < SUB / VW; ++cv) {
-        V v, w;
-        T *vp = reinterpret_cast<T *>(&v), *wp = reinterpret_cast<T *>(&w);
-#pragma unroll
-        for (int u = 0; u < VW; ++u) {
-          vp[u] = x[cv * VW + u];
-          wp[u] = upper ? x[SUB - 1 - cv * VW - u] : vp[u];
-        }
-        reinterpret_cast<V *>(out)[cv] = w;
-        if constexpr (NT == 2) reinterpret_cast<V *>(inv + (tri * SUB + lane) * LDI)[cv] = v;
-      }
-    }
-  }
-  if constexpr (NT == 2) {
-    // off-diagonal blocks: -A22^{-1} (A21 A11^{-1}), the inner product kept in
-    // the triangle's zero block; a warp takes CB columns, lane = row
-    constexpr int CB = 4;
-    const int row = lane % SUB;
-    const bool mine = lane < SUB;
-    // acc[c] = sum_k A[k sa + row] B[c sb + k]
-    auto product = [&](const T *A, int sa, const T *B, int sb, T (&acc)[CB]) {
-#pragma unroll
-      for (int c = 0; c < CB; ++c) acc[c] = T(0);
+      for (int i = 0; i < RB; ++i) x[i] = o + i == j ? T(1) : T(0);
+      // less A's part left of the diagonal times the rows above, which are kept
+      // on and above A's diagonal (x_k of column j in A's row j, column k >= j)
 #pragma unroll 4
-      for (int kv = 0; kv < SUB / VW; ++kv) {
-        T x[VW];
+      for (int k = cb; k < o; ++k) {
+        const T xk = j <= k ? A[k * NB + j] : T(0);
 #pragma unroll
-        for (int u = 0; u < VW; ++u) x[u] = A[(kv * VW + u) * sa + row];
-#pragma unroll
-        for (int c = 0; c < CB; ++c) {
-          const V v = reinterpret_cast<const V *>(B + c * sb)[kv];
+        for (int cv = 0; cv < RB / VW; ++cv) {
+          const V v = reinterpret_cast<const V *>(A + k * NB + o)[cv];
           const T *vp = reinterpret_cast<const T *>(&v);
 #pragma unroll
-          for (int u = 0; u < VW; ++u) acc[c] += x[u] * vp[u];
+          for (int u = 0; u < VW; ++u) x[cv * VW + u] -= vp[u] * xk;
         }
       }
-    };
-    T acc[CB];
-    __syncthreads();
-    for (int job = warp; job < 2 * SUB / CB; job += nw) {
-      const bool upper = job >= SUB / CB;
-      const int j = job % (SUB / CB) * CB;
-      T *A = upper ? Uk : Lk;
-      product(A + SUB, NB, inv + ((upper ? 2 : 0) * SUB + j) * LDI, LDI, acc);
+      if (o + RB > cb) {
 #pragma unroll
-      for (int c = 0; c < CB; ++c)
-        if (mine) A[(SUB + j + c) * NB + lane] = acc[c];
-    }
-    __syncthreads();
-    for (int job = warp; job < 2 * SUB / CB; job += nw) {
-      const bool upper = job >= SUB / CB;
-      const int j = job % (SUB / CB) * CB;
-      product(inv + (upper ? 3 : 1) * SUB * LDI, LDI, (upper ? Uk : Lk) + (SUB + j) * NB, NB, acc);
+        for (int k = 0; k < RB; ++k) {
+          __syncwarp();  // A's columns are read as needed (read ahead, they spill)
+          if (upper) x[k] *= udr[o + k];
 #pragma unroll
-      for (int c = 0; c < CB; ++c) {
-        if (!mine) continue;
-        if (upper) {
-          Uout[SUB - 1 - lane + (size_t)(NB - 1 - j - c) * NB] = -acc[c];
-          Uout[NB - 1 - lane + (size_t)(SUB - 1 - j - c) * NB] = T(0);
-        } else {
-          Lout[SUB + lane + (size_t)(j + c) * NB] = -acc[c];
-          Lout[lane + (size_t)(SUB + j + c) * NB] = T(0);
+          for (int cv = (k + 1) / VW; cv < RB / VW; ++cv) {
+            const V v = reinterpret_cast<const V *>(A + (o + k) * NB + o)[cv];
+            const T *vp = reinterpret_cast<const T *>(&v);
+#pragma unroll
+            for (int u = 0; u < VW; ++u)
+              if (cv * VW + u > k) x[cv * VW + u] -= vp[u] * x[k];
+          }
         }
       }
+      __syncwarp();
+      if (lane < CB) {
+#pragma unroll
+        for (int cv = 0; cv < RB / VW; ++cv) {
+          V w;
+          T *wp = reinterpret_cast<T *>(&w);
+#pragma unroll
+          for (int u = 0; u < VW; ++u) wp[u] = x[upper ? RB - 1 - cv * VW - u : cv * VW + u];
+          reinterpret_cast<V *>(out + (upper ? -o : o))[cv] = w;
+        }
+#pragma unroll
+        for (int k = 0; k < RB; ++k)
+          if (j <= o + k) A[(o + k) * NB + j] = x[k];
+      }
+      __syncwarp();
     }
   }
 }
@@ -1062,13 +1027,10 @@ template <typename T, int NB, int RPT>
 void launch_leaf_panel_reg(const LeafFactorTask<T> *tasks, int count, int rows, int k0,
                            int panel, int *info, cudaStream_t s) {
   // one thread per RPT live rows of the largest leaf's panel, and a warp for
-  // each of the inverses' triangular blocks
-  constexpr int SUB = panel_sub<T, NB>(), blocks = 2 * NB / SUB;
+  // each of the inverses' column blocks
+  constexpr int blocks = 2 * NB / panel_sub<NB>();
   const int threads = std::min(kRegThreads, std::max(32 * blocks, cdiv(cdiv(rows, RPT), 32) * 32));
-  // two blocks per triangle: their inverses
-  const size_t smem = blocks > 2 ? (size_t)blocks * SUB * (SUB * sizeof(T) + 16) : 0;
-  raise_smem_limit(reinterpret_cast<const void *>(leaf_panel_reg_kernel<T, NB, RPT>), smem);
-  leaf_panel_reg_kernel<T, NB, RPT><<<count, threads, smem, s>>>(tasks, k0, panel, info);
+  leaf_panel_reg_kernel<T, NB, RPT><<<count, threads, 0, s>>>(tasks, k0, panel, info);
   HODLR_LAUNCH_CHECK();
 }
 

@@ -302,3 +302,47 @@ def test_fp64_block_row_solves_edges(fs, cuda, n, ob64):
     X = np.linalg.solve(A, B)
     lim = 50 * n * np.linalg.cond(A) * 2.0 ** -53
     assert np.linalg.norm(h.solution() - X) <= lim * np.linalg.norm(X)
+
+
+def _gepp(A):
+    """(L, U, row order) of Gaussian elimination with partial pivoting."""
+    A, n = A.copy(), A.shape[0]
+    p = np.arange(n)
+    for k in range(n):
+        j = k + int(np.argmax(np.abs(A[k:, k])))
+        A[[k, j]], p[[k, j]] = A[[j, k]], p[[j, k]]
+        A[k + 1:, k] /= A[k, k]
+        A[k + 1:, k + 1:] -= np.outer(A[k + 1:, k], A[k, k + 1:])
+    return np.tril(A, -1) + np.eye(n), np.triu(A), p
+
+
+def _smooth_kernel(n, s, shift):
+    x = np.linspace(0, 1, n)
+    return np.exp(-((x[:, None] - x) / s) ** 2) + shift * np.eye(n)
+
+
+@pytest.mark.parametrize("prec,n,s,shift", [("fp64", 32, 0.1, 1e-8), ("fp64", 32, 0.2, 1e-8),
+                                            ("fp64", 32, 0.3, 1e-8), ("mixed", 48, 0.1, 1e-6),
+                                            ("mixed", 64, 0.1, 1e-7), ("mixed", 64, 0.05, 1e-7)])
+def test_panel_inverse_residual(fs, cuda, prec, n, s, shift):
+    """Kept factors of one panel whose triangles are ill-conditioned: the explicit
+    inverses Y of the triangles T have |T Y - I| <= n u |T| |Y|, so that a solve
+    with them leaves the residual below, where inverses whose error grows with
+    the square of the condition number do not."""
+    u, prec = (2.0 ** -53, fs.PREC_FP64) if prec == "fp64" else (2.0 ** -24, fs.PREC_MIXED)
+    dt = np.float64 if prec == fs.PREC_FP64 else np.float32
+    A = _smooth_kernel(n, s, shift).astype(dt).astype(np.float64)
+    B = np.random.default_rng(n).standard_normal((n, 4)).astype(dt).astype(np.float64)
+    h = fs.HodlrMatrix(4, n, 1, 1024).create_tree()
+    h.set_matrix(A)
+    h.set_rhs(B)
+    solver = fs.FastSolver()
+    solver.factor(h, prec)
+    solver.solve(h)
+    L, U, p = _gepp(A)
+    a = np.abs
+    w = a(np.linalg.inv(L)) @ a(B[p])
+    # |b - L y| <= 2 n u |L| |Y_L| |b|, likewise for U, and L U = P A + n u |L| |U|
+    lim = n * u * (2 * a(L) @ w + 3 * a(L) @ (a(U) @ (a(np.linalg.inv(U)) @ w)))
+    r = a((B - A.astype(np.longdouble) @ h.solution()).astype(np.float64))[p]
+    assert (r <= lim).all()
