@@ -15,12 +15,15 @@
 //     leaf_laswp_kernel   the panel's row interchanges on every other column
 //                         of D (LAPACK layout) and of X; a no-op for leaves
 //                         whose panel pivoted on the diagonal
-//     batched GEMM        U12 = L11^{-1} A12 (in place, D and X columns)
+//     leaf_panel_solve    U12 = L11^{-1} A12 (in place, D and X columns; FP32: an
+//                         item of the batched GEMM)
 //     batched GEMM        A22 -= L21 U12 (D trailing block and X rows below)
 //   then for each panel from the last: X[k] = U_kk^{-1} X[k];
 //                                      X[0:k0] -= U[0:k0, k] X[k]
 // so D ends as LAPACK's P L U factors, X as D^{-1} X.  The GEMMs are items of
 // the batched GEMM engine (gemm_simt.cu), one launch per step for all leaves.
+// FP64 solves use the triangles' inverses only where these are well-conditioned
+// (ill_conditioned below), substitution elsewhere.
 #include <algorithm>
 #include <cstdlib>
 #include <type_traits>
@@ -56,11 +59,6 @@ template <>
 struct Vec16<double> {
   using V = double2;
 };
-
-template <typename T>
-__device__ inline T tabs(T v) {
-  return v < T(0) ? -v : v;
-}
 
 // Register-resident panel LU in LAPACK's dgetf2 pivot order, with implicit row
 // interchanges (rows stay in their threads, each tracking its current
@@ -843,6 +841,35 @@ __global__ void __launch_bounds__(512, 1)
     }
 }
 
+// Whether an FP64 triangle T with the explicit inverse Y is solved by
+// substitution instead: max|T| max|Y| of about 64 or more, from the high words
+// of the two (their binary exponents; NaN and infinity count as largest).  A
+// product with Y leaves a residual of up to |T| |Y| rounding errors where
+// substitution leaves one.  On smooth-kernel leaves (Gaussian kernels, 100 to
+// 1000 rows) products alone left backward errors of up to 2e12 u, with this
+// bound they stay within four times substitution's 0.2 to 0.4 u; Gaussian
+// random leaves of 512 rows reach 20, so ordinary leaves keep the products.
+__device__ inline unsigned high_abs(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+__device__ inline bool ill_conditioned(unsigned tri, unsigned inv) {
+  const unsigned et = tri >> 20, ei = inv >> 20;
+  return et == 2047 || ei == 2047 || et + ei >= 2 * 1023 + 6;
+}
+// The same over a CTA: every thread's high words go in, a barrier, and every
+// thread has the answer.  slots: one per warp.
+template <int WARPS>
+__device__ inline bool ill_conditioned_cta(uint2 *slots, unsigned tri, unsigned inv) {
+  tri = __reduce_max_sync(0xffffffffu, tri);
+  inv = __reduce_max_sync(0xffffffffu, inv);
+  if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = make_uint2(tri, inv);
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    tri = max(tri, slots[w].x);
+    inv = max(inv, slots[w].y);
+  }
+  return ill_conditioned(tri, inv);
+}
+
 // ---- inverses of the outer diagonal blocks (two-level factorization).
 //
 // Outer block J (rows / columns j0 .. j0 + obe of a leaf) starts as its
@@ -971,6 +998,21 @@ __global__ void __launch_bounds__(kInvThreads)
   // own data), so that a thread's loads overlap
   const T *safe = tk.D + j0 + (long long)j0 * tk.ldd;
   constexpr int kAhead = sizeof(T) == 8 ? 2 : 4;  // columns whose loads overlap
+  unsigned largest = 0, largest_t = 0;  // FP64: high words of max|inverse|, max|triangle|
+  constexpr int kTri = 128 * NB / kInvThreads;
+  T tri[kTri];
+  if constexpr (sizeof(T) == 8) {
+    // U's part inside the panels, whose inverses stand in for it below: loads
+    // under way during the main ones
+    if (upper) {
+#pragma unroll
+      for (int q = 0; q < kTri; ++q) {
+        const int e = min(tid + q * kInvThreads, ob * NB - 1);
+        const int c = min(e / NB, obe - 1), i = min(c / NB * NB + e % NB, c);
+        tri[q] = tk.D[j0 + i + (long long)(j0 + c) * tk.ldd];
+      }
+    }
+  }
 #pragma unroll kAhead
   for (int c = warp; c < ob; c += kInvThreads / 32) {
     const int pc = c / NB;
@@ -985,9 +1027,22 @@ __global__ void __launch_bounds__(kInvThreads)
       in[q] = diag ? i < live : (upper ? pi < pc : pi > pc) && i < obe && c < obe;
       v[q] = *(in[q] ? (diag ? icol : dcol) + i : safe);
     }
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool diag = (lane + 32 * q) / NB == pc;
+        largest_t = max(largest_t, in[q] && !diag ? high_abs(v[q]) : 0u);
+      }
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (lane + 32 * q < ob) X[lane + 32 * q + c * ld] = in[q] ? v[q] : T(0);
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (upper) {
+#pragma unroll
+      for (int q = 0; q < kTri; ++q) largest_t = max(largest_t, high_abs(tri[q]));
+    }
   }
   __syncthreads();
   for (int b = NB; b < ob; b *= 2) {
@@ -1010,8 +1065,177 @@ __global__ void __launch_bounds__(kInvThreads)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = lane + 32 * q;
-      if (i < ob) dst[i + c * ob] = (i < obe && c < obe) ? X[i + c * ld] : T(0);
+      const T v = i < obe && c < obe ? X[i + c * ld] : T(0);
+      if (i < ob) dst[i + c * ob] = v;
+      if constexpr (sizeof(T) == 8) largest = max(largest, high_abs(v));
     }
+  if constexpr (sizeof(T) == 8) {
+    __shared__ uint2 slots[kInvThreads / 32];
+    const bool ill = ill_conditioned_cta<kInvThreads / 32>(
+        slots, upper ? largest_t : 1023u << 20, largest);  // max|L| = 1
+    if (tid == 0) tk.ill_b[2 * J + upper] = ill;
+    if (ill)  // leaf_block_solve_kernel solves, the product with this copies
+      for (int e = tid; e < ob * ob; e += kInvThreads)
+        dst[e] = e % ob == e / ob && e / ob < obe ? T(1) : T(0);
+  }
+}
+
+// ---- FP64 solves with a diagonal triangle.
+
+constexpr int kSolveThreads = 128;
+
+// x <- T^{-1} x by substitution, a thread per column (x: this thread's, or
+// null), T (order x order, unit-lower or upper) column-major in global memory
+// and staged as 32 x 32 blocks in Ts.  All kSolveThreads threads call it.  Only
+// ill-conditioned triangles come here: 32 rows at a time in registers.
+template <bool UPPER>
+__device__ void substitute_columns(const double *T, long long ldt, int order, double *x,
+                                   double *Ts) {
+  const int nblk = (order + 31) / 32;
+  auto stage = [&](int bi, int bk) {  // the identity beyond the triangle's order
+    __syncthreads();  // the previous block's reads are done
+    for (int e = threadIdx.x; e < 32 * 32; e += kSolveThreads) {
+      const int i = 32 * bi + e % 32, k = 32 * bk + e / 32;
+      Ts[e] = i < order && k < order ? T[i + k * ldt] : i == k ? 1.0 : 0.0;
+    }
+    __syncthreads();
+  };
+  for (int s = 0; s < nblk; ++s) {
+    const int bi = UPPER ? nblk - 1 - s : s;
+    double v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = x && 32 * bi + i < order ? x[32 * bi + i] : 0.0;
+    for (int q = 0; q < s; ++q) {
+      const int bk = UPPER ? nblk - 1 - q : q;
+      stage(bi, bk);
+      for (int k = 0; k < 32; ++k) {
+        const double xk = x && 32 * bk + k < order ? x[32 * bk + k] : 0.0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] -= Ts[i + 32 * k] * xk;
+      }
+    }
+    stage(bi, bi);
+#pragma unroll
+    for (int kk = 0; kk < 32; ++kk) {
+      const int k = UPPER ? 31 - kk : kk;
+      if (UPPER) v[k] /= Ts[k + 32 * k];
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (UPPER ? i < k : i > k) v[i] -= Ts[i + 32 * k] * v[k];
+    }
+    if (x) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (32 * bi + i < order) x[32 * bi + i] = v[i];
+    }
+  }
+}
+
+// The panel's rows of a chunk of 64 columns times the inverse of the panel's
+// triangle, in place: one rank-NB DMMA product of operands that are all read
+// before the first store.  grid (column chunk, leaf).  Against items of the tile
+// GEMM, which cannot substitute: 5.5 instead of 5.7 us a launch for one leaf of
+// 512 rows and 592 columns, 125 instead of 157 us in all inside the outer blocks
+// of 512 such leaves.  Every CTA decides from the inverse it loads anyway (marks
+// left by the panel kernel took that 1.5 us each).
+constexpr int kSolveCols = 64;
+
+template <int NB, bool UPPER>
+__global__ void __launch_bounds__(kSolveThreads)
+    leaf_panel_solve_kernel(const LeafFactorTask<double> *__restrict__ tasks, int panel, int b0,
+                            int b1, int with_x) {
+  constexpr int LD = NB + 4;                  // conflict-free fragments
+  constexpr int WM = NB / 16, WN = 4 / WM;    // warps over rows, columns
+  constexpr int NT = kSolveCols / WN / 8;     // column blocks of a warp
+  constexpr int PER = kSolveCols / 4 * NB / 32;  // values of a thread
+  __shared__ __align__(16) double xs[kSolveCols * LD > 32 * 32 ? kSolveCols * LD : 32 * 32];
+  const LeafFactorTask<double> tk = tasks[blockIdx.y];
+  const int n = tk.n, k0 = panel * NB;
+  if (k0 >= n) return;
+  const int kb = min(NB, n - k0);
+  const int nd = max(0, min(b1, n) - b0), total = nd + (with_x ? tk.ncols : 0);
+  const int c0 = blockIdx.x * kSolveCols;
+  if (c0 >= total) return;
+  // column c of this CTA (the last one repeated), at the panel's first row
+  auto column = [&](int c) {
+    const int q = min(c0 + c, total - 1);
+    return q < nd ? tk.D + k0 + (long long)(b0 + q) * tk.ldd
+                  : tk.X + k0 + (long long)(q - nd) * tk.ldx;
+  };
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int wm = warp % WM * 16, wn = warp / WM * (8 * NT);
+  const double *inv = (UPPER ? tk.Uinv : tk.Linv) + (size_t)panel * NB * NB + wm + g;
+  double a[NB / 4][2], v[PER], tri[NB * NB / kSolveThreads];
+  const int row = lane % NB, c1 = warp * (kSolveCols / 4) + lane / NB;
+#pragma unroll
+  for (int u = 0; u < PER; ++u) v[u] = column(c1 + u * (32 / NB))[min(row, kb - 1)];
+#pragma unroll
+  for (int k = 0; k < NB / 4; ++k) {
+    a[k][0] = inv[(4 * k + t) * NB];
+    a[k][1] = inv[(4 * k + t) * NB + 8];
+  }
+  unsigned largest = 0, largest_t = 1023u << 20;  // max|L| = 1
+  if (UPPER) {
+#pragma unroll
+    for (int q = 0; q < NB * NB / kSolveThreads; ++q) {
+      const int e = tid + q * kSolveThreads, j = min(e / NB, kb - 1), i = min(e % NB, j);
+      tri[q] = tk.D[k0 + i + (long long)(k0 + j) * tk.ldd];
+    }
+    largest_t = 0;
+#pragma unroll
+    for (int q = 0; q < NB * NB / kSolveThreads; ++q) largest_t = max(largest_t, high_abs(tri[q]));
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) xs[(c1 + q * (32 / NB)) * LD + row] = row < kb ? v[q] : 0.0;
+#pragma unroll
+  for (int k = 0; k < NB / 4; ++k) largest = max(largest, max(high_abs(a[k][0]), high_abs(a[k][1])));
+  __shared__ uint2 slots[kSolveThreads / 32];
+  if (ill_conditioned_cta<kSolveThreads / 32>(slots, largest_t, largest)) {
+    double *x = tid < kSolveCols && c0 + tid < total ? column(tid) : nullptr;
+    substitute_columns<UPPER>(tk.D + k0 + k0 * tk.ldd, tk.ldd, kb, x, xs);
+    return;
+  }
+  double c[NT][4];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[nt][q] = 0.0;
+#pragma unroll
+  for (int k = 0; k < NB / 4; ++k)
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+      dmma64(c[nt], a[k][0], a[k][1], xs[(wn + 8 * nt + g) * LD + 4 * k + t]);
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int col = wn + 8 * nt + 2 * t + u;
+      if (c0 + col >= total) continue;
+      double *d = column(col) + wm + g;
+      if (wm + g < kb) d[0] = c[nt][u];
+      if (wm + g + 8 < kb) d[8] = c[nt][2 + u];
+    }
+}
+
+// The CTAs of a leaf (grid (CTAs, leaf)) take its chunks of kSolveThreads
+// columns in turn.
+template <bool UPPER>
+__global__ void __launch_bounds__(kSolveThreads)
+    leaf_block_solve_kernel(const LeafFactorTask<double> *__restrict__ tasks, int ob, int J) {
+  __shared__ __align__(16) double Ts[32 * 32];
+  const LeafFactorTask<double> &tk = tasks[blockIdx.y];
+  const int n = tk.n, j0 = J * ob;
+  if (j0 >= n || !tk.ill_b[2 * J + UPPER]) return;
+  const int obe = min(ob, n - j0);
+  const int nd = UPPER ? 0 : n - j0 - obe, total = nd + tk.ncols;
+  for (int c0 = blockIdx.x * kSolveThreads; c0 < total; c0 += gridDim.x * kSolveThreads) {
+    const int c = c0 + (int)threadIdx.x;
+    double *x = nullptr;
+    if (c < nd) x = tk.D + j0 + (long long)(j0 + obe + c) * tk.ldd;
+    else if (c < total) x = tk.X + j0 + (long long)(c - nd) * tk.ldx;
+    substitute_columns<UPPER>(tk.D + j0 + j0 * tk.ldd, tk.ldd, obe, x, Ts);
+  }
 }
 
 }  // namespace
@@ -1109,6 +1333,29 @@ void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb
   else if (nb == 32) go(leaf_block_inverse_kernel<T, 32>);
   else if (nb == 16) go(leaf_block_inverse_kernel<T, 16>);
   else throw CudaError{cudaErrorInvalidValue};
+  HODLR_LAUNCH_CHECK();
+}
+
+void launch_leaf_panel_solve(const LeafFactorTask<double> *tasks, int count, int max_cols, int nb,
+                             int panel, int b0, int b1, bool with_x, bool upper, cudaStream_t s) {
+  if (count <= 0 || max_cols <= 0) return;
+  const dim3 grid(cdiv(max_cols, kSolveCols), count);
+  auto go = [&](auto kern) {
+    kern<<<grid, kSolveThreads, 0, s>>>(tasks, panel, b0, b1, with_x ? 1 : 0);
+  };
+  if (nb == 32) upper ? go(leaf_panel_solve_kernel<32, true>) : go(leaf_panel_solve_kernel<32, false>);
+  else if (nb == 16) upper ? go(leaf_panel_solve_kernel<16, true>) : go(leaf_panel_solve_kernel<16, false>);
+  else throw CudaError{cudaErrorInvalidValue};
+  HODLR_LAUNCH_CHECK();
+}
+
+void launch_leaf_block_solve(const LeafFactorTask<double> *tasks, int count, int max_cols, int ob,
+                             int J, bool upper, cudaStream_t s) {
+  if (count <= 0 || max_cols <= 0) return;
+  // few CTAs per leaf where there are many leaves: nearly always they have nothing to do
+  const dim3 grid(std::min(cdiv(max_cols, kSolveThreads), std::max(1, 1024 / count)), count);
+  if (upper) leaf_block_solve_kernel<true><<<grid, kSolveThreads, 0, s>>>(tasks, ob, J);
+  else leaf_block_solve_kernel<false><<<grid, kSolveThreads, 0, s>>>(tasks, ob, J);
   HODLR_LAUNCH_CHECK();
 }
 

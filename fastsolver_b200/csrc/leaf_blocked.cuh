@@ -4,7 +4,7 @@
 
 namespace hodlr {
 
-// Panel width: the panel (n x NB) lives in shared memory, so it narrows for
+// Panel width: the panel (n x NB) lives in registers, so it narrows for
 // leaves above 512 rows (the library accepts leaves of up to 1024 rows).
 template <typename T>
 inline int leaf_nb(int max_n) {
@@ -24,6 +24,8 @@ struct LeafFactorTask {
   int *swapflag;   // npanels: panel had row interchanges
   T *LinvB;        // nblocks x OB x OB: inverses of the unit-lower outer diagonal blocks
   T *UinvB;        // nblocks x OB x OB: inverses of the upper outer diagonal blocks
+  int *ill_b;      // nblocks x {L, U} (FP64, with LinvB): 1 where the outer block's
+                   // triangle is too ill-conditioned for its inverse
   long long ldd;
   long long ldx;
   int n;
@@ -46,6 +48,8 @@ void launch_leaf_init(const LeafFactorTask<T> *tasks, int count, int *info, cuda
 // nb x nb inverses, into task.LinvB + J ob^2 (column-major, ld ob, zero
 // outside the leaf); with `upper`, the inverses of the upper diagonal blocks
 // of all `nblocks` blocks into task.UinvB (J unused).
+// An FP64 triangle that is too ill-conditioned for its inverse leaves the
+// identity here and its mark in task.ill_b.
 template <typename T>
 void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb, int ob, int J,
                                bool upper, int nblocks, cudaStream_t s);
@@ -58,5 +62,18 @@ void launch_leaf_panel(const LeafFactorTask<T> *tasks, int count, int max_n, int
 template <typename T>
 void launch_leaf_laswp(const LeafFactorTask<T> *tasks, int count, int max_cols, int nb, int p0,
                        int np, int a0, int a1, int b0, int b1, bool with_x, cudaStream_t s);
+
+// FP64: the panel's rows of the D columns [b0, b1) (clamped to each leaf's n)
+// and, with with_x, of X multiplied by the inverse of the panel's unit-lower
+// diagonal triangle (upper: of its upper one), or solved with the triangle by
+// substitution where that is too ill-conditioned.  max_cols: an upper bound of
+// the columns in any leaf.
+void launch_leaf_panel_solve(const LeafFactorTask<double> *tasks, int count, int max_cols, int nb,
+                             int panel, int b0, int b1, bool with_x, bool upper, cudaStream_t s);
+// FP64: outer block J's rows of the D columns right of the block (not with
+// `upper`) and of X solved by substitution in the leaves whose ill_b marks the
+// block's triangle; nothing elsewhere.
+void launch_leaf_block_solve(const LeafFactorTask<double> *tasks, int count, int max_cols, int ob,
+                             int J, bool upper, cudaStream_t s);
 
 }  // namespace hodlr

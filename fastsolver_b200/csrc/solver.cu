@@ -95,12 +95,7 @@ void path_need(const Tree &t, bool factor, int chunk, size_t &part, size_t &wfin
 // One step of the two-level blocked leaf factorization (see LeafPlan and
 // leaf_blocked.cu) with its GEMM items on the host.
 template <typename T>
-struct HostStep {
-  using Kind = typename LeafPlan<T>::Kind;
-  Kind kind;
-  int k0 = 0, panel = 0, block = 0, np = 0;
-  int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
-  bool with_x = false;
+struct HostStep : LeafPlan<T>::StepInfo {
   std::vector<GemmItem<T, T>> it;
   std::vector<GemmSeg<T>> sg;
   void add(T *C, long long ldc, int M, int N, const T *A, long long lda, const T *B,
@@ -119,7 +114,8 @@ struct HostStep {
 // work in a step contributes no item.  binv: block-row solves by the inverses
 // of the outer diagonal blocks, in place on the block's rows, which one GEMM
 // tile row (128) covers (the GEMM launchers run launches of items of at most
-// 128 rows as one tile row).
+// 128 rows as one tile row).  FP64 steps solve with the triangles themselves
+// where these are ill-conditioned.
 template <typename T>
 void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int nblocks, bool binv,
                 std::vector<HostStep<T>> &fwd, std::vector<HostStep<T>> &bwd) {
@@ -139,6 +135,28 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
     return st;
   };
   constexpr int kAll = 1 << 30;
+  constexpr bool kSubst = std::is_same<T, double>::value;
+  // the panel's rows of the D columns [b0, b1) and X by its triangle
+  auto panel_solve = [&](int panel, int b0, int b1, bool with_x, bool upper) {
+    HostStep<T> st = step(Plan::kPanelSolve);
+    st.panel = panel;
+    st.b0 = b0; st.b1 = b1;
+    st.with_x = with_x;
+    st.upper = upper;
+    for (const LeafFactorTask<T> &k : tasks)
+      if (panel * NB < k.n)
+        st.cols = std::max(st.cols, std::max(0, std::min(b1, k.n) - b0) + (with_x ? k.ncols : 0));
+    return st;
+  };
+  auto block_solve = [&](int J, bool upper) {
+    HostStep<T> st = step(Plan::kBlockSolve);
+    st.block = J;
+    st.upper = upper;
+    for (const LeafFactorTask<T> &k : tasks)
+      if (J * OB < k.n)
+        st.cols = std::max(st.cols, (upper ? 0 : std::max(0, k.n - J * OB - OB)) + k.ncols);
+    return st;
+  };
   for (int J = 0; J < nblocks; ++J) {
     const int j0 = J * OB;
     // the block's panels: factor, interchange and update inside the block columns
@@ -157,11 +175,11 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         const int rest = k.n - k0 - kb;
         const T *Li = k.Linv + (size_t)pi * NB * NB;
         T *U12 = k.D + k0 + (long long)(k0 + kb) * k.ldd;
-        tr.add(U12, k.ldd, kb, N, Li, NB, U12, k.ldd, kb, false);
+        if (!kSubst) tr.add(U12, k.ldd, kb, N, Li, NB, U12, k.ldd, kb, false);
         up.add(k.D + (k0 + kb) + (long long)(k0 + kb) * k.ldd, k.ldd, rest, N,
                k.D + (k0 + kb) + (long long)k0 * k.ldd, k.ldd, U12, k.ldd, kb, true);
       }
-      fwd.push_back(std::move(tr));
+      fwd.push_back(kSubst ? panel_solve(pi, k0 + NB, j0 + OB, false, false) : std::move(tr));
       fwd.push_back(std::move(up));
     }
     // the block's interchanges on the columns left and right of it and on X
@@ -183,6 +201,7 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         tr.add(Xr, k.ldx, obe, k.ncols, Li, OB, Xr, k.ldx, obe, false, 1);
       }
       fwd.push_back(std::move(tr));
+      if (kSubst) fwd.push_back(block_solve(J, false));
     }
     // block rows: U12 = L11^{-1} A12 by panels on R = (D right of the block | X)
     for (int p = 0; p < (binv ? 0 : P); ++p) {
@@ -197,13 +216,15 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         const T *Li = k.Linv + (size_t)pi * NB * NB;
         T *Dr = k.D + k0 + (long long)(j0 + obe) * k.ldd;
         T *Xr = k.X + k0;
-        tr.add(Dr, k.ldd, kb, nd, Li, NB, Dr, k.ldd, kb, false);
-        tr.add(Xr, k.ldx, kb, k.ncols, Li, NB, Xr, k.ldx, kb, false);
+        if (!kSubst) {
+          tr.add(Dr, k.ldd, kb, nd, Li, NB, Dr, k.ldd, kb, false);
+          tr.add(Xr, k.ldx, kb, k.ncols, Li, NB, Xr, k.ldx, kb, false);
+        }
         const T *L = k.D + (k0 + kb) + (long long)k0 * k.ldd;
         up.add(Dr + kb, k.ldd, below, nd, L, k.ldd, Dr, k.ldd, kb, true);
         up.add(Xr + kb, k.ldx, below, k.ncols, L, k.ldd, Xr, k.ldx, kb, true);
       }
-      fwd.push_back(std::move(tr));
+      fwd.push_back(kSubst ? panel_solve(pi, j0 + OB, kAll, true, false) : std::move(tr));
       fwd.push_back(std::move(up));
     }
     // trailing update of depth OB: A22 -= L21 U12 on R, rows below the block
@@ -233,6 +254,7 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
                2);
       }
       bwd.push_back(std::move(tr));
+      if (kSubst) bwd.push_back(block_solve(J, true));
     }
     for (int p = binv ? -1 : P - 1; p >= 0; --p) {
       const int pi = J * P + p, k0 = pi * NB;
@@ -241,11 +263,12 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         if (k0 >= k.n) continue;
         const int kb = std::min(NB, k.n - k0);
         T *Xk = k.X + k0;
-        tr.add(Xk, k.ldx, kb, k.ncols, k.Uinv + (size_t)pi * NB * NB, NB, Xk, k.ldx, kb, false);
+        if (!kSubst)
+          tr.add(Xk, k.ldx, kb, k.ncols, k.Uinv + (size_t)pi * NB * NB, NB, Xk, k.ldx, kb, false);
         up.add(k.X + j0, k.ldx, k0 - j0, k.ncols, k.D + j0 + (long long)k0 * k.ldd, k.ldd, Xk,
                k.ldx, kb, true);
       }
-      bwd.push_back(std::move(tr));
+      bwd.push_back(kSubst ? panel_solve(pi, 0, 0, true, true) : std::move(tr));
       bwd.push_back(std::move(up));
     }
     HostStep<T> big = step(Plan::kUpdate);
@@ -297,6 +320,7 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
     lp.UinvB.ensure((size_t)nleaf * lp.nblocks * OB * OB);
   }
   lp.swapflag.ensure((size_t)nleaf * max_panels);
+  if (binv && std::is_same<T, double>::value) lp.ill_b.ensure((size_t)nleaf * lp.nblocks * 2);
   std::vector<LeafFactorTask<T>> tasks(nleaf);
   lp.laswp_cols = 0;
   for (int q = 0; q < nleaf; ++q) {
@@ -311,6 +335,7 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
     k.Linv = lp.Linv.p + (size_t)q * max_panels * NB * NB;
     k.Uinv = lp.Uinv.p + (size_t)q * max_panels * NB * NB;
     k.swapflag = lp.swapflag.p + (size_t)q * max_panels;
+    k.ill_b = lp.ill_b.p ? lp.ill_b.p + (size_t)q * lp.nblocks * 2 : nullptr;
     k.LinvB = binv ? lp.LinvB.p + (size_t)q * lp.nblocks * OB * OB : nullptr;
     k.UinvB = binv ? lp.UinvB.p + (size_t)q * lp.nblocks * OB * OB : nullptr;
     k.n = nd.nrow;
@@ -328,21 +353,15 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
   auto upload = [](const std::vector<HostStep<T>> &src, std::vector<std::unique_ptr<Step>> &dst) {
     for (const HostStep<T> &h : src) {
       auto st = std::make_unique<Step>();
-      st->kind = h.kind;
-      st->k0 = h.k0;
-      st->panel = h.panel;
-      st->block = h.block;
-      st->np = h.np;
-      st->a0 = h.a0; st->a1 = h.a1; st->b0 = h.b0; st->b1 = h.b1;
-      st->with_x = h.with_x;
+      static_cast<typename LeafPlan<T>::StepInfo &>(*st) = h;
       if (h.kind == LeafPlan<T>::kTrsm || h.kind == LeafPlan<T>::kUpdate) st->g.set(h.it, h.sg);
       dst.push_back(std::move(st));
     }
   };
   upload(fwd, lp.fwd);
   upload(bwd, lp.bwd);
-  lp.fwd_per_block = binv ? 4 * P + 4 : 6 * P + 2;
-  lp.bwd_per_block = binv ? 2 : 2 * P + 1;
+  lp.fwd_per_block = (int)lp.fwd.size() / std::max(lp.nblocks, 1);
+  lp.bwd_per_block = (int)lp.bwd.size() / std::max(lp.nblocks, 1);
 }
 
 template <typename TA, typename TC, typename TACC>
@@ -629,6 +648,18 @@ void run_leaf_step(Profiler &pf, const LeafSet<T> &L, const S &st, const GemmIte
       launch_leaf_block_inverse<T>(L.tasks, L.nleaf, L.nb, L.ob, st.block, false, 0, s);
       break;
     }
+    case Plan::kPanelSolve:
+    case Plan::kBlockSolve: {
+      if constexpr (std::is_same<T, double>::value) {
+        PhaseScope pt(pf, PH_LEAF_TRSM, s);
+        if (st.kind == Plan::kPanelSolve)
+          launch_leaf_panel_solve(L.tasks, L.nleaf, st.cols, L.nb, st.panel, st.b0, st.b1,
+                                  st.with_x, st.upper, s);
+        else
+          launch_leaf_block_solve(L.tasks, L.nleaf, st.cols, L.ob, st.block, st.upper, s);
+      }
+      break;
+    }
     case Plan::kTrsm:
     case Plan::kUpdate: {
       if (n == 0) break;
@@ -656,10 +687,10 @@ void run_leaf_plan(Profiler &pf, const LeafPlan<T> &lp, int *info, cudaStream_t 
   }
   {
     PhaseScope ps(pf, PH_GETRS, s);
+    Profiler off;  // (the backward solve's steps count as PH_GETRS alone)
     for (const auto &st : lp.bwd)
-      if (st->g.n > 0)
-        run_gemm<T, T, T>(st->g, false, st->kind == LeafPlan<T>::kTrsm ? T(1) : T(-1),
-                          st->kind == LeafPlan<T>::kTrsm ? T(0) : T(1), s);
+      run_leaf_step<T>(off, L, *st, st->g.items.p, st->g.segs.p, st->g.n, st->g.max_m, st->g.max_n,
+                       info, s);
   }
 }
 
@@ -898,13 +929,8 @@ void merge_leaf_plans(const std::vector<const LeafPlan<T> *> &src, const std::ve
   // backward lists start at each system's own last block
   auto merge_step = [&](const Step &proto, const std::vector<const Step *> &parts) {
     auto st = std::make_unique<Step>();
-    st->kind = proto.kind;
-    st->k0 = proto.k0;
-    st->panel = proto.panel;
-    st->block = proto.block;
-    st->np = proto.np;
-    st->a0 = proto.a0; st->a1 = proto.a1; st->b0 = proto.b0; st->b1 = proto.b1;
-    st->with_x = proto.with_x;
+    static_cast<typename LeafPlan<T>::StepInfo &>(*st) = proto;
+    for (const Step *p : parts) st->cols = std::max(st->cols, p->cols);
     if (proto.kind == LeafPlan<T>::kTrsm || proto.kind == LeafPlan<T>::kUpdate) {
       ItemAcc<T, T> acc;
       for (const Step *p : parts) acc.add(p->g);
@@ -1045,10 +1071,10 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
   const int OB = std::max(NB, leaf_ob_auto64((long long)tasks.size() * max_n, max_n));
   const int P = OB / NB, nblocks = cdiv(max_n, OB), np = nblocks * P;
   const bool binv = P > 1;
-  // per leaf: panel inverses, block inverses, row order, interchange flags
+  // per leaf: panel inverses, block inverses, row order, interchange flags, marks
   const size_t w_inv = (size_t)np * NB * NB, w_blk = binv ? (size_t)nblocks * OB * OB : 0;
   // (in doubles; even, so that every leaf's inverses start on 16 bytes)
-  const size_t ints = ((size_t)max_n + np + 3) / 4 * 2;
+  const size_t ints = ((size_t)max_n + np + 2 * nblocks + 3) / 4 * 2;
   const size_t per = 2 * w_inv + 2 * w_blk + ints;
   double *w = static_cast<double *>(scratch(sizeof(double) * per * tasks.size()));
   for (size_t q = 0; q < tasks.size(); ++q) {
@@ -1061,6 +1087,7 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
     int *ip = reinterpret_cast<int *>(b + 2 * w_inv + 2 * w_blk);
     if (!k.perm) k.perm = ip;
     k.swapflag = ip + max_n;
+    k.ill_b = k.swapflag + np;
   }
   std::vector<HostStep<T>> fwd, bwd;
   leaf_steps<T>(tasks, NB, OB, nblocks, binv, fwd, bwd);

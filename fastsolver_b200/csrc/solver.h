@@ -112,16 +112,22 @@ struct LeafPlan {
   DevBuf<T> Linv, Uinv;
   DevBuf<T> LinvB, UinvB;  // outer-block inverses (two-level plans with ob <= 128)
   DevBuf<int> swapflag;
+  DevBuf<int> ill_b;  // FP64: marks of ill-conditioned blocks (LeafFactorTask)
   std::vector<LeafFactorTask<T>> host_tasks;  // for apply plans with these factors
   int nleaf = 0, max_n = 0, laswp_cols = 0, nb = 0, ob = 0;
-  enum Kind { kPanel, kLaswp, kTrsm, kUpdate, kBlockInv };
-  struct Step {
+  // kPanelSolve, kBlockSolve (FP64): launch_leaf_panel_solve, launch_leaf_block_solve
+  enum Kind { kPanel, kLaswp, kTrsm, kUpdate, kBlockInv, kPanelSolve, kBlockSolve };
+  struct StepInfo {
     Kind kind = kPanel;
-    int k0 = 0, panel = 0;          // kPanel: the panel; kLaswp: first panel
-    int block = 0;                  // kBlockInv: the outer block
+    int k0 = 0, panel = 0;          // kPanel, kPanelSolve: the panel; kLaswp: first panel
+    int block = 0;                  // kBlockInv, kBlockSolve: the outer block
     int np = 0;                     // kLaswp: panels applied
-    int a0 = 0, a1 = 0, b0 = 0, b1 = 0;  // kLaswp: D column ranges (clamped per leaf)
-    bool with_x = false;            // kLaswp: X columns too
+    int a0 = 0, a1 = 0, b0 = 0, b1 = 0;  // D column ranges (clamped per leaf)
+    bool with_x = false;            // X columns too
+    bool upper = false;             // kPanelSolve, kBlockSolve: with U
+    int cols = 0;                   // ... and the most columns of a leaf
+  };
+  struct Step : StepInfo {
     GemmLaunch<T, T> g;             // kTrsm (C = A B) / kUpdate (C -= A B)
   };
   // fwd: the steps of block 0, then block 1, ... (fwd_per_block each);

@@ -346,3 +346,36 @@ def test_panel_inverse_residual(fs, cuda, prec, n, s, shift):
     lim = n * u * (2 * a(L) @ w + 3 * a(L) @ (a(U) @ (a(np.linalg.inv(U)) @ w)))
     r = a((B - A.astype(np.longdouble) @ h.solution()).astype(np.float64))[p]
     assert (r <= lim).all()
+
+
+@pytest.mark.parametrize("call", ["leaf", 0, 16, 128, 256])
+@pytest.mark.parametrize("n,s", [(17, 0.5), (31, 0.3), (33, 0.3), (100, 0.1), (128, 0.1), (129, 0.1),
+                                 (257, 0.1), (512, 0.02), (512, 0.1), (513, 0.1), (1000, 0.1)])
+def test_ill_conditioned_leaf_residual(fs, cuda, call, n, s):
+    """A leaf of a smooth kernel, as the leaf task body and as a whole solve (by
+    its outer block width): triangles with max|T| max|T^{-1}| above 2^7 are
+    solved by substitution, so the residual is that of the factors plus what
+    the inverses of the others leave."""
+    A = _smooth_kernel(n, s, 1e-12)
+    B = np.random.default_rng(n).standard_normal((n, 70))
+    order = 32 if n <= 512 else 16
+    if call == "leaf":
+        D, X = dev(A, n + 1), dev(B, n + 3)
+        import torch
+        assert fs.leaf_solve(D, X, torch.zeros(n, dtype=torch.int32, device="cuda")) == 0
+        x = host(X)
+    else:
+        h = fs.HodlrMatrix(70, n, 1, 1024).create_tree()
+        h.schedule = dict(leaf_ob64=call)
+        h.set_matrix(A)
+        h.set_rhs(B)
+        fs.FastSolver().bfs_solve(h)
+        x = h.solution()
+    if call == 128 or (n > 512 and call != 16):
+        order = 128
+    L, U, p = _gepp(A)
+    # per triangle |b - T x| <= 2 n u |T| |Y| |T| |x| with (|T| |Y|)_ij <= 2^7 order
+    lim = n * 2.0 ** -53 * (3 + 2 * 2 ** 7 * order ** 1.5) * np.linalg.norm(
+        np.abs(L) @ (np.abs(U) @ np.abs(x)), axis=0)
+    r = np.linalg.norm((B - A.astype(np.longdouble) @ x).astype(np.float64), axis=0)
+    assert (r <= lim).all()
