@@ -974,16 +974,15 @@ __host__ __device__ inline size_t inv_words(int ob, int nb) {
   return (size_t)inv_ld<T>(ob) * ob + (size_t)inv_ld<T>(h) * h;
 }
 
-// grid (leaf, 1): block J0's lower triangle; grid (leaf, blocks) with upper:
-// every block's upper one
+// grid (leaf, block J0, J0 + 1, ...)
 template <typename T, int NB>
 __global__ void __launch_bounds__(kInvThreads)
-    leaf_block_inverse_kernel(const LeafFactorTask<T> *__restrict__ tasks, int ob, int J0,
+    leaf_block_inverse_kernel(const LeafFactorTask<T> *__restrict__ tasks, int ob, int J0, int slots,
                               int upper) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const LeafFactorTask<T> tk = tasks[blockIdx.x];
   const int n = tk.n;
-  const int J = upper ? (int)blockIdx.y : J0;  // upper: every block, one per grid row
+  const int J = J0 + (int)blockIdx.y;
   const int j0 = J * ob;
   if (j0 >= n) return;
   const int obe = min(ob, n - j0);
@@ -1060,7 +1059,7 @@ __global__ void __launch_bounds__(kInvThreads)
     }
   }
   // zero outside the leaf's part of the block (rows / columns >= obe)
-  T *dst = (upper ? tk.UinvB : tk.LinvB) + (size_t)J * ob * ob;
+  T *dst = tk.Binv + (size_t)(J % slots) * ob * ob;
   for (int c = warp; c < ob; c += kInvThreads / 32)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -1319,15 +1318,15 @@ void launch_leaf_apply(const LeafFactorTask<T> *tasks, int count, int max_n, int
 }
 
 template <typename T>
-void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb, int ob, int J,
-                               bool upper, int nblocks, cudaStream_t s) {
-  if (count <= 0 || (upper && nblocks <= 0)) return;
-  if (ob > 128 || ob % nb) throw CudaError{cudaErrorInvalidValue};
-  dim3 grid(count, upper ? nblocks : 1);
+void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb, int ob, int J0,
+                               int blocks, int slots, bool upper, cudaStream_t s) {
+  if (count <= 0 || blocks <= 0) return;
+  if (ob > 128 || ob % nb || blocks > slots) throw CudaError{cudaErrorInvalidValue};
+  dim3 grid(count, blocks);
   const size_t smem = inv_words<T>(ob, nb) * sizeof(T);
   auto go = [&](auto kern) {
     raise_smem_limit(reinterpret_cast<const void *>(kern), smem);
-    kern<<<grid, kInvThreads, smem, s>>>(tasks, ob, J, upper ? 1 : 0);
+    kern<<<grid, kInvThreads, smem, s>>>(tasks, ob, J0, slots, upper ? 1 : 0);
   };
   if (nb == 64) go(leaf_block_inverse_kernel<T, 64>);
   else if (nb == 32) go(leaf_block_inverse_kernel<T, 32>);
@@ -1359,10 +1358,10 @@ void launch_leaf_block_solve(const LeafFactorTask<double> *tasks, int count, int
   HODLR_LAUNCH_CHECK();
 }
 
-template void launch_leaf_block_inverse<double>(const LeafFactorTask<double> *, int, int, int,
-                                                int, bool, int, cudaStream_t);
+template void launch_leaf_block_inverse<double>(const LeafFactorTask<double> *, int, int, int, int,
+                                                int, int, bool, cudaStream_t);
 template void launch_leaf_block_inverse<float>(const LeafFactorTask<float> *, int, int, int, int,
-                                               bool, int, cudaStream_t);
+                                               int, int, bool, cudaStream_t);
 
 template void launch_leaf_apply<double>(const LeafFactorTask<double> *, int, int, int, int,
                                         cudaStream_t);

@@ -22,9 +22,9 @@ struct LeafFactorTask {
   T *Linv;         // npanels x NB x NB: inverses of the unit-lower diagonal blocks
   T *Uinv;         // npanels x NB x NB: inverses of the upper diagonal blocks
   int *swapflag;   // npanels: panel had row interchanges
-  T *LinvB;        // nblocks x OB x OB: inverses of the unit-lower outer diagonal blocks
-  T *UinvB;        // nblocks x OB x OB: inverses of the upper outer diagonal blocks
-  int *ill_b;      // nblocks x {L, U} (FP64, with LinvB): 1 where the outer block's
+  T *Binv;         // slots x OB x OB: inverses of outer diagonal blocks' triangles, block J's
+                   // in slot J % slots (unit-lower forward, upper backward)
+  int *ill_b;      // nblocks x {L, U} (FP64, with Binv): 1 where the outer block's
                    // triangle is too ill-conditioned for its inverse
   long long ldd;
   long long ldx;
@@ -43,16 +43,15 @@ void launch_leaf_apply(const LeafFactorTask<T> *tasks, int count, int max_n, int
 
 template <typename T>
 void launch_leaf_init(const LeafFactorTask<T> *tasks, int count, int *info, cudaStream_t s);
-// Inverse of outer block J's unit-lower diagonal block (ob x ob, ob a
-// multiple of nb and at most 128) from the block's factored panels and their
-// nb x nb inverses, into task.LinvB + J ob^2 (column-major, ld ob, zero
-// outside the leaf); with `upper`, the inverses of the upper diagonal blocks
-// of all `nblocks` blocks into task.UinvB (J unused).
-// An FP64 triangle that is too ill-conditioned for its inverse leaves the
-// identity here and its mark in task.ill_b.
+// Inverses of the unit-lower (upper: the upper) diagonal triangles of the outer
+// blocks J0 .. J0 + blocks - 1 (ob x ob, ob a multiple of nb and at most 128, at
+// most `slots` blocks) from the blocks' factored panels and their nb x nb
+// inverses, into task.Binv (column-major, ld ob, zero outside the leaf).  An FP64
+// triangle that is too ill-conditioned for its inverse leaves the identity here
+// and its mark in task.ill_b.
 template <typename T>
-void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb, int ob, int J,
-                               bool upper, int nblocks, cudaStream_t s);
+void launch_leaf_block_inverse(const LeafFactorTask<T> *tasks, int count, int nb, int ob, int J0,
+                               int blocks, int slots, bool upper, cudaStream_t s);
 template <typename T>
 void launch_leaf_panel(const LeafFactorTask<T> *tasks, int count, int max_n, int nb, int k0,
                        int panel, int *info, cudaStream_t s);

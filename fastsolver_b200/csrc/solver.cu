@@ -46,6 +46,7 @@ struct PathSpec {
   TE *M = nullptr;     // per-node solve matrices, (2r)^2 each
   NodeStore *ns = nullptr;
   const LeafPlan<T> *factors = nullptr;  // apply paths: the blocked leaf factors
+  std::shared_ptr<LeafPlan<T>> leaf;     // factor paths: a built leaf plan to share, or null
   int nb_force = 0;                      // leaf panel width (0: by the largest leaf)
   int ob = 0;                            // leaf outer block width (0: one level)
   bool factor = false;
@@ -118,7 +119,7 @@ struct HostStep : LeafPlan<T>::StepInfo {
 // where these are ill-conditioned.
 template <typename T>
 void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int nblocks, bool binv,
-                std::vector<HostStep<T>> &fwd, std::vector<HostStep<T>> &bwd) {
+                int slots, std::vector<HostStep<T>> &fwd, std::vector<HostStep<T>> &bwd) {
   using Plan = LeafPlan<T>;
   const int P = OB / NB;
   auto step = [](typename Plan::Kind kind) {
@@ -194,7 +195,7 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
       for (const LeafFactorTask<T> &k : tasks) {
         if (j0 >= k.n) continue;
         const int obe = std::min(OB, k.n - j0);
-        const T *Li = k.LinvB + (size_t)J * OB * OB;
+        const T *Li = k.Binv + (size_t)(J % slots) * OB * OB;
         T *Dr = k.D + j0 + (long long)(j0 + obe) * k.ldd;
         T *Xr = k.X + j0;
         tr.add(Dr, k.ldd, obe, k.n - j0 - obe, Li, OB, Dr, k.ldd, obe, false, 1);
@@ -250,8 +251,8 @@ void leaf_steps(const std::vector<LeafFactorTask<T>> &tasks, int NB, int OB, int
         if (j0 >= k.n) continue;
         const int obe = std::min(OB, k.n - j0);
         T *Xk = k.X + j0;
-        tr.add(Xk, k.ldx, obe, k.ncols, k.UinvB + (size_t)J * OB * OB, OB, Xk, k.ldx, obe, false,
-               2);
+        tr.add(Xk, k.ldx, obe, k.ncols, k.Binv + (size_t)(J % slots) * OB * OB, OB, Xk, k.ldx, obe,
+               false, 2);
       }
       bwd.push_back(std::move(tr));
       if (kSubst) bwd.push_back(block_solve(J, true));
@@ -295,6 +296,18 @@ int leaf_ob_auto64(long long rows, int max_n) {
   return max_n > 512 || (max_n > 128 && rows * max_n >= (8 << 20)) ? 128 : 0;
 }
 
+// Slots of outer-block inverses per leaf.  FP32: all blocks, so that the upper
+// inverses are one launch.  FP64: as many as fit in 32 MB over all leaves, at
+// least one; lower and upper ones of all blocks took 0.5 GB at N = 262144 (512
+// leaves of 512 rows), where one launch per block instead of one for all costs 0.4 %
+// of the solve.
+template <typename T>
+int binv_slots(long long leaves, int nblocks, int ob) {
+  if (sizeof(T) == 4) return nblocks;
+  const long long fit = (32LL << 20) / std::max(1LL, leaves * ob * ob * (long long)sizeof(T));
+  return (int)std::min<long long>(nblocks, std::max(1LL, fit));
+}
+
 // The blocked factorization of every leaf of a tree as uploaded steps.
 template <typename T>
 void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long ldx,
@@ -316,8 +329,8 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
   const bool binv = P > 1 && OB <= 128;
   lp.binv = binv;
   if (binv) {
-    lp.LinvB.ensure((size_t)nleaf * lp.nblocks * OB * OB);
-    lp.UinvB.ensure((size_t)nleaf * lp.nblocks * OB * OB);
+    lp.slots = binv_slots<T>(nleaf, lp.nblocks, OB);
+    lp.Binv.ensure((size_t)nleaf * lp.slots * OB * OB);
   }
   lp.swapflag.ensure((size_t)nleaf * max_panels);
   if (binv && std::is_same<T, double>::value) lp.ill_b.ensure((size_t)nleaf * lp.nblocks * 2);
@@ -336,8 +349,7 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
     k.Uinv = lp.Uinv.p + (size_t)q * max_panels * NB * NB;
     k.swapflag = lp.swapflag.p + (size_t)q * max_panels;
     k.ill_b = lp.ill_b.p ? lp.ill_b.p + (size_t)q * lp.nblocks * 2 : nullptr;
-    k.LinvB = binv ? lp.LinvB.p + (size_t)q * lp.nblocks * OB * OB : nullptr;
-    k.UinvB = binv ? lp.UinvB.p + (size_t)q * lp.nblocks * OB * OB : nullptr;
+    k.Binv = binv ? lp.Binv.p + (size_t)q * lp.slots * OB * OB : nullptr;
     k.n = nd.nrow;
     k.ncols = factor_cols_all ? nd.col_beg + nd.ncol : m;
     k.info_slot = q;
@@ -349,7 +361,7 @@ void build_leaf_plan(const Tree &t, T *Dbase, long long ldd, T *Xbase, long long
   lp.fwd.clear();
   lp.bwd.clear();
   std::vector<HostStep<T>> fwd, bwd;
-  leaf_steps<T>(tasks, NB, OB, lp.nblocks, binv, fwd, bwd);
+  leaf_steps<T>(tasks, NB, OB, lp.nblocks, binv, lp.slots, fwd, bwd);
   auto upload = [](const std::vector<HostStep<T>> &src, std::vector<std::unique_ptr<Step>> &dst) {
     for (const HostStep<T> &h : src) {
       auto st = std::make_unique<Step>();
@@ -419,8 +431,13 @@ void build_path(const Tree &t, const PathSpec<T, TE> &sp, PathPlan<T, TE> &plan,
   plan.nleaf = (int)t.leaves.size();
   const int m = t.nrhs;
   if (sp.factor) {
-    build_leaf_plan<T>(t, sp.D, sp.ldd, sp.X, sp.ldx, sp.ipiv, sp.perm, true, m, plan.leaf,
-                       sp.nb_force, sp.ob);
+    if (sp.leaf) {
+      plan.leaf = sp.leaf;
+    } else {
+      if (!plan.leaf) plan.leaf = std::make_shared<LeafPlan<T>>();
+      build_leaf_plan<T>(t, sp.D, sp.ldd, sp.X, sp.ldx, sp.ipiv, sp.perm, true, m, *plan.leaf,
+                         sp.nb_force, sp.ob);
+    }
   } else {
     std::vector<LeafFactorTask<T>> at = sp.factors->host_tasks;
     for (size_t q = 0; q < at.size(); ++q) {
@@ -619,7 +636,7 @@ struct PhaseScope {
 template <typename T>
 struct LeafSet {
   const LeafFactorTask<T> *tasks;
-  int nleaf, max_n, laswp_cols, nb, ob;
+  int nleaf, max_n, laswp_cols, nb, ob, slots;
 };
 
 // Enqueues one step (a plan's Step or a HostStep) with its GEMM items on the
@@ -645,7 +662,7 @@ void run_leaf_step(Profiler &pf, const LeafSet<T> &L, const S &st, const GemmIte
     }
     case Plan::kBlockInv: {
       PhaseScope pt(pf, PH_LEAF_TRSM, s);
-      launch_leaf_block_inverse<T>(L.tasks, L.nleaf, L.nb, L.ob, st.block, false, 0, s);
+      launch_leaf_block_inverse<T>(L.tasks, L.nleaf, L.nb, L.ob, st.block, 1, L.slots, false, s);
       break;
     }
     case Plan::kPanelSolve:
@@ -671,26 +688,35 @@ void run_leaf_step(Profiler &pf, const LeafSet<T> &L, const S &st, const GemmIte
   }
 }
 
+// Before the backward steps of block J of nblocks: the upper inverses of it and
+// the blocks before it, as many as there are slots, unless they are there.
+template <typename T>
+void run_upper_inverses(const LeafSet<T> &L, int J, int nblocks, cudaStream_t s) {
+  if ((nblocks - 1 - J) % L.slots != 0) return;
+  const int J0 = std::max(0, J - L.slots + 1);
+  launch_leaf_block_inverse<T>(L.tasks, L.nleaf, L.nb, L.ob, J0, J - J0 + 1, L.slots, true, s);
+}
+
 template <typename T>
 void run_leaf_plan(Profiler &pf, const LeafPlan<T> &lp, int *info, cudaStream_t s) {
-  const LeafSet<T> L{lp.tasks.p, lp.nleaf, lp.max_n, lp.laswp_cols, lp.nb, lp.ob};
+  const LeafSet<T> L{lp.tasks.p, lp.nleaf, lp.max_n, lp.laswp_cols, lp.nb, lp.ob, lp.slots};
   {
     PhaseScope ps(pf, PH_GETRF, s);
     launch_leaf_init<T>(lp.tasks.p, lp.nleaf, info, s);
     for (const auto &st : lp.fwd)
       run_leaf_step<T>(pf, L, *st, st->g.items.p, st->g.segs.p, st->g.n, st->g.max_m, st->g.max_n,
                        info, s);
-    if (lp.binv) {  // the upper block inverses of every block, for the backward solve
-      PhaseScope pt(pf, PH_LEAF_TRSM, s);
-      launch_leaf_block_inverse<T>(lp.tasks.p, lp.nleaf, lp.nb, lp.ob, 0, true, lp.nblocks, s);
-    }
   }
   {
     PhaseScope ps(pf, PH_GETRS, s);
     Profiler off;  // (the backward solve's steps count as PH_GETRS alone)
-    for (const auto &st : lp.bwd)
+    for (size_t i = 0; i < lp.bwd.size(); ++i) {
+      const auto &st = lp.bwd[i];
+      if (lp.binv && i % lp.bwd_per_block == 0)
+        run_upper_inverses(L, lp.nblocks - 1 - (int)i / lp.bwd_per_block, lp.nblocks, s);
       run_leaf_step<T>(off, L, *st, st->g.items.p, st->g.segs.p, st->g.n, st->g.max_m, st->g.max_n,
                        info, s);
+    }
   }
 }
 
@@ -702,7 +728,7 @@ void run_path(Profiler &pf, const PathPlan<T, TE> &plan, int form, int *info, cu
               int parts = kPathLeaves | kPathLevels, const LevelHook *hook = nullptr) {
   if (!(parts & kPathLeaves)) {
   } else if (plan.factor) {
-    run_leaf_plan<T>(pf, plan.leaf, info, s);
+    run_leaf_plan<T>(pf, *plan.leaf, info, s);
   } else {
     PhaseScope ps(pf, PH_GETRS, s);
     launch_leaf_apply<T>(plan.apply_tasks.p, plan.nleaf, plan.apply_max_n, plan.apply_max_cols,
@@ -919,6 +945,7 @@ void merge_leaf_plans(const std::vector<const LeafPlan<T> *> &src, const std::ve
   dst.fwd_per_block = src[0]->fwd_per_block;
   dst.bwd_per_block = src[0]->bwd_per_block;
   dst.binv = src[0]->binv;
+  dst.slots = dst.nblocks;  // FP32: every system has a slot per block
   dst.tasks.upload(tasks);
   dst.host_tasks = tasks;
   dst.nleaf = (int)tasks.size();
@@ -966,9 +993,10 @@ void merge_paths(const std::vector<const PathPlan<T, TE> *> &src, const std::vec
   dst.apply_nb = dst.apply_max_n = dst.apply_max_cols = 0;
   if (dst.factor) {
     std::vector<const LeafPlan<T> *> lps;
-    for (const auto *p : src) lps.push_back(&p->leaf);
-    merge_leaf_plans<T>(lps, info_off, dst.leaf);
-    dst.nleaf = dst.leaf.nleaf;
+    for (const auto *p : src) lps.push_back(p->leaf.get());
+    dst.leaf = std::make_shared<LeafPlan<T>>();
+    merge_leaf_plans<T>(lps, info_off, *dst.leaf);
+    dst.nleaf = dst.leaf->nleaf;
   } else {
     std::vector<LeafFactorTask<T>> at;
     for (const auto *p : src) {
@@ -1071,26 +1099,26 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
   const int OB = std::max(NB, leaf_ob_auto64((long long)tasks.size() * max_n, max_n));
   const int P = OB / NB, nblocks = cdiv(max_n, OB), np = nblocks * P;
   const bool binv = P > 1;
+  const int slots = binv_slots<T>((long long)tasks.size(), nblocks, OB);
   // per leaf: panel inverses, block inverses, row order, interchange flags, marks
-  const size_t w_inv = (size_t)np * NB * NB, w_blk = binv ? (size_t)nblocks * OB * OB : 0;
+  const size_t w_inv = (size_t)np * NB * NB, w_blk = binv ? (size_t)slots * OB * OB : 0;
   // (in doubles; even, so that every leaf's inverses start on 16 bytes)
   const size_t ints = ((size_t)max_n + np + 2 * nblocks + 3) / 4 * 2;
-  const size_t per = 2 * w_inv + 2 * w_blk + ints;
+  const size_t per = 2 * w_inv + w_blk + ints;
   double *w = static_cast<double *>(scratch(sizeof(double) * per * tasks.size()));
   for (size_t q = 0; q < tasks.size(); ++q) {
     LeafFactorTask<T> &k = tasks[q];
     double *b = w + q * per;
     k.Linv = b;
     k.Uinv = b + w_inv;
-    k.LinvB = binv ? b + 2 * w_inv : nullptr;
-    k.UinvB = binv ? b + 2 * w_inv + w_blk : nullptr;
-    int *ip = reinterpret_cast<int *>(b + 2 * w_inv + 2 * w_blk);
+    k.Binv = binv ? b + 2 * w_inv : nullptr;
+    int *ip = reinterpret_cast<int *>(b + 2 * w_inv + w_blk);
     if (!k.perm) k.perm = ip;
     k.swapflag = ip + max_n;
     k.ill_b = k.swapflag + np;
   }
   std::vector<HostStep<T>> fwd, bwd;
-  leaf_steps<T>(tasks, NB, OB, nblocks, binv, fwd, bwd);
+  leaf_steps<T>(tasks, NB, OB, nblocks, binv, slots, fwd, bwd);
   // one block of descriptors: tasks | items | segments
   std::vector<Item> items;
   std::vector<Seg> segs;
@@ -1113,26 +1141,27 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
     HODLR_CUDA_TRY(cudaMemcpyAsync(dev, blob.data(), blob.size(), cudaMemcpyHostToDevice, s));
   Profiler off;
   const LeafSet<T> L{reinterpret_cast<const LeafFactorTask<T> *>(dev), (int)tasks.size(), max_n,
-                     cols, NB, OB};
+                     cols, NB, OB, slots};
   const Item *di = reinterpret_cast<const Item *>(dev + o_items);
   const Seg *ds = reinterpret_cast<const Seg *>(dev + o_segs);
-  auto run = [&](const std::vector<HostStep<T>> &steps) {
-    for (const HostStep<T> &h : steps) {
-      int mm = 0, mn = 0;
-      for (const Item &x : h.it) {
-        mm = std::max(mm, x.M);
-        mn = std::max(mn, x.N);
-      }
-      run_leaf_step<T>(off, L, h, di, ds, (int)h.it.size(), mm, mn, info, s);
-      di += h.it.size();
-      ds += h.sg.size();
+  auto run = [&](const HostStep<T> &h) {
+    int mm = 0, mn = 0;
+    for (const Item &x : h.it) {
+      mm = std::max(mm, x.M);
+      mn = std::max(mn, x.N);
     }
+    run_leaf_step<T>(off, L, h, di, ds, (int)h.it.size(), mm, mn, info, s);
+    di += h.it.size();
+    ds += h.sg.size();
   };
   launch_leaf_init<T>(L.tasks, L.nleaf, info, s);
-  run(fwd);
-  if (bwd.empty() || max_n == 0) return;
-  if (binv) launch_leaf_block_inverse<T>(L.tasks, L.nleaf, NB, OB, 0, true, nblocks, s);
-  run(bwd);
+  for (const HostStep<T> &h : fwd) run(h);
+  const size_t per_block = bwd.size() / std::max(nblocks, 1);
+  for (size_t i = 0; i < bwd.size(); ++i) {
+    if (binv && i % per_block == 0)
+      run_upper_inverses(L, nblocks - 1 - (int)(i / per_block), nblocks, s);
+    run(bwd[i]);
+  }
 }
 
 void Profiler::begin(int ph, cudaStream_t s, cudaEvent_t &a) {
@@ -1220,9 +1249,10 @@ void System::ensure_fp64() {
     f.factor = true; f.red_chunk = red_chunk; f.bc_chunk = bc_chunk;
     f.ob = ob64 > 0 ? ob64 : leaf_ob_auto64(N, nmax);
     f.leaf_size = leaf_size;
+    if (form == 1) f.leaf = fused64[0].leaf;
     build_path(tree, f, fused64[form], form);
     PathSpec<double, double> a = f;
-    a.X = Y64.p; a.factor = false; a.factors = &fused64[form].leaf;
+    a.X = Y64.p; a.factor = false; a.factors = fused64[form].leaf.get();
     build_path(tree, a, apply64[form], form);
   }
 }
@@ -1251,7 +1281,7 @@ void System::ensure_mixed() {
   f.ob = ob32;
   build_path(tree, f, fused32, 0);
   PathSpec<float, float> a = f;
-  a.X = Y32.p; a.factor = false; a.factors = &fused32.leaf;
+  a.X = Y32.p; a.factor = false; a.factors = fused32.leaf.get();
   a.red_chunk = kSweepChunk;
   a.max_slots = kSweepMaxSlots;
   build_path(tree, a, apply32, 0);
@@ -1361,7 +1391,7 @@ void Batch::build(const std::vector<System *> &systems) {
   for (size_t k = 0; k < sys.size(); ++k) {
     System *S = sys[k];
     S->ensure_mixed();
-    const int nbk = S->fused32.leaf.nb, obk = S->fused32.leaf.ob;
+    const int nbk = S->fused32.leaf->nb, obk = S->fused32.leaf->ob;
     const bool wide = S->m > 16;
     Group *g = nullptr;
     for (auto &q : groups)

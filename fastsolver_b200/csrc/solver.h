@@ -110,7 +110,7 @@ template <typename T>
 struct LeafPlan {
   DevBuf<LeafFactorTask<T>> tasks;
   DevBuf<T> Linv, Uinv;
-  DevBuf<T> LinvB, UinvB;  // outer-block inverses (two-level plans with ob <= 128)
+  DevBuf<T> Binv;  // outer-block inverses (two-level plans with ob <= 128)
   DevBuf<int> swapflag;
   DevBuf<int> ill_b;  // FP64: marks of ill-conditioned blocks (LeafFactorTask)
   std::vector<LeafFactorTask<T>> host_tasks;  // for apply plans with these factors
@@ -133,7 +133,7 @@ struct LeafPlan {
   // fwd: the steps of block 0, then block 1, ... (fwd_per_block each);
   // bwd: the steps of the last block first (bwd_per_block each)
   std::vector<std::unique_ptr<Step>> fwd, bwd;
-  int nblocks = 0, fwd_per_block = 0, bwd_per_block = 0;
+  int nblocks = 0, slots = 0, fwd_per_block = 0, bwd_per_block = 0;
   bool binv = false;  // block rows solved with the outer blocks' inverses
 };
 
@@ -142,7 +142,8 @@ struct PathPlan {
   bool built = false;
   bool factor = false;  // getrf + node factor (fused) vs getrs + node apply only
   int nleaf = 0;
-  LeafPlan<T> leaf;     // factor paths: the blocked leaf factorization
+  // factor paths: the blocked leaf factorization (the same one for both node forms)
+  std::shared_ptr<LeafPlan<T>> leaf;
   DevBuf<LeafFactorTask<T>> apply_tasks;  // apply paths: the factors' tasks on X
   int apply_nb = 0, apply_max_n = 0, apply_max_cols = 0;
   std::vector<std::unique_ptr<LevelPlan<T, TE>>> levels;  // deepest first

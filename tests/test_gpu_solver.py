@@ -379,3 +379,33 @@ def test_ill_conditioned_leaf_residual(fs, cuda, call, n, s):
         np.abs(L) @ (np.abs(U) @ np.abs(x)), axis=0)
     r = np.linalg.norm((B - A.astype(np.longdouble) @ x).astype(np.float64), axis=0)
     assert (r <= lim).all()
+
+
+def test_block_inverse_memory(fs, cuda):
+    """The outer blocks' inverses take one block of 128 columns per leaf where that
+    is over 32 MB (256 leaves), and both node forms use the same leaf buffers."""
+    import torch
+    r, leaf, used = 8, 512, []
+    # (the small systems first: code is loaded at a kernel's first launch)
+    for N, ob in ((2048, 16), (2048, 128), (131072, 16), (131072, 128)):
+        h = fs.HodlrMatrix(1, N, r, leaf).create_tree()
+        h.schedule = dict(leaf_ob64=ob)
+        D = torch.zeros((leaf, N), dtype=torch.float64, device="cuda").T
+        at = torch.arange(N, device="cuda")
+        D[at, at % leaf] = 2.0
+        h.set_matrix(D, *(torch.zeros((r * h.max_depth, N), dtype=torch.float64, device="cuda").T
+                          for _ in range(2)))
+        h.set_rhs(torch.ones((1, N), dtype=torch.float64, device="cuda").T)
+        del D
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        before = torch.cuda.mem_get_info()[0]
+        fs.FastSolver().bfs_solve(h)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        np.testing.assert_array_equal(h.solution(), 0.5)
+        cols = h.ncols
+        del h
+    slack = 16 << 20  # descriptors, node blocks, V^T products, the allocator's granularity
+    assert used[3] - used[2] <= 8 * N // leaf * 128 * 128 + slack
+    # X, the factors, Y and row orders and, once, the panels' inverses (2 x 32 columns)
+    assert used[2] <= 8 * N * (cols + leaf + 64 + 2) + slack
