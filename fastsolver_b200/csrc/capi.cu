@@ -188,7 +188,7 @@ int hodlr_leaf_solve(int n, int nrhs, double *D, int ldd, double *X, int ldx, in
     LeafFactorTask<double> tk{};
     tk.D = D; tk.ldd = ldd; tk.X = X; tk.ldx = ldx; tk.ipiv = ipiv;
     tk.n = n; tk.ncols = nrhs; tk.info_slot = 0;
-    run_leaf_bodies({tk}, info_dev, s, take);
+    run_leaf_bodies({tk}, leaf_body_shape(1, n), info_dev, s, take);
     return finish_info(info, info_dev, s);
   });
 }
@@ -210,13 +210,15 @@ int hodlr_leaf_solve_batched(int count, const hodlr_leaf_desc *descs, int max_n,
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
     for (const hodlr_leaf_desc &d : h)
       if (d.n > max_n || d.nrhs > max_nrhs || d.ldd < d.n || d.ldx < d.n) return -2;
-    // groups of leaves whose scratch (the inverses of their diagonal blocks)
-    // stays within 64 MB, and of at least enough leaves to fill the GPU
-    const size_t per = (size_t)std::max(max_n, 16) * 1024;
-    const int group = (int)std::max<size_t>(296, ((size_t)64 << 20) / per);
-    for (int i0 = 0; i0 < count; i0 += group) {
+    // One shape for the call, so that a leaf's result does not depend on its
+    // group; smaller groups where the device has no room for a full one.
+    int largest = 0;
+    for (const hodlr_leaf_desc &d : h) largest = std::max(largest, d.n);
+    const LeafBodyShape shape = leaf_body_shape(count, largest);
+    for (int i0 = 0, group = shape.group; i0 < count;) {
+      const int i1 = std::min(count, i0 + group);
       std::vector<LeafFactorTask<double>> t;
-      for (int i = i0; i < std::min(count, i0 + group); ++i) {
+      for (int i = i0; i < i1; ++i) {
         LeafFactorTask<double> k{};
         k.D = h[i].D; k.X = h[i].X; k.ipiv = h[i].ipiv; k.perm = h[i].perm;
         k.ldd = h[i].ldd; k.ldx = h[i].ldx; k.n = h[i].n; k.ncols = h[i].nrhs;
@@ -224,7 +226,15 @@ int hodlr_leaf_solve_batched(int count, const hodlr_leaf_desc *descs, int max_n,
         t.push_back(k);
       }
       ScratchList scr(s);
-      run_leaf_bodies(std::move(t), info, s, scr.taker());
+      try {
+        run_leaf_bodies(std::move(t), shape, info, s, scr.taker());
+      } catch (const CudaError &e) {
+        if (e.err != cudaErrorMemoryAllocation || group == 1) throw;
+        cudaGetLastError();
+        group = (group + 1) / 2;
+        continue;
+      }
+      i0 = i1;
     }
     HODLR_CUDA_TRY(cudaStreamSynchronize(s));
     return 0;

@@ -1084,28 +1084,52 @@ size_t padded_bytes(const std::vector<E> &v) {
 
 }  // namespace
 
-void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaStream_t s,
-                     const std::function<void *(size_t)> &scratch) {
+LeafBodyShape leaf_body_shape(long long leaves, int max_n) {
+  LeafBodyShape S;
+  S.max_n = max_n;
+  S.nb = leaf_nb<double>(max_n);
+  S.ob = std::max(S.nb, leaf_ob_auto64(leaves * max_n, max_n));
+  S.nblocks = cdiv(max_n, S.ob);
+  // the leaves of a group: as many as fit in the scratch with one slot of block
+  // inverses, and then as many slots as still fit
+  S.slots = 1;
+  const long long base = S.leaf_bytes(), cap = kLeafBodyScratch;
+  S.group = (int)std::max(1LL, std::min(leaves, cap / base));
+  if (S.ob > S.nb) {
+    const long long more = (cap / S.group - base) / ((long long)sizeof(double) * S.ob * S.ob);
+    S.slots = (int)std::min<long long>(S.nblocks, 1 + std::max(0LL, more));
+  }
+  return S;
+}
+
+size_t LeafBodyShape::leaf_words() const {
+  // panel inverses, block inverses, then as ints: row order, pivots, interchange
+  // flags, marks (doubles; even, so that every leaf's inverses start on 16 bytes)
+  const size_t np = (size_t)nblocks * (ob / nb);
+  const size_t ints = (2 * (size_t)max_n + np + 2 * nblocks + 3) / 4 * 2;
+  return 2 * np * nb * nb + (ob > nb ? (size_t)slots * ob * ob : 0) + ints;
+}
+
+size_t LeafBodyShape::leaf_bytes() const {
+  // the task and at most four GEMM items per panel and six per outer block
+  const size_t items = 4 * (size_t)nblocks * (ob / nb) + 6 * (size_t)nblocks;
+  return sizeof(double) * leaf_words() + sizeof(LeafFactorTask<double>) +
+         items * (sizeof(GemmItem<double, double>) + sizeof(GemmSeg<double>));
+}
+
+void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, const LeafBodyShape &S, int *info,
+                     cudaStream_t s, const std::function<void *(size_t)> &scratch) {
   using T = double;
   using Item = GemmItem<T, T>;
   using Seg = GemmSeg<T>;
   if (tasks.empty()) return;
-  int max_n = 0, cols = 0;
-  for (const auto &k : tasks) {
-    max_n = std::max(max_n, k.n);
-    cols = std::max(cols, k.n + k.ncols);
-  }
-  const int NB = leaf_nb<T>(max_n);
-  const int OB = std::max(NB, leaf_ob_auto64((long long)tasks.size() * max_n, max_n));
-  const int P = OB / NB, nblocks = cdiv(max_n, OB), np = nblocks * P;
-  const bool binv = P > 1;
-  const int slots = binv_slots<T>((long long)tasks.size(), nblocks, OB);
-  // per leaf: panel inverses, block inverses, row order, interchange flags, marks
-  const size_t w_inv = (size_t)np * NB * NB, w_blk = binv ? (size_t)slots * OB * OB : 0;
-  // (in doubles; even, so that every leaf's inverses start on 16 bytes)
-  const size_t ints = ((size_t)max_n + np + 2 * nblocks + 3) / 4 * 2;
-  const size_t per = 2 * w_inv + w_blk + ints;
-  double *w = static_cast<double *>(scratch(sizeof(double) * per * tasks.size()));
+  int cols = 0;
+  for (const auto &k : tasks) cols = std::max(cols, k.n + k.ncols);
+  const int NB = S.nb, OB = S.ob, nblocks = S.nblocks, slots = S.slots, max_n = S.max_n;
+  const bool binv = OB > NB;
+  const size_t np = (size_t)nblocks * (OB / NB), w_inv = np * NB * NB;
+  const size_t w_blk = binv ? (size_t)slots * OB * OB : 0, per = S.leaf_words();
+  double *w = static_cast<double *>(scratch(std::max<size_t>(sizeof(T) * per * tasks.size(), 16)));
   for (size_t q = 0; q < tasks.size(); ++q) {
     LeafFactorTask<T> &k = tasks[q];
     double *b = w + q * per;
@@ -1114,7 +1138,7 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaS
     k.Binv = binv ? b + 2 * w_inv : nullptr;
     int *ip = reinterpret_cast<int *>(b + 2 * w_inv + w_blk);
     if (!k.perm) k.perm = ip;
-    k.swapflag = ip + max_n;
+    k.swapflag = ip + 2 * max_n;
     k.ill_b = k.swapflag + np;
   }
   std::vector<HostStep<T>> fwd, bwd;

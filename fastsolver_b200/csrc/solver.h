@@ -391,12 +391,25 @@ struct Batch {
   }
 };
 
-// The leaf task body on `tasks` (D, X, ipiv, perm or null, ldd, ldx, n, ncols
-// and info_slot set; n <= 1024) by the blocked factorization of
-// leaf_blocked.cu: `scratch(b)` returns b bytes of device scratch, 256-byte
-// aligned, that live until the work enqueued on s is done.
-void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, int *info, cudaStream_t s,
-                     const std::function<void *(size_t)> &scratch);
+// The blocked factorization that the leaf task body runs for a call of `leaves`
+// leaves of at most max_n rows (leaf_body_shape; max_n <= 1024), in groups of at
+// most `group` leaves, whose scratch and descriptors stay within kLeafBodyScratch
+// (a leaf takes 0.29 MB at 512 rows on one level, 0.41 MB at 512 and at 1024 rows
+// with 128-column blocks, so that a full group fills the GPU).
+constexpr long long kLeafBodyScratch = 64LL << 20;
+struct LeafBodyShape {
+  int max_n = 0, nb = 0, ob = 0, nblocks = 0, slots = 0, group = 0;
+  size_t leaf_words() const;  // scratch of a leaf, in doubles
+  size_t leaf_bytes() const;  // ... and with its descriptors, in bytes
+};
+LeafBodyShape leaf_body_shape(long long leaves, int max_n);
+
+// The leaf task body on a group of `tasks` (D, X, ipiv, perm or null, ldd, ldx, n,
+// ncols and info_slot set) by the blocked factorization of leaf_blocked.cu:
+// `scratch(b)` returns b bytes of device scratch, 256-byte aligned, that live
+// until the work enqueued on s is done.  Asks for all scratch before it enqueues.
+void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, const LeafBodyShape &shape,
+                     int *info, cudaStream_t s, const std::function<void *(size_t)> &scratch);
 
 }  // namespace hodlr
 

@@ -125,9 +125,12 @@ typedef struct {
   int nrhs;
 } hodlr_leaf_desc;
 
-/* All leaves of a level (or of many systems) in one launch pair.  `descs` is
- * a device array of `count` descriptors, max_n the largest n among them;
- * info (device, `count` ints) receives each leaf's INFO.  Asynchronous.
+/* All leaves of a level (or of many systems) together.  `descs` is a device
+ * array of `count` descriptors, max_n the largest n among them; info (device,
+ * `count` ints) receives each leaf's INFO.  Reads the descriptors back first and
+ * returns when the work is done.  Runs in groups of leaves that take up to 64 MB
+ * of device scratch (less where that much is not free).  How a leaf is blocked,
+ * hence the rounding of its result, depends on count and the largest n.
  * Batched form of solver_tasks.cc:424-450 over the leaves that
  * fast_solver.cc:197-201 visits. */
 int hodlr_leaf_solve_batched(int count, const hodlr_leaf_desc *descs,

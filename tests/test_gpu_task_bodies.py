@@ -272,3 +272,64 @@ def test_fp32_skinny_elementwise(fs, cuda, m, n, k, odd):
             err = np.abs(Cg.cpu().numpy().T[:m].astype(np.float64) - (alpha * (op @ Bd) + beta * Cd))
             lim = (k + 4) * 2.0 ** -24 * (abs(alpha) * (np.abs(op) @ np.abs(Bd)) + abs(beta * Cd))
             assert (err <= lim).all()
+
+
+def _batch_descs(D, X, piv, n, c):
+    """Descriptors of the leaves D[i] (n x n), X[i] (n x c), contiguous and column-major."""
+    import ctypes
+    import torch
+
+    class Desc(ctypes.Structure):
+        _fields_ = [("D", ctypes.c_void_p), ("X", ctypes.c_void_p), ("ipiv", ctypes.c_void_p),
+                    ("perm", ctypes.c_void_p), ("ldd", ctypes.c_longlong),
+                    ("ldx", ctypes.c_longlong), ("n", ctypes.c_int), ("nrhs", ctypes.c_int)]
+
+    arr = (Desc * D.shape[0])(*[Desc(D[i].data_ptr(), X[i].data_ptr(),
+                                     piv[i].data_ptr() if piv is not None else None, None, n, n, n, c)
+                                for i in range(D.shape[0])])
+    return torch.frombuffer(bytearray(bytes(arr)), dtype=torch.uint8).cuda()
+
+
+@pytest.mark.parametrize("count,n", [(300, 250), (400, 512), (170, 1000)])
+def test_leaf_solve_batched_scratch(fs, cuda, count, n):
+    """The call's scratch stays within 64 MB, and equal leaves get equal results
+    whichever group they fall into."""
+    import threading
+    import torch
+    from fastsolver_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.randn(n, n, generator=gen, device="cuda", dtype=torch.float64)
+    B = torch.randn(3, n, generator=gen, device="cuda", dtype=torch.float64)
+    D, X = A.repeat(count, 1, 1), B.repeat(count, 1, 1)
+    piv = torch.zeros(count, n, dtype=torch.int32, device="cuda")
+    raw = _batch_descs(D, X, piv, n, 3)
+    info = torch.zeros(count, dtype=torch.int32, device="cuda")
+    small = torch.zeros(1, n, n, dtype=torch.float64, device="cuda")
+    small[0].fill_diagonal_(1.0)
+    one = _batch_descs(small, X[:1].clone(), piv, n, 3)
+    assert _lib.lib.hodlr_leaf_solve_batched(1, one.data_ptr(), n, 3, info.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    low, done = [torch.cuda.mem_get_info()[0]], threading.Event()
+    before = low[0]
+
+    def watch():
+        while not done.is_set():
+            low[0] = min(low[0], torch.cuda.mem_get_info()[0])
+
+    th = threading.Thread(target=watch)
+    th.start()
+    try:
+        for _ in range(5):
+            D.copy_(A.expand_as(D))
+            X.copy_(B.expand_as(X))
+            torch.cuda.synchronize()
+            assert _lib.lib.hodlr_leaf_solve_batched(count, raw.data_ptr(), n, 3, info.data_ptr(),
+                                                     None) == 0
+    finally:
+        done.set()
+        th.join()
+    assert (info == 0).all()
+    assert before - low[0] <= (64 << 20) + (34 << 20)  # the pool grows by 32 MB
+    assert (X == X[0]).all() and (D == D[0]).all() and (piv == piv[0]).all()
+    x = torch.linalg.solve(A.T, B.T)
+    assert float((X[0].T - x).norm() / x.norm()) <= 20 * n * float(torch.linalg.cond(A)) * 2.0 ** -53
