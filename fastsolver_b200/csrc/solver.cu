@@ -1138,6 +1138,7 @@ void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, const LeafBodySh
     k.Binv = binv ? b + 2 * w_inv : nullptr;
     int *ip = reinterpret_cast<int *>(b + 2 * w_inv + w_blk);
     if (!k.perm) k.perm = ip;
+    if (!k.ipiv) k.ipiv = ip + max_n;
     k.swapflag = ip + 2 * max_n;
     k.ill_b = k.swapflag + np;
   }

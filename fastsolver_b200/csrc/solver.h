@@ -404,8 +404,8 @@ struct LeafBodyShape {
 };
 LeafBodyShape leaf_body_shape(long long leaves, int max_n);
 
-// The leaf task body on a group of `tasks` (D, X, ipiv, perm or null, ldd, ldx, n,
-// ncols and info_slot set) by the blocked factorization of leaf_blocked.cu:
+// The leaf task body on a group of `tasks` (D, X, ldd, ldx, n, ncols and info_slot
+// set; ipiv and perm set or null) by the blocked factorization of leaf_blocked.cu:
 // `scratch(b)` returns b bytes of device scratch, 256-byte aligned, that live
 // until the work enqueued on s is done.  Asks for all scratch before it enqueues.
 void run_leaf_bodies(std::vector<LeafFactorTask<double>> tasks, const LeafBodyShape &shape,

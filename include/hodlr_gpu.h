@@ -117,8 +117,8 @@ int hodlr_gemm_broadcast(double alpha, double beta, int k, int r, int c,
 typedef struct {
   double *D;  /* n x n, ldd */
   double *X;  /* n x nrhs, ldx */
-  int *ipiv;  /* n ints */
-  int *perm;  /* n ints: final row order (row i of P^T D is row perm[i]) */
+  int *ipiv;  /* n ints, or null: the pivots are not returned */
+  int *perm;  /* n ints: final row order (row i of P^T D is row perm[i]), or null */
   long long ldd;
   long long ldx;
   int n;

@@ -333,3 +333,43 @@ def test_leaf_solve_batched_scratch(fs, cuda, count, n):
     assert (X == X[0]).all() and (D == D[0]).all() and (piv == piv[0]).all()
     x = torch.linalg.solve(A.T, B.T)
     assert float((X[0].T - x).norm() / x.norm()) <= 20 * n * float(torch.linalg.cond(A)) * 2.0 ** -53
+
+
+@pytest.mark.parametrize("n", [1, 33, 300, 700])
+def test_leaf_solve_batched_without_pivots(fs, cuda, n):
+    """Descriptors without ipiv (and perm) are solved like those with them."""
+    import torch
+    from fastsolver_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.randn(3, n, n, generator=gen, device="cuda", dtype=torch.float64)
+    B = torch.randn(3, 2, n, generator=gen, device="cuda", dtype=torch.float64)
+    out = []
+    for piv in (torch.zeros(3, n, dtype=torch.int32, device="cuda"), None):
+        D, X = A.clone(), B.clone()
+        info = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+        raw = _batch_descs(D, X, piv, n, 2)
+        assert _lib.lib.hodlr_leaf_solve_batched(3, raw.data_ptr(), n, 2, info.data_ptr(), None) == 0
+        assert (info == 0).all()
+        out.append((D, X))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    x = torch.linalg.solve(A.transpose(1, 2), B.transpose(1, 2)).transpose(1, 2)
+    cond = float(torch.linalg.cond(A).max())
+    assert float((out[1][1] - x).norm() / x.norm()) <= 20 * n * cond * 2.0 ** -53
+
+
+def test_leaf_solve_batched_empty_leaves(fs, cuda):
+    """A batch of leaves without rows, and one with some among others."""
+    import torch
+    from fastsolver_b200 import _lib
+    none = torch.zeros(3, 0, 0, dtype=torch.float64, device="cuda")
+    raw = _batch_descs(none, none, None, 0, 0)
+    for max_n in (0, 7):
+        info = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+        assert _lib.lib.hodlr_leaf_solve_batched(3, raw.data_ptr(), max_n, 0, info.data_ptr(),
+                                                 None) == 0
+        assert (info == 0).all()
+    D = 2 * torch.eye(7, dtype=torch.float64, device="cuda").repeat(2, 1, 1)
+    X = torch.ones(2, 1, 7, dtype=torch.float64, device="cuda")
+    raw = torch.cat([_batch_descs(none[:1], none[:1], None, 0, 0), _batch_descs(D, X, None, 7, 1)])
+    assert _lib.lib.hodlr_leaf_solve_batched(3, raw.data_ptr(), 7, 1, info.data_ptr(), None) == 0
+    assert (info == 0).all() and (X == 0.5).all()
