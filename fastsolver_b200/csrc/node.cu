@@ -129,10 +129,18 @@ __device__ inline int tied_lane(unsigned high, unsigned mx, unsigned low, int po
 //      registers (every row, also those already pivotal), with one barrier of
 //      the row warps per column: search by one warp reduction and one ballot
 //      unless keys tie, the winner publishes its 8 values and its reciprocal.
-//      What is left in the panel, X, are the multipliers: the inverse's part;
-//   2. the panel's pivot rows are copied as they were before it;
-//   3. every other column: A = (pivot rows: 0, others: A) + X (old pivot rows),
-//      one rank-8 DMMA product.
+//      What is left are every row's multipliers, X; those of a pivot row before
+//      its own column go to Lp;
+//   2. the panel's pivot rows, each as it is at its own column: as before the
+//      panel, in the panel's own columns (now the inverse's) the unit rows, less
+//      Lp times the ones before them;
+//   3. every column: A = (pivot rows and own columns: 0, others: A) + X (those
+//      rows), one rank-8 DMMA product.
+// So every element goes through the steps of the column-by-column elimination.
+// (With X the panel's part of the inverse and the pivot rows as they were before
+// the panel the products multiply with explicit inverses of 8 x 8 pivot blocks:
+// on smooth-kernel systems of order 16 to 144 the residual of the solution grew
+// up to 1e8-fold.)
 // What bounds it is the serial chain of a column (~700 cycles: search,
 // publish, barrier, combine), no longer the re-reading of the matrix: column
 // by column it took 1.9 k cycles with the matrix in registers (s <= 64) and
@@ -144,6 +152,7 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
   __shared__ __align__(16) double wrow[2][kNodeWarps][PB];
   __shared__ double wrcp[2][kNodeWarps];
   __shared__ int4 wmeta[2][kNodeWarps];
+  __shared__ double Lp[PB][PB];
   __shared__ int s_info;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -155,8 +164,8 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
   if (tid == 0) s_info = 0;
   for (int k0 = 0; k0 < s; k0 += PB) {
     const int nb = min(PB, s - k0);
-    double a[PB];
     if (warp < nrw) {
+      double a[PB];
       const double2 *ar = reinterpret_cast<const double2 *>(A + min(tid, s - 1) * lda + k0);
 #pragma unroll
       for (int c = 0; c < PB / 2; ++c) {
@@ -184,7 +193,7 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
           wrcp[slot][warp] = rc;
           double2 *d = reinterpret_cast<double2 *>(wrow[slot][warp]);
 #pragma unroll
-          for (int c = 0; c < PB / 2; ++c) d[c] = make_double2(a[2 * c], a[2 * c + 1]);
+          for (int c = jj / 2; c < PB / 2; ++c) d[c] = make_double2(a[2 * c], a[2 * c + 1]);
         }
         asm volatile("bar.sync 1, %0;\n" ::"r"(nrw * 32) : "memory");
         const unsigned wkey = lane < nrw ? (unsigned)wmeta[slot][lane].x : 0u;
@@ -200,7 +209,7 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
         double u[PB];
         const double2 *ur = reinterpret_cast<const double2 *>(wrow[slot][pw]);
 #pragma unroll
-        for (int c = 0; c < PB / 2; ++c) {
+        for (int c = jj / 2; c < PB / 2; ++c) {
           const double2 v = ur[c];
           u[2 * c] = v.x;
           u[2 * c + 1] = v.y;
@@ -213,36 +222,58 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
           act = false;
           mark[tid] = k0;
           prow[jj] = tid;
+          a[jj] = rinv;
 #pragma unroll
-          for (int c = 0; c < PB; ++c) a[c] = c == jj ? rinv : a[c] * rinv;
+          for (int c = jj + 1; c < PB; ++c) a[c] *= rinv;
         } else {
           if (pos == k) pos = m.z;
-          const double f = a[jj] * rinv;
+          a[jj] = -(a[jj] * rinv);
 #pragma unroll
-          for (int c = 0; c < PB; ++c) a[c] = c == jj ? -f : a[c] - f * u[c];
+          for (int c = jj + 1; c < PB; ++c) a[c] += a[jj] * u[c];
         }
       }
       if (rowok) {
+        const int own = act ? 0 : max(pos - k0, 0);  // the column here whose pivot this row is
+        if (own > 0) {
+#pragma unroll
+          for (int c = 0; c < PB; ++c) Lp[own][c] = a[c];
+        }
         double2 *xr = reinterpret_cast<double2 *>(X + tid * kXld);
+#pragma unroll
+        for (int c = 0; c < PB; ++c)
+          if (c < own || c >= nb) a[c] = 0.0;
 #pragma unroll
         for (int c = 0; c < PB / 2; ++c) xr[c] = make_double2(a[2 * c], a[2 * c + 1]);
       }
     }
     __syncthreads();
     if (s_info != 0) return s_info;  // uniform
-    for (int e = tid; e < PB * tn * 8; e += kNodeThreads) {
-      const int jj = e & (PB - 1), c = e / PB;
-      Bb[jj * ldb + c] = jj < nb ? A[prow[jj] * lda + c] : 0.0;
+    if (const int c = tid; c < tn * 8) {
+      static_assert(kMaxNodeS <= kNodeThreads, "a thread per column");
+      double u[PB];
+#pragma unroll
+      for (int jj = 0; jj < PB; ++jj) u[jj] = jj < nb ? A[prow[jj] * lda + c] : 0.0;
+      if (c >= k0 && c < k0 + PB) {
+#pragma unroll
+        for (int jj = 0; jj < PB; ++jj) u[jj] = c == k0 + jj ? 1.0 : 0.0;
+      }
+#pragma unroll
+      for (int jj = 0; jj < PB; ++jj) {
+        Bb[jj * ldb + c] = u[jj];
+#pragma unroll
+        for (int k = jj + 1; k < PB; ++k)
+          if (k < nb) u[k] += Lp[k][jj] * u[jj];
+      }
     }
     __syncthreads();
     for (int tile = warp; tile < tm * tn; tile += kNodeWarps) {
       const int mt = tile % tm, nt = tile / tm;
-      if (nt == k0 / PB) continue;
+      const bool own = nt == k0 / PB;
       const int ra = mt * 16 + g, rb = ra + 8;
       double2 *p0 = reinterpret_cast<double2 *>(A + ra * lda + nt * 8 + 2 * t);
       double2 *p1 = reinterpret_cast<double2 *>(A + rb * lda + nt * 8 + 2 * t);
       const double2 v0 = *p0, v1 = *p1;
-      const bool z0 = mark[ra] == k0, z1 = mark[rb] == k0;  // this panel's pivot rows
+      const bool z0 = own || mark[ra] == k0, z1 = own || mark[rb] == k0;  // pivot rows here
       double c[4] = {z0 ? 0.0 : v0.x, z0 ? 0.0 : v0.y, z1 ? 0.0 : v1.x, z1 ? 0.0 : v1.y};
       const double *x0 = X + ra * kXld + t, *x1 = X + rb * kXld + t;
       const double *bp = Bb + t * ldb + nt * 8 + g;
@@ -250,11 +281,6 @@ __device__ inline int gauss_jordan(double *A, int lda, int s, double *X, double 
       dmma(c, x0[4], x1[4], bp[4 * ldb]);
       *p0 = make_double2(c[0], c[1]);
       *p1 = make_double2(c[2], c[3]);
-    }
-    if (rowok) {
-      double2 *ar = reinterpret_cast<double2 *>(A + tid * lda + k0);
-#pragma unroll
-      for (int c = 0; c < PB / 2; ++c) ar[c] = make_double2(a[2 * c], a[2 * c + 1]);
     }
     __syncthreads();
   }

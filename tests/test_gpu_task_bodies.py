@@ -373,3 +373,34 @@ def test_leaf_solve_batched_empty_leaves(fs, cuda):
     raw = torch.cat([_batch_descs(none[:1], none[:1], None, 0, 0), _batch_descs(D, X, None, 7, 1)])
     assert _lib.lib.hodlr_leaf_solve_batched(3, raw.data_ptr(), 7, 1, info.data_ptr(), None) == 0
     assert (info == 0).all() and (X == 0.5).all()
+
+
+@pytest.mark.parametrize("s,width", [(9, 1.0), (16, 1.0), (17, 0.5), (37, 1.0), (64, 1.0), (100, 1.0),
+                                     (144, 1.0)])
+def test_node_elimination_ill_conditioned(fs, cuda, s, width):
+    """An ill-conditioned S = I - V1Tu1 V0Tu0 (V1Tu1 = I): the residual of the
+    column-by-column Gauss-Jordan elimination with partial pivoting."""
+    x = np.linspace(0, 1, s)
+    K = np.exp(-((x[:, None] - x) / width) ** 2) + 1e-12 * np.eye(s)
+    V0Tu0 = np.eye(s) - K
+    S = np.eye(s) - V0Tu0                      # as the kernel forms it
+    d1 = np.random.default_rng(s).standard_normal((s, 3))
+    g = [dev(V0Tu0), dev(np.eye(s)), dev(np.zeros((s, 3))), dev(d1)]
+    assert fs.node_lu_solve(*g) == 0
+    eta0 = host(g[3])
+    A, p = S.copy(), np.arange(s)
+    for k in range(s):
+        j = k + int(np.argmax(np.abs(A[k:, k])))
+        A[[k, j]], p[[k, j]] = A[[j, k]], p[[j, k]]
+        A[k + 1:, k] /= A[k, k]
+        A[k + 1:, k + 1:] -= np.outer(A[k + 1:, k], A[k, k + 1:])
+    L, U = np.abs(np.tril(A, -1) + np.eye(s)), np.triu(A)
+    Ui = np.linalg.inv(U)
+    X = np.abs(Ui @ np.linalg.inv(np.tril(A, -1) + np.eye(s)))   # |S^{-1}| of the permuted rows
+    aU = np.abs(U)
+    # columns x_j of the inverse: |e_j - S x_j| <= 8 s u |L| |U| |U^{-1}| |U| |x_j|, and
+    # s u |S| |X| |d| for the product with the right-hand sides
+    w = X @ np.abs(d1[p])
+    lim = s * 2.0 ** -53 * (8 * (L @ (aU @ (np.abs(Ui) @ (aU @ w)))) + np.abs(S[p]) @ w)
+    r = np.abs((S.astype(np.longdouble) @ eta0 - d1).astype(np.float64))[p]
+    assert (r <= lim).all(), (r / lim).max()
