@@ -409,3 +409,15 @@ def test_block_inverse_memory(fs, cuda):
     assert used[3] - used[2] <= 8 * N // leaf * 128 * 128 + slack
     # X, the factors, Y and row orders and, once, the panels' inverses (2 x 32 columns)
     assert used[2] <= 8 * N * (cols + leaf + 64 + 2) + slack
+
+
+@pytest.mark.parametrize("r", [104, 105, 144])
+def test_mixed_large_ranks(fs, oracle, cuda, r):
+    """The mixed node factorization on both sides of the rank up to which the V^T u
+    blocks are staged in shared memory, and at the largest rank."""
+    s = make_gauss(oracle, 1500, 3, r, 400, seed=r)
+    h = gpu_system(fs, s)
+    it, rr = fs.FastSolver().solve_refined(h, fs.PREC_MIXED, tol=1e-12, maxiter=10)
+    assert rr <= 1e-12
+    X, _ = oracle.bfs_solve(s, nthreads=8)
+    assert relerr(h.solution(), X[:, :3]) < 1e-11
