@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "gemm_dmma.cuh"
+#include "warp_f64.cuh"
 
 namespace hodlr {
 
@@ -61,17 +62,6 @@ __device__ inline void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::
 template <int N>
 __device__ inline void cpa_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// Fragments of m16n8k4 .f64 (g = lane / 4, t = lane % 4): A a0 = A[g][t],
-// a1 = A[g + 8][t]; B b = B[t][g]; C c0..c3 = C[g][2t], C[g][2t + 1],
-// C[g + 8][2t], C[g + 8][2t + 1].
-__device__ inline void dmma(double (&c)[4], double a0, double a1, double b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-      "{%0, %1, %2, %3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(b));
 }
 
 template <int BM, bool TRANS>

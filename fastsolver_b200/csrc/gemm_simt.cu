@@ -30,36 +30,31 @@ constexpr int NT = 256;
 // Tiled items (N > 32): BM x 128 tile per CTA (BM = 64 or 128), 256 threads,
 // TM x 8 register tile per thread (thread x -> rows, y -> columns, so the
 // epilogue's column-major accesses coalesce), K staged in BK-deep slices through a
-// two-stage cp.async pipeline.  Register fragments are interleaved in
-// 16-byte vectors (2 doubles / 4 floats) so that the shared-memory reads of
-// the 16 row groups of a warp are contiguous (no bank conflicts) and the
-// column fragments are warp-broadcasts.
+// two-stage cp.async pipeline.  Register fragments are interleaved in 16-byte
+// vectors so that the shared-memory reads of the 16 row groups of a warp are
+// contiguous (no bank conflicts) and the column fragments are warp-broadcasts.
 // ---------------------------------------------------------------------------
 
-__device__ inline void cp_async_elem(void *smem, const void *gmem, int bytes, bool pred) {
+__device__ inline void cp_async_elem(float *smem, const float *gmem, bool pred) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  const int n = pred ? bytes : 0;
-  if (bytes == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(pred ? 4 : 0));
 }
 __device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ inline void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
 
-template <typename T, typename TC, bool TRANS, int BM>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
-    gemm_tile_kernel(const GemmItem<T, TC> *__restrict__ items,
-                     const GemmSeg<T> *__restrict__ segs, T alpha, T beta) {
-  constexpr int BN = 128;
-  constexpr int BK = sizeof(T) == 8 ? 8 : 16;
-  constexpr int VW = 16 / sizeof(T);       // elements per 16-byte vector
+template <bool TRANS, int BM>
+__global__ void __launch_bounds__(NT, 2)
+    gemm_tile_kernel(const GemmItem<float, float> *__restrict__ items,
+                     const GemmSeg<float> *__restrict__ segs, float alpha, float beta) {
+  using T = float;
+  constexpr int BN = 128, BK = 16;
+  constexpr int VW = 4;                    // elements per 16-byte vector
   constexpr int TM = BM / 16, TN = BN / 16;
   constexpr int AP = BM + 4, BP = BN + 4;  // padded row strides (16-byte multiples)
   constexpr int NA = BK * BM / NT, NBL = BK * BN / NT;
   __shared__ __align__(16) T As[2][BK * AP];
   __shared__ __align__(16) T Bs[2][BK * BP];
-  const GemmItem<T, TC> it = items[blockIdx.x];
+  const GemmItem<T, T> it = items[blockIdx.x];
   const int m0 = blockIdx.y * BM, n0 = blockIdx.z * BN;
   if (m0 >= it.M || n0 >= it.N) return;
   const int tid = threadIdx.x;
@@ -77,7 +72,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
       if (preload) {
         const int gm = m0 + (i / VW) * (16 * VW) + tx * VW + (i % VW);
         const int gn = n0 + (j / VW) * (16 * VW) + ty * VW + (j % VW);
-        if (gm < it.M && gn < it.N) v = alpha * T(it.Cin[gm + (long long)gn * it.ldcin]);
+        if (gm < it.M && gn < it.N) v = alpha * it.Cin[gm + (long long)gn * it.ldcin];
       }
       acc[i][j] = v;
     }
@@ -100,7 +95,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
         const T *src = ok ? (TRANS ? sg.A + gk + (long long)gm * sg.lda
                                    : sg.A + gm + (long long)gk * sg.lda)
                           : sg.A;
-        cp_async_elem(&As[buf][k * AP + m], src, sizeof(T), ok);
+        cp_async_elem(&As[buf][k * AP + m], src, ok);
       }
 #pragma unroll
       for (int u = 0; u < NBL; ++u) {
@@ -109,7 +104,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
         const int gk = k0 + k, gn = n0 + n;
         const bool ok = gk < K && gn < it.N;
         const T *src = ok ? sg.B + gk + (long long)gn * sg.ldb : sg.B;
-        cp_async_elem(&Bs[buf][k * BP + n], src, sizeof(T), ok);
+        cp_async_elem(&Bs[buf][k * BP + n], src, ok);
       }
     };
     issue(0, 0);
@@ -121,20 +116,19 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
       __syncthreads();
       const T *Ab = As[kt & 1];
       const T *Bb = Bs[kt & 1];
-      using V = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
 #pragma unroll
       for (int kk = 0; kk < BK; ++kk) {
         T a[TM], b[TN];
 #pragma unroll
         for (int g = 0; g < TM / VW; ++g) {
-          const V va = *reinterpret_cast<const V *>(Ab + kk * AP + g * (16 * VW) + tx * VW);
+          const float4 va = *reinterpret_cast<const float4 *>(Ab + kk * AP + g * (16 * VW) + tx * VW);
           const T *pv = reinterpret_cast<const T *>(&va);
 #pragma unroll
           for (int v = 0; v < VW; ++v) a[g * VW + v] = pv[v];
         }
 #pragma unroll
         for (int g = 0; g < TN / VW; ++g) {
-          const V vb = *reinterpret_cast<const V *>(Bb + kk * BP + g * (16 * VW) + ty * VW);
+          const float4 vb = *reinterpret_cast<const float4 *>(Bb + kk * BP + g * (16 * VW) + ty * VW);
           const T *pv = reinterpret_cast<const T *>(&vb);
 #pragma unroll
           for (int v = 0; v < VW; ++v) b[g * VW + v] = pv[v];
@@ -156,8 +150,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 2 : 1)
       const int gm = m0 + (i / VW) * (16 * VW) + tx * VW + (i % VW);
       if (gm >= it.M) continue;
       T v = alpha * acc[i][j];
-      if (it.Cin && !preload) v += beta * T(it.Cin[gm + (long long)gn * it.ldcin]);
-      it.C[gm + (long long)gn * it.ldc] = TC(v);
+      if (it.Cin && !preload) v += beta * it.Cin[gm + (long long)gn * it.ldcin];
+      it.C[gm + (long long)gn * it.ldc] = v;
     }
   }
 }
@@ -189,12 +183,12 @@ void launch_gemm_items(const GemmItem<TA, TC> *items, const GemmSeg<TA> *segs, i
   } else {
     if (max_m <= 64) {
       dim3 grid(nitems, cdiv(max_m, 64), cdiv(max_n, 128));
-      if (trans) gemm_tile_kernel<T, TC, true, 64><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
-      else gemm_tile_kernel<T, TC, false, 64><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
+      if (trans) gemm_tile_kernel<true, 64><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
+      else gemm_tile_kernel<false, 64><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
     } else {
       dim3 grid(nitems, cdiv(max_m, 128), cdiv(max_n, 128));
-      if (trans) gemm_tile_kernel<T, TC, true, 128><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
-      else gemm_tile_kernel<T, TC, false, 128><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
+      if (trans) gemm_tile_kernel<true, 128><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
+      else gemm_tile_kernel<false, 128><<<grid, NT, 0, s>>>(items, segs, alpha, beta);
     }
     HODLR_LAUNCH_CHECK();
   }

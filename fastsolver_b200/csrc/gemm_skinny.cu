@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "gemm_skinny.cuh"
 #include "skinny_units.cuh"
+#include "warp_f64.cuh"
 
 namespace hodlr {
 
@@ -53,19 +54,11 @@ __global__ void __launch_bounds__(kTNThreads, 3)
 }
 
 // ---------------------------------------------------------------- FP64 on the DMMA pipe
-// FP64 items of at most 16 columns (the HODLR matvec's D x + U t and V^T x)
-// run on the FP64 tensor-core instruction mma.m16n8k4.f64: one instruction
-// per 16 x 8 x 4 block instead of 512 FMAs, so the kernels stay bound by the
-// operand stream instead of by instruction issue.  Fragments (PTX layout of
-// m16n8k4 .f64, g = lane / 4, t = lane % 4): A a0 = A[g][t], a1 = A[g + 8][t];
-// B b = B[t][g]; C c0..c3 = C[g][2t], C[g][2t + 1], C[g + 8][2t], C[g + 8][2t + 1].
-__device__ inline void dmma(double (&c)[4], double a0, double a1, double b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-      "{%0, %1, %2, %3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
+// FP64 items (at most 32 columns: the HODLR matvec's D x + U t and V^T x, the node
+// products, the leaves' block rows of few right-hand sides) run on the FP64
+// tensor-core instruction mma.m16n8k4.f64 (warp_f64.cuh): one instruction per
+// 16 x 8 x 4 block instead of 512 FMAs, so the kernels stay bound by the operand
+// stream instead of by instruction issue.
 
 // NN: C (M x N) = beta Cin + alpha sum_s A_s B_s, A_s column-major; one CTA
 // per (item, ROWS-row block) and all of an item's columns (8 NT8; with two

@@ -30,23 +30,13 @@
 
 #include "common.cuh"
 #include "leaf_blocked.cuh"
+#include "warp_f64.cuh"
 
 namespace hodlr {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-// Fragments of m16n8k4 .f64 (g = lane / 4, t = lane % 4): A a0 = A[g][t],
-// a1 = A[g + 8][t]; B b = B[t][g]; C c0..c3 = C[g][2t], C[g][2t + 1],
-// C[g + 8][2t], C[g + 8][2t + 1].
-__device__ inline void dmma64(double (&c)[4], double a0, double a1, double b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-      "{%0, %1, %2, %3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
 
 // 16-byte vector of T
 template <typename T>
@@ -104,16 +94,6 @@ __device__ inline unsigned key_high(unsigned k) { return k; }
 __device__ inline unsigned key_high(unsigned long long k) { return (unsigned)(k >> 32); }
 __device__ inline unsigned key_low(unsigned) { return 0u; }
 __device__ inline unsigned key_low(unsigned long long k) { return (unsigned)k; }
-
-// Of the lanes whose `high` is the warp's largest (mx; `win` their ballot,
-// more than one): the one with the largest low word, lowest position on ties.
-__device__ inline int tied_lane(unsigned high, unsigned mx, unsigned low, int pos) {
-  bool top = high == mx;
-  const unsigned ml = __reduce_max_sync(0xffffffffu, top ? low : 0u);
-  top = top && low == ml;
-  const unsigned pm = __reduce_min_sync(0xffffffffu, top ? (unsigned)pos : 0xffffffffu);
-  return __ffs(__ballot_sync(0xffffffffu, top && (unsigned)pos == pm)) - 1;
-}
 
 template <typename T, int NB, int RPT>
 __global__ void __launch_bounds__(kRegThreads, 1)
@@ -793,7 +773,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
       for (int k = 0; k < NBM / 4; ++k) {
         if (4 * k >= nb) break;
-        dmma64(c, d[k][0], d[k][1], ys[(4 * k + t) * XS + 8 * dn + g]);
+        dmma(c, d[k][0], d[k][1], ys[(4 * k + t) * XS + 8 * dn + g]);
       }
 #pragma unroll
       for (int v = 0; v < 4; ++v)  // kept negated: the updates subtract
@@ -823,7 +803,7 @@ __global__ void __launch_bounds__(512, 1)
           for (int k = 0; k < 4; ++k)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
-              dmma64(acc[j][nt], c[k][0], c[k][1], y[4 * k * XS + 8 * nt]);
+              dmma(acc[j][nt], c[k][0], c[k][1], y[4 * k * XS + 8 * nt]);
         }
       }
     }
@@ -955,7 +935,7 @@ __device__ inline void block_product(int M, int N, int K, const double *A, int l
 #pragma unroll 4
     for (int k = k0 + t; k < k1; k += 4) {
       const double a0 = A[m + k * lda], a1 = A[m + 8 + k * lda], b = B[k + (n + g) * ldb];
-      dmma64(c, a0, a1, b);
+      dmma(c, a0, a1, b);
     }
 #pragma unroll
     for (int v = 0; v < 4; ++v)
@@ -1204,7 +1184,7 @@ __global__ void __launch_bounds__(kSolveThreads)
   for (int k = 0; k < NB / 4; ++k)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
-      dmma64(c[nt], a[k][0], a[k][1], xs[(wn + 8 * nt + g) * LD + 4 * k + t]);
+      dmma(c[nt], a[k][0], a[k][1], xs[(wn + 8 * nt + g) * LD + 4 * k + t]);
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll

@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "node.cuh"
+#include "warp_f64.cuh"
 
 namespace hodlr {
 
@@ -69,20 +70,10 @@ __host__ __device__ inline NodeSmem node_smem(int max_s, int max_r, bool stage) 
   return m;
 }
 
-__device__ inline void dmma(double (&c)[4], double a0, double a1, double b) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-      "{%0, %1, %2, %3};\n"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(b));
-}
-
 // out(i, j, sum_k a(i, k) b(k, j)) for i < rows, j < cols on the FP64 tensor
 // pipe, every warp taking 16 x 8 tiles in turn.  a and b are read up to the
 // next multiples of 16 rows, 8 columns and 4 k; a(i, k) b(k, j) must be 0 for
-// k >= K.  Fragments (g = lane / 4, t = lane % 4): A a0 = A[g][t], a1 =
-// A[g + 8][t]; B b = B[t][g]; C c0..c3 = C[g][2t], C[g][2t + 1], C[g + 8][2t],
-// C[g + 8][2t + 1].
+// k >= K.
 template <typename FA, typename FB, typename FO>
 __device__ inline void node_product(int rows, int cols, int K, FA a, FB b, FO out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -110,16 +101,6 @@ __device__ inline void node_product(int rows, int cols, int K, FA a, FB b, FO ou
       if (i < rows && j < cols) out(i, j, c[v]);
     }
   }
-}
-
-// Of the lanes whose high key word is the warp's largest (more than one): the
-// one with the largest low word, lowest position on ties.
-__device__ inline int tied_lane(unsigned high, unsigned mx, unsigned low, int pos) {
-  bool top = high == mx;
-  const unsigned ml = __reduce_max_sync(0xffffffffu, top ? low : 0u);
-  top = top && low == ml;
-  const unsigned pm = __reduce_min_sync(0xffffffffu, top ? (unsigned)pos : 0xffffffffu);
-  return __ffs(__ballot_sync(0xffffffffu, top && (unsigned)pos == pm)) - 1;
 }
 
 // Inverse of the s x s matrix A (row-major, row stride lda, zero up to the
@@ -398,8 +379,11 @@ void launch_node_factor(const NodeTask<TW, TE> *tasks, int count, int max_s, int
                                         cudaSharedmemCarveoutMaxShared));
     kern<<<count, kNodeThreads, smem, s>>>(tasks, form, max_s, max_r, info);
   };
-  // V0Tu0 and V1Tu1 in shared memory where they fit beside the matrix (FP32
-  // up to r = 104, FP64 up to r = 72); beyond, the products read them from L2
+  // V0Tu0 and V1Tu1 in shared memory where they fit beside the matrix (FP32 up to
+  // r = 104, FP64 up to r = 88), also where that leaves one CTA per SM (FP64 above
+  // r = 56); beyond, the products read them from L2.  All levels of 131072 rows,
+  // leaves of 512, staged / not: FP64 r = 30 225 / 232 us, 56 434 / 449, 64 509 / 560,
+  // 88 924 / 1021; mixed r = 64 504 / 572, 80 749 / 899, 104 1212 / 1458.
   const size_t staged = node_smem<TW>(max_s, max_r, true).total;
   if (form == 0 && staged <= kSmemLimit) go(node_factor_kernel<TW, TE, true>, staged);
   else go(node_factor_kernel<TW, TE, false>, node_smem<TW>(max_s, max_r, false).total);

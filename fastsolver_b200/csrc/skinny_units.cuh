@@ -72,12 +72,6 @@ __device__ inline T ldg_unit(const T *p) {
   else return __ldg(p);
 }
 
-template <typename T>
-struct Vec {
-  using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  static constexpr int W = 16 / sizeof(T);
-};
-
 // ---------------------------------------------------------------- NN (rows)
 constexpr int kRowThreads = 128;
 constexpr int kNnSlab = 128;  // k-values of B in shared memory

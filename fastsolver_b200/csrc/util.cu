@@ -194,9 +194,7 @@ __global__ void colratio_batched_kernel(const RatioTask *__restrict__ tasks) {
   }
 }
 
-// dst[t][e] = sum_q src[t] + q * stride, fixed order (deterministic)
-// (the slot values are loaded four at a time ahead of the adds, which keep
-// the order q = 0, 1, 2, ...: the same sums)
+// dst <- the launch's own parameter bytes: descriptors without a host copy to wait for
 constexpr int kParamWords = 496;  // 8-byte words per launch, below the 4 KB parameter space
 struct ParamBlock {
   unsigned long long w[kParamWords];
@@ -206,6 +204,7 @@ __global__ void param_copy_kernel(unsigned long long *dst, int words,
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = b.w[i];
 }
 
+// (eta0 | eta1) of a node into its two outputs, unless the node was singular
 __global__ void node_output_kernel(const double *eta, int r0, int r1, int c, double *o0,
                                    long long l0, double *o1, long long l1, const int *info) {
   if (*info != 0) return;
@@ -219,6 +218,9 @@ __global__ void node_output_kernel(const double *eta, int r0, int r1, int c, dou
   }
 }
 
+// dst[t][e] = sum_q src[t] + q * stride, fixed order (deterministic)
+// (the slot values are loaded four at a time ahead of the adds, which keep
+// the order q = 0, 1, 2, ...: the same sums)
 template <typename T>
 __global__ void sum_slots_kernel(const SumTask<T> *__restrict__ tasks) {
   const SumTask<T> tk = tasks[blockIdx.y];
