@@ -668,6 +668,7 @@ void run_leaf_step(Profiler &pf, const LeafSet<T> &L, const S &st, const GemmIte
     case Plan::kPanelSolve:
     case Plan::kBlockSolve: {
       if constexpr (std::is_same<T, double>::value) {
+        if (st.cols == 0) break;
         PhaseScope pt(pf, PH_LEAF_TRSM, s);
         if (st.kind == Plan::kPanelSolve)
           launch_leaf_panel_solve(L.tasks, L.nleaf, st.cols, L.nb, st.panel, st.b0, st.b1,

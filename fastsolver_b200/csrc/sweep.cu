@@ -85,9 +85,10 @@ __device__ bool grid_sync(unsigned *bar, unsigned &gen, long long limit) {
   return s_ok != 0;
 }
 
-// Three CTAs (12 warps) per SM at 168 registers: at 32 columns the units'
-// accumulators make the kernel spill a little, yet two CTAs without spills ran
-// the sweeps of N = 1048576 in 20.7 instead of 18.2 ms.
+// Three CTAs (12 warps) per SM at 168 registers: the units' accumulators make the
+// kernel spill, 0.16 KB per thread at 16 columns and 1.3 KB at 32 (nothing at 8),
+// yet at 32 two CTAs without spills ran the sweeps of N = 1048576 in 20.7 instead
+// of 18.2 ms.
 template <int NC>
 __global__ void __launch_bounds__(kThreads, 3)
     sweep_levels_kernel(const SweepLevel *__restrict__ levels, int nlevels, unsigned *bar) {
