@@ -394,8 +394,8 @@ struct Batch {
 // The blocked factorization that the leaf task body runs for a call of `leaves`
 // leaves of at most max_n rows (leaf_body_shape; max_n <= 1024), in groups of at
 // most `group` leaves, whose scratch and descriptors stay within kLeafBodyScratch
-// (a leaf takes 0.29 MB at 512 rows on one level, 0.41 MB at 512 and at 1024 rows
-// with 128-column blocks, so that a full group fills the GPU).
+// (a leaf takes 0.28 MB at 512 rows on one level, 0.41 MB there and 0.43 MB at 1024
+// rows with 128-column blocks, so that a full group fills the GPU).
 constexpr long long kLeafBodyScratch = 64LL << 20;
 struct LeafBodyShape {
   int max_n = 0, nb = 0, ob = 0, nblocks = 0, slots = 0, group = 0;

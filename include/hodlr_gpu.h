@@ -382,7 +382,9 @@ int hodlr_batch_phase_times(hodlr_batch batch, double *ms, long long *launches, 
  *   leaf_ob64    the same for the FP64 path (panel width 32, or 16 above 512
  *                rows), 0 = by the leaves (128 for leaves above 512 rows and
  *                for large systems, else one level; up to the panel width,
- *                e.g. 16, is one level always);
+ *                e.g. 16, is one level always).  Blocks above the panel width
+ *                and up to 128 columns take device memory for their inverses:
+ *                32 MB, or one block per leaf where that is more;
  *   reduce_rows  rows per split-K slot of the reduce V^T [d | u] (16..65536,
  *                a multiple of 16; at most 64 slots per child);
  *   bcast_rows   rows per item of the broadcast d -= u eta (16..65536, a
