@@ -834,14 +834,16 @@ __device__ inline bool ill_conditioned(unsigned tri, unsigned inv) {
   const unsigned et = tri >> 20, ei = inv >> 20;
   return et == 2047 || ei == 2047 || et + ei >= 2 * 1023 + 6;
 }
-// The same over a CTA: every thread's high words go in, a barrier, and every
-// thread has the answer.  slots: one per warp.
-template <int WARPS>
-__device__ inline bool ill_conditioned_cta(uint2 *slots, unsigned tri, unsigned inv) {
+// The same over a CTA: every thread's high words go in, the caller's barrier, and
+// every thread has the answer.  slots: one per warp.
+__device__ inline void publish_largest(uint2 *slots, unsigned tri, unsigned inv) {
   tri = __reduce_max_sync(0xffffffffu, tri);
   inv = __reduce_max_sync(0xffffffffu, inv);
   if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = make_uint2(tri, inv);
-  __syncthreads();
+}
+template <int WARPS>
+__device__ inline bool ill_conditioned_cta(const uint2 *slots) {
+  unsigned tri = 0, inv = 0;
 #pragma unroll
   for (int w = 0; w < WARPS; ++w) {
     tri = max(tri, slots[w].x);
@@ -1050,8 +1052,9 @@ __global__ void __launch_bounds__(kInvThreads)
     }
   if constexpr (sizeof(T) == 8) {
     __shared__ uint2 slots[kInvThreads / 32];
-    const bool ill = ill_conditioned_cta<kInvThreads / 32>(
-        slots, upper ? largest_t : 1023u << 20, largest);  // max|L| = 1
+    publish_largest(slots, upper ? largest_t : 1023u << 20, largest);  // max|L| = 1
+    __syncthreads();
+    const bool ill = ill_conditioned_cta<kInvThreads / 32>(slots);
     if (tid == 0) tk.ill_b[2 * J + upper] = ill;
     if (ill)  // leaf_block_solve_kernel solves, the product with this copies
       for (int e = tid; e < ob * ob; e += kInvThreads)
@@ -1170,11 +1173,8 @@ __global__ void __launch_bounds__(kSolveThreads)
 #pragma unroll
   for (int k = 0; k < NB / 4; ++k) largest = max(largest, max(high_abs(a[k][0]), high_abs(a[k][1])));
   __shared__ uint2 slots[kSolveThreads / 32];
-  if (ill_conditioned_cta<kSolveThreads / 32>(slots, largest_t, largest)) {
-    double *x = tid < kSolveCols && c0 + tid < total ? column(tid) : nullptr;
-    substitute_columns<UPPER>(tk.D + k0 + k0 * tk.ldd, tk.ldd, kb, x, xs);
-    return;
-  }
+  publish_largest(slots, largest_t, largest);
+  __syncthreads();
   double c[NT][4];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
@@ -1185,6 +1185,11 @@ __global__ void __launch_bounds__(kSolveThreads)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
       dmma(c[nt], a[k][0], a[k][1], xs[(wn + 8 * nt + g) * LD + 4 * k + t]);
+  if (ill_conditioned_cta<kSolveThreads / 32>(slots)) {
+    double *x = tid < kSolveCols && c0 + tid < total ? column(tid) : nullptr;
+    substitute_columns<UPPER>(tk.D + k0 + k0 * tk.ldd, tk.ldd, kb, x, xs);
+    return;
+  }
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
